@@ -194,7 +194,12 @@ __device__ __forceinline__ bool inplace_convert_b1(uint8_t* stage, int c, Sync&&
   return true;
 }
 
-template <class Tr, int STG>
+// DIRECT (with STG = 2): every unit is one accumulator chunk (no K split,
+// K <= 32 * CHUNK), which the epilogue reads from TMEM block by block instead
+// of promoting it into registers: one rolled copy of the epilogue's code (the
+// unrolled one missed in the instruction cache, the roles of this kernel
+// evicting one another: 3.2 stalled warps an issue on the sigmoid form).
+template <class Tr, int STG, bool DIRECT>
 __global__ void __maxnreg__((FusedInplaceCfg<Tr, STG>::MAX_REGS))
     tc_fused_inplace_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                             const __grid_constant__ TcParams p) {
@@ -339,6 +344,7 @@ __global__ void __maxnreg__((FusedInplaceCfg<Tr, STG>::MAX_REGS))
     uint8_t* stg = staging + (warp - 2) * F::STAGING_PER_WARP;
     const uint32_t tempty_rank0 = mapa_shared(smem_u32(&tempty[0]), 0);
     int ci = 0;
+    uint32_t cph = 0;  // phase of this warp's C-load barrier
     for (int unit = unit0; unit < units; unit += unit_step) {
       Unit u;
       resolve_unit(p, &tmA, &tmB, unit, u);
@@ -353,27 +359,53 @@ __global__ void __maxnreg__((FusedInplaceCfg<Tr, STG>::MAX_REGS))
       };
       if (unit == unit0) prefetch_unit(unit);
       const int nchunks = (u.kb1 - u.kb0 + chunk - 1) / chunk;
-      float master[W];
-#pragma unroll
-      for (int j = 0; j < W; ++j) master[j] = 0.f;
-      bool ok = true;
-      for (int c = 0; c < nchunks; ++c) {
-        const int g = ci + c, buf = g % NBUF;
-        if (!__all_sync(0xffffffffu, mbar_wait(&tfull[buf], (g / NBUF) & 1, kErrTimeoutAccum, p.ctl))) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        Tr::accumulate(lane_base + (uint32_t)(buf * NACC * BN + colsub), master);
+      auto octx = [&]() {
+        OutCtx o = out_ctx(p, u);
+        o.tbar = &ebar[STG * (warp - 2)];
+        return o;
+      };
+      auto release = [&](int buf) {
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(tempty_rank0 + (uint32_t)(buf * sizeof(uint64_t)));
+        if (lane == 0) mbar_arrive_cluster_signal(tempty_rank0 + (uint32_t)(buf * sizeof(uint64_t)));
+      };
+      bool loaded = false;
+      if constexpr (STG >= 2)
+        loaded = EpiF32::load_c64(octx(), reinterpret_cast<float*>(stg), lane, row0, col0 + colsub);
+      bool ok = true;
+      if constexpr (DIRECT) {
+        const int buf = ci % NBUF;
+        ok = __all_sync(0xffffffffu, mbar_wait(&tfull[buf], (ci / NBUF) & 1, kErrTimeoutAccum, p.ctl));
+        if (ok) {
+          tc_fence_after();
+          prefetch_unit(unit + unit_step);
+          Tr::direct(octx(), lane_base + (uint32_t)(buf * NACC * BN + colsub), stg, lane, row0, col0 + colsub, loaded,
+                     cph, [&] { release(buf); });
+        }
+      } else {
+        float master[W];
+#pragma unroll
+        for (int j = 0; j < W; ++j) master[j] = 0.f;
+        for (int c = 0; c < nchunks; ++c) {
+          const int g = ci + c, buf = g % NBUF;
+          if (!__all_sync(0xffffffffu, mbar_wait(&tfull[buf], (g / NBUF) & 1, kErrTimeoutAccum, p.ctl))) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          Tr::accumulate(lane_base + (uint32_t)(buf * NACC * BN + colsub), master);
+          release(buf);
+        }
+        if (ok) {
+          prefetch_unit(unit + unit_step);
+          const OutCtx o = octx();
+          Tr::template finish<STG>(o, master, stg, lane, row0, col0 + colsub, u.z, loaded, cph);
+        }
       }
-      if (!ok) break;
-      prefetch_unit(unit + unit_step);
-      OutCtx o = out_ctx(p, u);
-      o.tbar = &ebar[STG * (warp - 2)];  // the epilogue uses tbar[0 .. STG-1]
-      Tr::template finish<STG>(o, master, stg, lane, row0, col0 + colsub, u.z);
+      if (!ok) {
+        if (loaded) EpiF32::wait_c64(octx(), cph);  // the C load writes this CTA's shared memory
+        break;
+      }
       ci += nchunks;
     }
     if (lane == 0) bulk_wait_all();  // this warp's TMA stores of C have completed
@@ -462,13 +494,13 @@ static cudaError_t launch_fused_kernel(K kernel, int threads, int smem, std::ato
 
 // BF16x3: a = A [128 rows][64 K] boxes, b = B [64 K][64 columns] boxes (no swizzle);
 // BF16x6: a = A [128 rows][32 K] boxes (128-byte swizzle), b = B [32 K][64 columns].
-template <class Tr, int STG>
+template <class Tr, int STG, bool DIRECT = false>
 static cudaError_t launch_fused_inplace(const CUtensorMap& a, const CUtensorMap& b, const TcParams& p, int sms,
                                         cudaStream_t st) {
   using F = FusedInplaceCfg<Tr, STG>;
   static std::atomic<uint64_t> attr_set{0};
   static std::atomic<int> clusters_cached[64];
-  return launch_fused_kernel(tc_fused_inplace_kernel<Tr, STG>, F::THREADS, F::SMEM, attr_set, clusters_cached, a, b, p,
+  return launch_fused_kernel(tc_fused_inplace_kernel<Tr, STG, DIRECT>, F::THREADS, F::SMEM, attr_set, clusters_cached, a, b, p,
                              sms, st);
 }
 

@@ -226,6 +226,10 @@ static Plan make_plan(const cucosma_gemm_desc* d, const DeviceInfo* di, bool all
   return pl;
 }
 
+// Every unit's K fits one promotion chunk: the kernels whose epilogue reads
+// TMEM directly.
+static bool one_chunk(const Tiling& t) { return t.splits == 1 && t.kblocks <= kPromoteChunk; }
+
 static int plan_launches(const Plan& pl) {
   if (pl.fused) return 1 + (pl.t.splits > 1 ? 1 : 0);
   if (pl.kind != 2) return 3 + (pl.t.splits > 1 ? 1 : 0);
@@ -273,7 +277,7 @@ namespace {
 
 // Kernel parameters of one tiling (shared fields of every precision path).
 TcParams tc_params(const cucosma_gemm_desc* d, const Tiling& t, const Plan& pl, void* C, uint8_t* w,
-                   const DeviceInfo* di) {
+                   const DeviceInfo* di, bool boxes2d = false) {
   TcParams p{};
   p.m = (int)d->m;
   p.n = (int)d->n;
@@ -298,32 +302,29 @@ TcParams tc_params(const cucosma_gemm_desc* d, const Tiling& t, const Plan& pl, 
     p.partial = 0;
     p.out = C;
     p.ldo = d->ldc;
-    // FP32 results leave through TMA when C allows a tensor map (16-byte
-    // aligned base and rows) and its rows end on a 16-byte boundary (a box
-    // store clips the columns past N only to the 16-byte granule: on B200 it
-    // wrote the rest of the last granule); otherwise the epilogue stores rows
-    // itself.  CUCOSMA_TMA_EPILOGUE=0 turns the TMA path off.
+    // FP32 results leave through TMA (validation made C's base and rows
+    // 16-byte aligned): the kernels with two staging blocks a warp move whole
+    // 32-column chunks by 3-D boxes and store the last N % 32 columns as rows;
+    // those with one block (boxes2d) use 2-D boxes when rows end on a 16-byte
+    // boundary (a box store clips the columns past N only to the 16-byte
+    // granule: on B200 it wrote the rest of the last granule).
+    // CUCOSMA_TMA_EPILOGUE=0 turns the TMA paths off.
     static const bool tma_epilogue = [] {
       const char* e = std::getenv("CUCOSMA_TMA_EPILOGUE");
       return !(e && e[0] == '0');
     }();
-    if (tma_epilogue && pl.kind != 2 && C != nullptr && (reinterpret_cast<uintptr_t>(C) & 15) == 0 &&
-        (d->ldc * 4) % 16 == 0 && d->n % 4 == 0)
-      p.tma_out = encode_2d(&p.tmc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, C, (uint64_t)d->n, (uint64_t)d->m,
-                            (uint64_t)d->ldc, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B) &&
-                          encode_2d(&p.tmc_pf, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, C, (uint64_t)d->n,
-                                    (uint64_t)d->m, (uint64_t)d->ldc, 64, 32, CU_TENSOR_MAP_SWIZZLE_NONE)
-                      ? 1
-                      : 0;
-    static const bool tma_wide = [] {
-      const char* e = std::getenv("CUCOSMA_TMA_WIDE");
-      return !(e && e[0] == '0');
-    }();
-    if (p.tma_out && tma_wide && d->n % 32 == 0)
-      p.tma_wide = encode_3d(&p.tmc3, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, C, 32, (uint64_t)d->n / 32, (uint64_t)d->m,
-                             32, (uint64_t)d->ldc, 32, 2, 32, CU_TENSOR_MAP_SWIZZLE_128B)
-                       ? 1
-                       : 0;
+    if (tma_epilogue && pl.kind != 2) {
+      const uint64_t N = (uint64_t)d->n, M = (uint64_t)d->m, ldc = (uint64_t)d->ldc;
+      const CUtensorMapDataType f32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+      if (boxes2d && N % 4 == 0)
+        p.tma_out = encode_2d(&p.tmc, f32, 4, C, N, M, ldc, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B) ? 1 : 0;
+      if (!boxes2d && N >= 32)
+        p.tma_wide = encode_3d(&p.tmc3, f32, 4, C, 32, N / 32, M, 32, ldc, 32, 2, 32, CU_TENSOR_MAP_SWIZZLE_128B) ? 1 : 0;
+      // prefetches of C (beta != 0 only)
+      if ((p.tma_out || p.tma_wide) && d->beta != 0.0 &&
+          !encode_2d(&p.tmc_pf, f32, 4, C, N, M, ldc, 64, 32, CU_TENSOR_MAP_SWIZZLE_NONE))
+        p.tma_out = p.tma_wide = 0;
+    }
   }
   return p;
 }
@@ -402,20 +403,23 @@ cucosma_status tc_gemm_ex(const cucosma_gemm_desc* d, const void* A, const void*
         !encode_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, B, n, k, d->ldb, pl.bn_local, kw,
                    CU_TENSOR_MAP_SWIZZLE_NONE))
       return CUCOSMA_STATUS_LAUNCH_FAILED;
-    const TcParams p = tc_params(d, pl.t, pl, C, w, di);
-    prof_begin(st);
     // C-heavy shapes (C traffic above a quarter of the operands'): the
     // variant with two staging blocks per epilogue warp and three stages
     // (256 x 1,048,576 x 256, beta 0.5: 0.85 against 0.94 ms on B200)
     const double c_bytes = (double)d->m * d->n * 4.0 * (d->beta != 0.0 ? 2.0 : 1.0);
     const double ab_bytes = ((double)d->m * d->k + (double)d->k * d->n) * 4.0;
     const bool c_heavy = c_bytes > 0.25 * ab_bytes;
+    const TcParams p = tc_params(d, pl.t, pl, C, w, di, !c_heavy);
+    prof_begin(st);
+    const bool direct = c_heavy && one_chunk(pl.t);
     if (pl.kind == 1)
-      e = c_heavy ? launch_fused_inplace<Bf16x6Pair, 2>(ta, tb, p, di->sms, st)
-                  : launch_fused_inplace<Bf16x6Pair, 1>(ta, tb, p, di->sms, st);
+      e = direct    ? launch_fused_inplace<Bf16x6Pair, 2, true>(ta, tb, p, di->sms, st)
+          : c_heavy ? launch_fused_inplace<Bf16x6Pair, 2>(ta, tb, p, di->sms, st)
+                    : launch_fused_inplace<Bf16x6Pair, 1>(ta, tb, p, di->sms, st);
     else
-      e = c_heavy ? launch_fused_inplace<Bf16x3Pair128, 2>(ta, tb, p, di->sms, st)
-                  : launch_fused_inplace<Bf16x3Pair128, 1>(ta, tb, p, di->sms, st);
+      e = direct    ? launch_fused_inplace<Bf16x3Pair128, 2, true>(ta, tb, p, di->sms, st)
+          : c_heavy ? launch_fused_inplace<Bf16x3Pair128, 2>(ta, tb, p, di->sms, st)
+                    : launch_fused_inplace<Bf16x3Pair128, 1>(ta, tb, p, di->sms, st);
     prof_end(st);
     launches += 1;
     if (e == cudaSuccess && pl.t.splits > 1) {
@@ -440,7 +444,7 @@ cucosma_status tc_gemm_ex(const cucosma_gemm_desc* d, const void* A, const void*
         !encode_3d(&tb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w + pl.off_b, k, n, nt, pl.kpad, (uint64_t)n * pl.kpad,
                    pl.bk, pl.bn_local, nt, CU_TENSOR_MAP_SWIZZLE_64B))
       return CUCOSMA_STATUS_LAUNCH_FAILED;
-    const TcParams p = tc_params(d, pl.t, pl, C, w, di);
+    const TcParams p = tc_params(d, pl.t, pl, C, w, di, pl.variant == kV3Wide);
     const int units = pl.t.tiles_m * pl.t.tiles_n * pl.t.splits;
     const int grid = std::min(units, di->sms);
     auto pair_grid = [&](int clusters) { return 2 * std::max(1, std::min(units, clusters)); };
@@ -453,7 +457,11 @@ cucosma_status tc_gemm_ex(const cucosma_gemm_desc* d, const void* A, const void*
         break;
       case kV3Small: e = launch<Bf16x3Promoted>(ta, tb, p, grid, st); break;
       case kV3Wide: e = launch<Bf16x3Wide>(ta, tb, p, grid, st); break;
-      case kV3Pair: e = launch<Bf16x3Pair>(ta, tb, p, pair_grid(max_pair_clusters<Bf16x3Pair>(di->sms)), st); break;
+      case kV3Pair:
+        if (one_chunk(pl.t))
+          e = launch<Bf16x3PairDirect>(ta, tb, p, pair_grid(max_pair_clusters<Bf16x3PairDirect>(di->sms)), st);
+        else
+          e = launch<Bf16x3Pair>(ta, tb, p, pair_grid(max_pair_clusters<Bf16x3Pair>(di->sms)), st); break;
       default: e = launch<Bf16x3>(ta, tb, p, grid, st);
     }
     prof_end(st);

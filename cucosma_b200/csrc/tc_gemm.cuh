@@ -42,16 +42,18 @@ struct alignas(64) GroupEntry {
 };
 
 struct TcParams {
-  // FP32 output C through TMA (tma_out = 1): 32 x 32 boxes, 128-byte
-  // swizzle; used by the epilogue for whole-problem outputs (not split-K
-  // partials, not grouped launches).
+  // FP32 output C through TMA (not split-K partials, not grouped launches).
+  // tmc (tma_out = 1): 32 x 32 boxes, 128-byte swizzle, for the kernels with
+  // one staging block a warp; needs N % 4 == 0, since a box store clips the
+  // columns past N only to the 16-byte granule.
   CUtensorMap tmc;
-  // The same C with 64-column boxes (no swizzle), for L2 prefetches only:
-  // 256-byte row requests (128-byte ones cap a stream near 4.6 TB/s on B200).
+  // C with 64-column boxes (no swizzle), for L2 prefetches only: 256-byte row
+  // requests (128-byte ones cap a stream near 4.6 TB/s on B200).
   CUtensorMap tmc_pf;
-  // With N a multiple of 32: C as {32 columns, N / 32 column chunks, M rows}
+  // tmc3 (tma_wide = 1): C as {32 columns, N / 32 whole column chunks, M rows}
   // with [32 rows][2 chunks][32] boxes (128-byte swizzle per 128-byte line),
-  // so the epilogue's loads and stores are 256-byte row requests.
+  // so the epilogue's loads and stores are 256-byte row requests; the last
+  // N % 32 columns are outside the map.
   CUtensorMap tmc3;
   int tma_out, tma_wide;
   int m, n, k;
@@ -90,11 +92,10 @@ struct OutCtx {
   int64_t ldo, ws_split_stride;
   const int32_t* ea;
   const int32_t* eb;
-  const CUtensorMap* tmc;     // non-null: the FP32 epilogue moves C by TMA
-  const CUtensorMap* tmc_pf;  // its 64-column prefetch boxes
-  const CUtensorMap* tmc3;    // non-null: 64-column 3-D boxes (needs two staging blocks)
-  uint64_t* tbar;          // this epilogue warp's barriers for its C loads (one per staging block)
-  int stg_blocks;          // 32 x 32 staging blocks this warp has (1 or 2)
+  const CUtensorMap* tmc;     // non-null: 32 x 32 boxes of C (one staging block a warp)
+  const CUtensorMap* tmc_pf;  // non-null: 64-column boxes for L2 prefetches of C
+  const CUtensorMap* tmc3;    // non-null: 64-column 3-D boxes of C's whole chunks (two staging blocks)
+  uint64_t* tbar;             // this epilogue warp's barriers for its C loads
   WaitCtl ctl;
 };
 

@@ -109,7 +109,7 @@ __device__ __forceinline__ void resolve_unit(const TcParams& p, const CUtensorMa
 // last element).
 __device__ __forceinline__ void prefetch_c_block(const OutCtx& o, int row0, int col0, int cols, int es, int lane) {
   if (o.partial || o.beta == 0.0 || col0 >= o.n) return;
-  if (o.tmc != nullptr) {
+  if (o.tmc_pf != nullptr) {
     // the TMA epilogue's boxes, prefetched by the async proxy (the
     // epilogue's own proxy fences then have no prefetches of their own to
     // wait for)
@@ -137,10 +137,10 @@ __device__ __forceinline__ OutCtx out_ctx(const TcParams& p, const Unit& u) {
   o.beta = p.beta;
   o.ctl = p.ctl;
   o.tbar = nullptr;
-  o.stg_blocks = 1;
-  o.tmc = (u.group < 0 && p.tma_out && !p.partial) ? &p.tmc : nullptr;
-  o.tmc_pf = &p.tmc_pf;
-  o.tmc3 = (o.tmc != nullptr && p.tma_wide) ? &p.tmc3 : nullptr;
+  const bool whole = u.group < 0 && !p.partial;
+  o.tmc = (whole && p.tma_out) ? &p.tmc : nullptr;
+  o.tmc3 = (whole && p.tma_wide) ? &p.tmc3 : nullptr;
+  o.tmc_pf = (o.tmc != nullptr || o.tmc3 != nullptr) ? &p.tmc_pf : nullptr;
   if (u.group < 0) {
     o.m = p.m;
     o.n = p.n;
@@ -478,6 +478,7 @@ __global__ void __maxnreg__(Tr::MAX_REGS)
       if (lane == 0) mbar_arrive(rank == 0 ? &tempty[idx] : &tfwd[idx]);
     };
     int ci = 0;
+    uint32_t cph = 0;  // phase of this warp's C-load barrier
     bool ok = true;
     for (int unit = unit0; unit < units && ok; unit += unit_step) {
       Unit u;
@@ -492,20 +493,25 @@ __global__ void __maxnreg__(Tr::MAX_REGS)
         Unit v;
         resolve_unit(p, &tmA, &tmB, un, v);
         prefetch_c_block(out_ctx(p, v), v.tm * TILE_M + (int)rank * 128 + 32 * q,
-                         v.tn * BN + (Tr::PROMOTE ? colsub : 0), Tr::PROMOTE ? W : BN, Tr::kInt8 ? 8 : 4, lane);
+                         v.tn * BN + colsub, W, Tr::kInt8 ? 8 : 4, lane);
       };
       if (unit == unit0) prefetch_unit(unit);
       // the output context is built where it is used (fewer registers held across the chunk loop)
       auto octx = [&]() {
         OutCtx o = out_ctx(p, u);
         o.tbar = &ebar[2 * (warp - 2)];
-        o.stg_blocks = Tr::STAGING_PER_WARP / (32 * 32 * 4);
         return o;
       };
       if constexpr (Tr::PROMOTE) {
         float master[W];
 #pragma unroll
         for (int j = 0; j < W; ++j) master[j] = 0.f;
+        // (with 128 accumulators a thread the load starts after the last chunk:
+        // holding its state across the chunk loop spilled)
+        constexpr bool kEarlyC = W <= 64;
+        bool loaded = false;
+        if constexpr (kEarlyC)
+          loaded = Tr::Epilogue::load_c64(octx(), reinterpret_cast<float*>(stg), lane, row0, col0 + colsub);
         for (int cs = u.kb0; cs < u.kb1; cs += chunk, ++ci) {
           const int buf = ci % NBUF;
           ok = __all_sync(0xffffffffu, mbar_wait(&tfull[buf], (ci / NBUF) & 1, kErrTimeoutAccum, p.ctl));
@@ -522,9 +528,29 @@ __global__ void __maxnreg__(Tr::MAX_REGS)
             release(buf);
           }
         }
-        if (!ok) break;
+        if (!ok) {
+          if (loaded) Tr::Epilogue::wait_c64(octx(), cph);  // the C load writes this CTA's shared memory
+          break;
+        }
+        if constexpr (!kEarlyC)
+          loaded = Tr::Epilogue::load_c64(octx(), reinterpret_cast<float*>(stg), lane, row0, col0 + colsub);
         prefetch_unit(unit + unit_step);
-        Tr::finish(octx(), master, stg, lane, row0, col0 + colsub, z);
+        Tr::finish(octx(), master, stg, lane, row0, col0 + colsub, z, loaded, cph);
+      } else if constexpr (Tr::DIRECT) {
+        const int buf = ci % NBUF;
+        const OutCtx o = octx();
+        const int col = col0 + colsub;
+        const bool loaded = Tr::Epilogue::load_c64(o, reinterpret_cast<float*>(stg), lane, row0, col);
+        ok = __all_sync(0xffffffffu, mbar_wait(&tfull[buf], (ci / NBUF) & 1, kErrTimeoutAccum, p.ctl));
+        if (!ok) {
+          if (loaded) Tr::Epilogue::wait_c64(o, cph);  // the C load writes this CTA's shared memory
+          break;
+        }
+        tc_fence_after();
+        prefetch_unit(unit + unit_step);
+        Tr::direct(o, lane_base + (uint32_t)(buf * NACC * BN + colsub), stg, lane, row0, col, loaded, cph,
+                   [&] { release(buf); });
+        ++ci;
       } else {
         const int buf = ci % NBUF;
         ok = __all_sync(0xffffffffu, mbar_wait(&tfull[buf], (ci / NBUF) & 1, kErrTimeoutAccum, p.ctl));
@@ -580,19 +606,31 @@ struct EpiF32 {
 
   // This lane's row of the block: epi(alpha * acc + beta * C) with C read
   // from (and the result written back to) the swizzled staging row s4.
+  // The chunks of C are read kBatch at a time before any result is written:
+  // the compiler cannot tell a chunk's store from the next chunk's load, so
+  // chunk by chunk every load (and the activation behind it) waited out its
+  // latency in turn.
   template <int EPI>
   static __device__ __forceinline__ void combine_row_t(float4* s4, const float (&acc)[32], float alpha, float beta,
                                                        int lane) {
+    constexpr int kBatch = 4;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const int pos = c ^ (lane & 7);
-      const float4 cv = beta != 0.f ? s4[pos] : make_float4(0.f, 0.f, 0.f, 0.f);
-      float4 r;
-      r.x = epi_t<EPI>(combine(acc[4 * c], alpha, beta, &cv.x));
-      r.y = epi_t<EPI>(combine(acc[4 * c + 1], alpha, beta, &cv.y));
-      r.z = epi_t<EPI>(combine(acc[4 * c + 2], alpha, beta, &cv.z));
-      r.w = epi_t<EPI>(combine(acc[4 * c + 3], alpha, beta, &cv.w));
-      s4[pos] = r;
+    for (int b = 0; b < 8; b += kBatch) {
+      float4 r[kBatch];
+      // (a select, not a branch: straight-line code lets the batches' activations overlap)
+#pragma unroll
+      for (int c = 0; c < kBatch; ++c)
+        r[c] = beta != 0.f ? s4[(b + c) ^ (lane & 7)] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int c = 0; c < kBatch; ++c) {
+        const int j = 4 * (b + c);
+        r[c].x = epi_t<EPI>(combine(acc[j], alpha, beta, &r[c].x));
+        r[c].y = epi_t<EPI>(combine(acc[j + 1], alpha, beta, &r[c].y));
+        r[c].z = epi_t<EPI>(combine(acc[j + 2], alpha, beta, &r[c].z));
+        r[c].w = epi_t<EPI>(combine(acc[j + 3], alpha, beta, &r[c].w));
+      }
+#pragma unroll
+      for (int c = 0; c < kBatch; ++c) s4[(b + c) ^ (lane & 7)] = r[c];
     }
   }
   static __device__ __forceinline__ void combine_row(int epi, float4* s4, const float (&acc)[32], float alpha,
@@ -605,80 +643,187 @@ struct EpiF32 {
       combine_row_t<kEpiNone>(s4, acc, alpha, beta, lane);
   }
 
-  // Write one 32 x 32 block of results: acc[j] is this lane's row (row0 +
-  // lane) at column col + j.
-  //  * store_block_tma (p.tmc set): lane 0 waits until the previous block's store has read
-  //    the buffer, brings the C block in (beta != 0; out-of-range rows and
-  //    columns read as zero), every lane combines its row in place, and lane
-  //    0 stores the block (out-of-range parts are not written) -- a handful
-  //    of instructions per element, no predicates, C moved as whole boxes.
-  //  * store_block (split-K partials, grouped problems, unaligned C): C is
-  //    fetched by cp.async (lanes = columns, all rows in flight; C was
-  //    prefetched into L2), combined per row, and stored as 128-byte rows;
-  //    partials are stored raw.
+  // One 32 x 32 block through the 2-D map (kernels with a single 4 KB staging
+  // block a warp): lane 0 waits until the previous block's store has read the
+  // buffer, brings the C block in (beta != 0; out-of-range rows and columns
+  // read as zero), every lane combines its row in place, and lane 0 stores
+  // the block (out-of-range parts are not written).
   static __device__ __forceinline__ void store_block_tma(const OutCtx& p, const float (&acc)[32], float* stg, int lane,
                                                          int row0, int col) {
     if (col >= p.n) return;  // the whole block lies right of C (col is the block's first column)
     const float alpha = (float)p.alpha, beta = (float)p.beta;
     float4* s4 = reinterpret_cast<float4*>(stg) + lane * 8;  // this lane's row
-    {
-      if (lane == 0) bulk_wait_read_all();
-      __syncwarp();
-      if (beta != 0.f) {
-        if (lane == 0) {
-          const uint64_t token = mbar_arrive_expect_tx_token(p.tbar, 32 * 32 * 4);
-          tma_load_2d(stg, p.tmc, col, row0, p.tbar);
-          if (!mbar_wait_token(p.tbar, token, kErrTimeoutOutput, p.ctl))
-            mbar_wait_token(p.tbar, token, kErrTimeoutDrain, p.ctl);  // once more before the buffer is reused
-        }
-        __syncwarp();
-      }
-      combine_row(p.epilogue, s4, acc, alpha, beta, lane);
-      fence_proxy_async_smem();  // the block is read by TMA (async proxy)
-      __syncwarp();
+    if (lane == 0) bulk_wait_read_all();
+    __syncwarp();
+    if (beta != 0.f) {
       if (lane == 0) {
-        tma_store_2d(p.tmc, stg, col, row0);
-        bulk_commit();
+        const uint64_t token = mbar_arrive_expect_tx_token(p.tbar, 32 * 32 * 4);
+        tma_load_2d(stg, p.tmc, col, row0, p.tbar);
+        if (!mbar_wait_token(p.tbar, token, kErrTimeoutOutput, p.ctl))
+          mbar_wait_token(p.tbar, token, kErrTimeoutDrain, p.ctl);  // once more before the buffer is reused
       }
+      __syncwarp();
+    }
+    combine_row(p.epilogue, s4, acc, alpha, beta, lane);
+    fence_proxy_async_smem();  // the block is read by TMA (async proxy)
+    __syncwarp();
+    if (lane == 0) {
+      tma_store_2d(p.tmc, stg, col, row0);
+      bulk_commit();
     }
   }
 
+  // Row stores of one 32 x 32 block whose raw accumulators acc (this lane's
+  // row) pass through the staging block, lanes = columns: split-K partials,
+  // grouped problems, and the last N % 32 columns of C, which the box stores
+  // cannot clip exactly.  With a second staging block (STG >= 2) C is brought
+  // there by cp.async, all rows in flight.  The row loops are one call, not
+  // inlined per block: the callers hold up to 128 accumulators a thread.
+  template <int EPI, int STG>
+  static __device__ __forceinline__ void rows_loop(float* w, int64_t ldo, const float* stg, int lane, int rows,
+                                                   float alpha, float beta) {
+#pragma unroll 4
+    for (int r = 0; r < rows; ++r) {
+      float* o = w + (int64_t)r * ldo;
+      const float* c = STG >= 2 ? stg + 32 * 32 + sw(r, lane) : o;
+      *o = epi_t<EPI>(combine(stg[sw(r, lane)], alpha, beta, c));
+    }
+  }
+  // epilogue < 0: raw partial sums.
+  template <int STG>
+  static __device__ __noinline__ void rows_out(float* w, int64_t ldo, float* stg, int lane, int rows, int epilogue,
+                                               float alpha, float beta) {
+    if (epilogue < 0) {
+#pragma unroll 4
+      for (int r = 0; r < rows; ++r) w[(int64_t)r * ldo] = stg[sw(r, lane)];
+      return;
+    }
+    if (STG >= 2 && beta != 0.f) {
+#pragma unroll 4
+      for (int r = 0; r < rows; ++r) cp_async4(&stg[32 * 32 + sw(r, lane)], w + (int64_t)r * ldo);
+      cp_async_wait_all();  // each lane reads back only what it copied
+    }
+    if (epilogue == kEpiSigmoid)
+      rows_loop<kEpiSigmoid, STG>(w, ldo, stg, lane, rows, alpha, beta);
+    else if (epilogue == kEpiRelu)
+      rows_loop<kEpiRelu, STG>(w, ldo, stg, lane, rows, alpha, beta);
+    else
+      rows_loop<kEpiNone, STG>(w, ldo, stg, lane, rows, alpha, beta);
+  }
+  template <int STG>
   static __device__ __forceinline__ void store_block(const OutCtx& p, float* o, const float (&acc)[32], float* stg,
                                                      int lane, int row0, int col) {
     if (col >= p.n) return;  // the whole block lies right of C (col is the block's first column)
-    const float alpha = (float)p.alpha, beta = (float)p.beta;
-    float4* s4 = reinterpret_cast<float4*>(stg) + lane * 8;  // this lane's row
-    const int cl = col + lane;  // this lane's column in the store pass
-    if (p.partial) {
+    if (lane == 0) bulk_wait_read_all();  // box stores issued earlier have read the staging
+    __syncwarp();
+    float4* s4 = reinterpret_cast<float4*>(stg) + lane * 8;
 #pragma unroll
-      for (int c = 0; c < 8; ++c)
-        s4[c ^ (lane & 7)] = make_float4(acc[4 * c], acc[4 * c + 1], acc[4 * c + 2], acc[4 * c + 3]);
-    } else {
-      if (beta != 0.f) {
-#pragma unroll 4
-        for (int r = 0; r < 32; ++r) {
-          const int row = row0 + r;
-          if (row < p.m && cl < p.n)
-            cp_async4(&stg[sw(r, lane)], o + (int64_t)row * p.ldo + cl);
-          else
-            stg[sw(r, lane)] = 0.f;
+    for (int c = 0; c < 8; ++c)
+      s4[c ^ (lane & 7)] = make_float4(acc[4 * c], acc[4 * c + 1], acc[4 * c + 2], acc[4 * c + 3]);
+    __syncwarp();
+    if (col + lane < p.n)
+      rows_out<STG>(o + (int64_t)row0 * p.ldo + col + lane, p.ldo, stg, lane, min(32, p.m - row0),
+                    p.partial ? -1 : p.epilogue, (float)p.alpha, (float)p.beta);
+    fence_proxy_async_smem();  // the staging may next be written by a TMA load
+    __syncwarp();
+  }
+
+  // 64-column blocks through the 3-D map: one 8 KB staging block [32 rows]
+  // [2 chunks][32] (line 2r + h of row r, chunk h, 128-byte swizzle per line),
+  // one box load of C (beta != 0) and one box store, 256-byte row requests
+  // each.  The map has N / 32 chunks (rounded down), so a box never touches
+  // the last N % 32 columns; full_chunks() says how many of the block's two
+  // chunks the box covers.
+  static __device__ __forceinline__ int full_chunks(const OutCtx& p, int col) {
+    return p.tmc3 == nullptr || col >= p.n ? 0 : min(2, (p.n - col) / 32);
+  }
+  // Makes the staging free for the block at (row0, col) and starts its C
+  // load, early enough that it lands while the accumulator is finished.
+  // Returns whether a load was issued (warp-uniform; it completes a phase of
+  // the warp's barrier).
+  static __device__ __forceinline__ bool load_c64(const OutCtx& p, float* stg, int lane, int row0, int col) {
+    const bool ld = p.beta != 0.0 && full_chunks(p, col) > 0;
+    if (lane == 0) {
+      bulk_wait_read_all();  // the previous block's store has read the staging
+      if (ld) {
+        mbar_arrive_expect_tx(&p.tbar[0], 2 * 32 * 32 * 4);
+        tma_load_3d_hint(stg, p.tmc3, 0, col / 32, row0, &p.tbar[0], l2_evict_first_policy());
+      }
+    }
+    __syncwarp();
+    return ld;
+  }
+  static __device__ __forceinline__ void wait_c64(const OutCtx& p, uint32_t parity) {
+    if (!mbar_wait(&p.tbar[0], parity, kErrTimeoutOutput, p.ctl))
+      mbar_wait(&p.tbar[0], parity, kErrTimeoutDrain, p.ctl);  // once more before the buffer is reused
+    __syncwarp();
+  }
+  static __device__ __forceinline__ void store_c64(const OutCtx& p, float* stg, int lane, int row0, int col) {
+    fence_proxy_async_smem();  // the block is read by TMA (async proxy)
+    __syncwarp();
+    if (lane == 0) {
+      tma_store_3d_hint(p.tmc3, stg, 0, col / 32, row0, l2_evict_first_policy());
+      bulk_commit();
+    }
+  }
+
+  // Unpromoted result (the unit's whole K in one accumulator chunk): the
+  // warp's W columns in 64-column blocks read from TMEM (the corrections'
+  // accumulator, if there is one, added first, as the promotion does).  The
+  // loop over blocks is rolled and holds one block in registers, so the code
+  // of the three activations stays small.  loaded: the first block's C load
+  // was started by load_c64 before the accumulator was waited for; parity is
+  // left at the phase the next load will complete.  release() is called as
+  // soon as the accumulator has been read.
+  template <int W, int STRIDE, int NACC, class Release>
+  static __device__ __forceinline__ void direct(const OutCtx& p, uint32_t tacc, float* stg, int lane, int row0,
+                                                int col0, bool loaded, uint32_t& parity, Release&& release) {
+    const float alpha = (float)p.alpha, beta = (float)p.beta;
+#pragma unroll 1
+    for (int c0 = 0; c0 < W; c0 += 64) {
+      const int col = col0 + c0;
+      if (c0 > 0) loaded = load_c64(p, stg, lane, row0, col);
+      const int full = full_chunks(p, col);
+      float acc[64];
+      {
+        uint32_t v0[32], v1[32];
+        const uint32_t t = tacc + (uint32_t)((NACC - 1) * STRIDE + c0);
+        tmem_ld32(t, v0);
+        tmem_ld32(t + 32, v1);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          acc[j] = __fadd_rn(0.f, __uint_as_float(v0[j]));
+          acc[32 + j] = __fadd_rn(0.f, __uint_as_float(v1[j]));
         }
-        cp_async_wait_all();
-        __syncwarp();
       }
-      combine_row(p.epilogue, s4, acc, alpha, beta, lane);
-    }
-    __syncwarp();
-    if (cl < p.n) {
-      float* w = o + cl;
-      const int64_t ld = p.ldo;
-#pragma unroll 4
-      for (int r = 0; r < 32; ++r) {
-        const int row = row0 + r;
-        if (row < p.m) w[(int64_t)row * ld] = stg[sw(r, lane)];
+      if constexpr (NACC == 2) {
+        uint32_t v0[32], v1[32];
+        tmem_ld32(tacc + (uint32_t)c0, v0);
+        tmem_ld32(tacc + (uint32_t)(c0 + 32), v1);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          acc[j] = __fadd_rn(acc[j], __uint_as_float(v0[j]));
+          acc[32 + j] = __fadd_rn(acc[32 + j], __uint_as_float(v1[j]));
+        }
       }
+      if (c0 == W - 64) release();
+      if (full > 0) {
+        if (loaded) {
+          wait_c64(p, parity);
+          parity ^= 1;
+        }
+        float4* s4 = reinterpret_cast<float4*>(stg);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          combine_row(p.epilogue, s4 + (2 * lane + h) * 8, cols32(acc, 32 * h), alpha, beta, 2 * lane + h);
+        store_c64(p, stg, lane, row0, col);
+      }
+      float* o = reinterpret_cast<float*>(p.out);
+      if (full < 1) store_block<2>(p, o, cols32(acc, 0), stg, lane, row0, col);
+      if (full < 2) store_block<2>(p, o, cols32(acc, 32), stg, lane, row0, col + 32);
     }
-    __syncwarp();
   }
 
   template <int BN>
@@ -701,7 +846,7 @@ struct EpiF32 {
       if (p.tmc != nullptr)
         store_block_tma(p, acc, stg, lane, row0, col0 + c0);
       else
-        store_block(p, o, acc, stg, lane, row0, col0 + c0);
+        store_block<2>(p, o, acc, stg, lane, row0, col0 + c0);
     }
   }
 
@@ -742,118 +887,69 @@ struct EpiF32 {
     }
   }
 
-  // TMA path with two staging blocks: block i + 1's C load is in flight
-  // while block i is combined and stored (each buffer is reloaded once the
-  // store issued from it two blocks earlier has read it).
-  template <int BN>
-  static __device__ __forceinline__ void finish_tma2(const OutCtx& p, const float (&master)[BN], float* stg, int lane,
-                                                     int row0, int col0) {
-    const float alpha = (float)p.alpha, beta = (float)p.beta;
-    const bool ld = beta != 0.f;
-    if (lane == 0) bulk_wait_read_all();  // the previous tile's stores have read both blocks
-    __syncwarp();
-    uint64_t tok[2] = {0, 0};
-    if (ld && lane == 0 && col0 < p.n) {
-      tok[0] = mbar_arrive_expect_tx_token(&p.tbar[0], 32 * 32 * 4);
-      tma_load_2d(stg, p.tmc, col0, row0, &p.tbar[0]);
-    }
-#pragma unroll
-    for (int i = 0; i < BN / 32; ++i) {
-      const int col = col0 + 32 * i;
-      if (col >= p.n) break;
-      float* b = stg + (i & 1) * (32 * 32);
-      if (ld) {
-        if (lane == 0 && !mbar_wait_token(&p.tbar[i & 1], tok[i & 1], kErrTimeoutOutput, p.ctl))
-          mbar_wait_token(&p.tbar[i & 1], tok[i & 1], kErrTimeoutDrain, p.ctl);
-        __syncwarp();
-      } else if (i >= 2) {
-        if (lane == 0) bulk_wait_read_but_last();  // the store from this block two steps ago has read it
-        __syncwarp();
-      }
-      combine_row(p.epilogue, reinterpret_cast<float4*>(b) + lane * 8, cols32(master, 32 * i), alpha, beta, lane);
-      fence_proxy_async_smem();  // the block is read by TMA (async proxy)
-      __syncwarp();
-      if (lane == 0) {
-        tma_store_2d(p.tmc, b, col, row0);
-        bulk_commit();
-        if (ld && i + 1 < BN / 32 && col + 32 < p.n) {
-          bulk_wait_read_but_last();  // the other block's previous store has read it
-          float* nb = stg + ((i + 1) & 1) * (32 * 32);
-          tok[(i + 1) & 1] = mbar_arrive_expect_tx_token(&p.tbar[(i + 1) & 1], 32 * 32 * 4);
-          tma_load_2d(nb, p.tmc, col + 32, row0, &p.tbar[(i + 1) & 1]);
-        }
-      }
-    }
-  }
-
-  // 64-column blocks through the 3-D map: one 8 KB staging block [32 rows]
-  // [2 chunks][32] (line 2r + h of row r, chunk h, 128-byte swizzle), one box
-  // load of C (beta != 0) and one box store per block, 256-byte rows each.
-  template <int BN>
-  static __device__ __forceinline__ void finish_tma_wide(const OutCtx& p, const float (&master)[BN], float* stg,
-                                                         int lane, int row0, int col0) {
-    const float alpha = (float)p.alpha, beta = (float)p.beta;
-    float4* s4 = reinterpret_cast<float4*>(stg);
-    const uint64_t pol = l2_evict_first_policy();
-#pragma unroll
-    for (int i = 0; i < BN / 64; ++i) {
-      const int col = col0 + 64 * i;
-      if (col >= p.n) break;
-      if (lane == 0) bulk_wait_read_all();  // the previous block's store has read the buffer
-      __syncwarp();
-      if (beta != 0.f) {
-        if (lane == 0) {
-          const uint64_t token = mbar_arrive_expect_tx_token(&p.tbar[0], 2 * 32 * 32 * 4);
-          tma_load_3d_hint(stg, p.tmc3, 0, col / 32, row0, &p.tbar[0], pol);
-          if (!mbar_wait_token(&p.tbar[0], token, kErrTimeoutOutput, p.ctl))
-            mbar_wait_token(&p.tbar[0], token, kErrTimeoutDrain, p.ctl);
-        }
-        __syncwarp();
-      }
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int line = 2 * lane + h;
-        combine_row(p.epilogue, s4 + line * 8, cols32(master, 64 * i + 32 * h), alpha, beta, line);
-      }
-      fence_proxy_async_smem();  // the block is read by TMA (async proxy)
-      __syncwarp();
-      if (lane == 0) {
-        tma_store_3d_hint(p.tmc3, stg, 0, col / 32, row0, pol);
-        bulk_commit();
-      }
-    }
-  }
-
-  // STG: 32 x 32 staging blocks the warp has (2 in tc_gemm_kernel, 1 in the
-  // fused kernels), fixed at compile time so only the matching paths exist.
+  // Promoted result in registers.  STG: 32 x 32 staging blocks the warp has
+  // (2 in tc_gemm_kernel, 1 in a fused kernel), fixed at compile time so only
+  // the matching paths exist.  With two, 64-column blocks go through the 3-D
+  // map; the first block's C load was started by load_c64 before the last
+  // accumulator chunk was waited for (loaded; parity: its barrier phase, left
+  // at the phase the next load will complete).
   template <int BN, int STG>
   static __device__ __forceinline__ void finish(const OutCtx& p, const float (&master)[BN], uint8_t* stg_raw,
-                                                int lane, int row0, int col0, int z) {
+                                                int lane, int row0, int col0, int z, bool loaded, uint32_t& parity) {
     float* stg = reinterpret_cast<float*>(stg_raw);
-    if (p.tmc != nullptr) {
-      if constexpr (STG >= 2) {
-        if (p.tmc3 != nullptr && BN % 64 == 0)
-          finish_tma_wide<BN>(p, master, stg, lane, row0, col0);
-        else
-          finish_tma2<BN>(p, master, stg, lane, row0, col0);
+    float* o = reinterpret_cast<float*>(p.out) + (p.partial ? (int64_t)z * p.ws_split_stride : 0);
+    if constexpr (STG >= 2) {
+      static_assert(BN % 64 == 0, "64-column blocks");
+      const float alpha = (float)p.alpha, beta = (float)p.beta;
+      float4* s4 = reinterpret_cast<float4*>(stg);
+      // Warps whose columns are all whole chunks and those at the right edge
+      // apart (together, the accumulators stayed live longer and spilled).
+      if (full_chunks(p, col0 + BN - 64) == 2) {
+#pragma unroll
+        for (int i = 0; i < BN / 64; ++i) {
+          if (i > 0) loaded = load_c64(p, stg, lane, row0, col0 + 64 * i);
+          if (loaded) {
+            wait_c64(p, parity);
+            parity ^= 1;
+          }
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int line = 2 * lane + h;
+            combine_row(p.epilogue, s4 + line * 8, cols32(master, 64 * i + 32 * h), alpha, beta, line);
+          }
+          store_c64(p, stg, lane, row0, col0 + 64 * i);
+        }
         return;
       }
 #pragma unroll
-      for (int c0 = 0; c0 < BN; c0 += 32) {
-        float acc[32];
+      for (int i = 0; i < BN / 64; ++i) {
+        const int col = col0 + 64 * i;
+        if (col >= p.n) break;
+        const int full = full_chunks(p, col);
+        if (i > 0) loaded = load_c64(p, stg, lane, row0, col);
+        if (loaded) {
+          wait_c64(p, parity);
+          parity ^= 1;
+        }
 #pragma unroll
-        for (int j = 0; j < 32; ++j) acc[j] = master[c0 + j];
-        store_block_tma(p, acc, stg, lane, row0, col0 + c0);
+        for (int h = 0; h < 2; ++h) {
+          if (h < full) {
+            const int line = 2 * lane + h;
+            combine_row(p.epilogue, s4 + line * 8, cols32(master, 64 * i + 32 * h), alpha, beta, line);
+            if (h == full - 1) store_c64(p, stg, lane, row0, col);
+          } else {
+            store_block<2>(p, o, cols32(master, 64 * i + 32 * h), stg, lane, row0, col + 32 * h);
+          }
+        }
       }
       return;
     }
-    float* o = reinterpret_cast<float*>(p.out) + (p.partial ? (int64_t)z * p.ws_split_stride : 0);
 #pragma unroll
     for (int c0 = 0; c0 < BN; c0 += 32) {
-      float acc[32];
-#pragma unroll
-      for (int j = 0; j < 32; ++j) acc[j] = master[c0 + j];
-      store_block(p, o, acc, stg, lane, row0, col0 + c0);
+      if (p.tmc != nullptr)
+        store_block_tma(p, cols32(master, c0), stg, lane, row0, col0 + c0);
+      else
+        store_block<1>(p, o, cols32(master, c0), stg, lane, row0, col0 + c0);
     }
   }
 };
@@ -987,7 +1083,8 @@ constexpr int kSmemBudget = 227 * 1024;
 // 128-byte swizzled row, so slice p sits in tile p / 4 at byte offset
 // (p % 4) * 32 -- selected like a K offset inside the swizzle atom.
 template <int NT_, int BN_, int SWZ_, int NA_, int NB_, int NACC_, bool INT8_, class Epi, bool PROMOTE_ = false,
-          int CHUNK_ = 0, int EPI_WARPS_ = 4, int SUB_ = 0, bool PAIR_ = false, bool SPLIT_ = false>
+          int CHUNK_ = 0, int EPI_WARPS_ = 4, int SUB_ = 0, bool PAIR_ = false, bool SPLIT_ = false,
+          bool DIRECT_ = false>
 struct TraitsBase {
   static constexpr int NT = NT_, BN = BN_, SWZ = SWZ_, NA = NA_, NB = NB_, NACC = NACC_;
   static constexpr bool kInt8 = INT8_;
@@ -1011,6 +1108,9 @@ struct TraitsBase {
   // first and frees them, so the next chunk's correction MMAs (issued first
   // in every k-block) overlap the drain of the main accumulator.
   static constexpr bool SPLIT = SPLIT_;
+  // DIRECT: every unit's K fits one accumulator chunk (kPromoteChunk k-blocks),
+  // so the epilogue reads TMEM straight into C blocks, 64 columns a warp.
+  static constexpr bool DIRECT = DIRECT_;
   // 4 epilogue warps (one per TMEM lane quadrant) or 8 (each quadrant
   // split into two column halves, so promoted register accumulators fit).
   static constexpr int EPI_WARPS = EPI_WARPS_;
@@ -1021,7 +1121,9 @@ struct TraitsBase {
   static constexpr int MAX_REGS = (16384 / (32 * WARPS_PER_SMSP)) / 8 * 8 > 255 ? 255
                                                                                : (16384 / (32 * WARPS_PER_SMSP)) / 8 * 8;
   static constexpr int COLS_PER_EW = BN / (EPI_WARPS / 4);
-  static_assert(EPI_WARPS == 4 || (EPI_WARPS == 8 && PROMOTE_), "8 epilogue warps only for promotion");
+  static_assert(EPI_WARPS == 4 || (EPI_WARPS == 8 && PROMOTE_) || (DIRECT_ && COLS_PER_EW % 64 == 0),
+                "8 epilogue warps only for promotion or 64-column blocks");
+  static_assert(!DIRECT_ || !PROMOTE_, "direct: no promotion");
   static constexpr bool PACKED = INT8_;
   static constexpr int BK = PACKED ? 32 : SWZ / 2;  // K elements per stage
   static constexpr int KSTEPS = PACKED ? 1 : SWZ / 32;
@@ -1059,6 +1161,7 @@ struct TraitsBase {
                                                   int col0, int z) {
     Epi::template run<BN>(p, tacc, stg, lane, row0, col0, z);
   }
+  using Epilogue = Epi;
   static constexpr bool kDrain = Epi::kDrain;
   static __device__ __forceinline__ void drain(uint32_t tacc, uint8_t* stg, int lane) {
     Epi::template drain<BN>(tacc, stg, lane);
@@ -1076,8 +1179,13 @@ struct TraitsBase {
   }
   template <int STG = STAGING_PER_WARP / 4096>
   static __device__ __forceinline__ void finish(const OutCtx& p, const float (&master)[COLS_PER_EW], uint8_t* stg,
-                                                int lane, int row0, int col0, int z) {
-    if constexpr (PROMOTE) Epi::template finish<COLS_PER_EW, STG>(p, master, stg, lane, row0, col0, z);
+                                                int lane, int row0, int col0, int z, bool loaded, uint32_t& parity) {
+    if constexpr (PROMOTE) Epi::template finish<COLS_PER_EW, STG>(p, master, stg, lane, row0, col0, z, loaded, parity);
+  }
+  template <class Release>
+  static __device__ __forceinline__ void direct(const OutCtx& p, uint32_t tacc, uint8_t* stg, int lane, int row0,
+                                                int col, bool loaded, uint32_t& parity, Release&& release) {
+    Epi::template direct<COLS_PER_EW, BN, NACC>(p, tacc, reinterpret_cast<float*>(stg), lane, row0, col, loaded, parity, release);
   }
 };
 
@@ -1134,6 +1242,18 @@ struct Bf16x6 : TraitsBase<6, 128, 64, 3, 3, 2, false, EpiF32, true, kPromoteChu
 //               (one buffer, split release); the 256 x 128 tiles need about
 //               1.5x the L2-to-shared-memory bandwidth per flop.
 struct Bf16x3Pair : TraitsBase<3, 256, 64, 2, 2, 1, false, EpiF32, true, kPromoteChunk, 8, 0, true> {
+  static constexpr TermTable<3> kTerms{{1, 0, 0}, {0, 1, 0}, {0, 0, 0}, {true, false, false}};
+};
+// The 256 x 256 pair for K <= 32 * kPromoteChunk: one accumulator chunk a
+// tile, so moving C is the work (16384 x 16384 x 256, beta 0.5: 2.1 of 2.2 GB)
+// and no register accumulator is needed.  The epilogue warps read TMEM 64
+// columns at a time in a rolled loop, and a warp's first C block loads while
+// the tile's MMAs run.  Measured on B200 on that shape: 0.60 -> 0.50 ms alone,
+// 0.68 -> 0.58 ms back to back (both at the 1000 W power limit there), with
+// the sigmoid 0.88 -> 0.59 ms; beta = 0 unchanged.  16 epilogue warps with the
+// whole C tile staged leave three ring stages, which cost more on beta = 0
+// (0.47 ms against 0.43) than they gained on beta != 0 (0.54 against 0.52).
+struct Bf16x3PairDirect : TraitsBase<3, 256, 64, 2, 2, 1, false, EpiF32, false, 0, 8, 0, true, false, true> {
   static constexpr TermTable<3> kTerms{{1, 0, 0}, {0, 1, 0}, {0, 0, 0}, {true, false, false}};
 };
 struct Bf16x3Pair128 : TraitsBase<3, 128, 64, 2, 2, 1, false, EpiF32, true, kPromoteChunk, 8, 0, true> {
