@@ -11,8 +11,11 @@
 //       B-planes = rows of B itself (B^T's K-major layout is B);
 //   dB: A-planes = columns of A (A^T, transposing split),
 //       B-planes = columns of G (G^T, transposing split, G computed again).
-// Six launches (four splits, two GEMMs), one caller workspace reused by both
-// products in stream order.
+// Three launches: every plane in one split kernel (G is formed once and
+// written in both layouts), then the two GEMMs, each product with its own
+// part of the caller's workspace.  A workspace that holds only the larger
+// product (half of what the query asks for) runs one product after the
+// other in it.
 #include <algorithm>
 
 #include "../../include/cucosma.h"
@@ -39,6 +42,8 @@ void sub_desc(const cucosma_gemm_desc* f, int64_t m, int64_t n, int64_t k, int64
   d->alpha = 1.0;
   d->beta = 0.0;
 }
+
+size_t part_bytes(size_t b) { return (b + 255) & ~size_t(255); }
 
 int xform_of(int epilogue) {
   return epilogue == CUCOSMA_EPILOGUE_SIGMOID ? kXformSigmoidGrad
@@ -70,14 +75,15 @@ extern "C" cucosma_status cucosma_gemm_backward_workspace_size(const cucosma_gem
   if (!di) return CUCOSMA_STATUS_LAUNCH_FAILED;
   // Each product's plan as the backward call builds it: tuned, and with its
   // planes prepared here (never the fused-split kernel, which keeps none).
+  // The planes of both exist at once, one part after the other.
   auto need = [&](int64_t m, int64_t n, int64_t k, int64_t ldc) {
     cucosma_gemm_desc d0, tuned;
     cucosma_plan_info pi;
     sub_desc(f, m, n, k, ldc, &d0);
     tc_plan_info(apply_tuning(&d0, &tuned, di), di, &pi, false);
-    return pi.workspace_bytes;
+    return part_bytes(pi.workspace_bytes);
   };
-  *bytes = std::max(need(f->m, f->k, f->n, f->k), need(f->k, f->n, f->m, f->n));
+  *bytes = need(f->m, f->k, f->n, f->k) + need(f->k, f->n, f->m, f->n);
   return CUCOSMA_STATUS_SUCCESS;
 }
 
@@ -99,9 +105,7 @@ extern "C" cucosma_status cucosma_gemm_backward(const cucosma_gemm_desc* f, cons
   const DeviceInfo* di = device_info();
   if (!di) return CUCOSMA_STATUS_LAUNCH_FAILED;
   if (di->cc_major != 10 || di->cc_minor != 0) return CUCOSMA_STATUS_ARCH_MISMATCH;
-  size_t need = 0;
-  if ((s = cucosma_gemm_backward_workspace_size(f, &need)) != CUCOSMA_STATUS_SUCCESS) return s;
-  if (!workspace || workspace_bytes < need) return CUCOSMA_STATUS_WORKSPACE_TOO_SMALL;
+  if (!workspace) return CUCOSMA_STATUS_WORKSPACE_TOO_SMALL;
   if (!al16(workspace)) return CUCOSMA_STATUS_MISALIGNED;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   uint8_t* w = static_cast<uint8_t*>(workspace);
@@ -110,43 +114,50 @@ extern "C" cucosma_status cucosma_gemm_backward(const cucosma_gemm_desc* f, cons
   const float scale = (float)f->alpha;
   const float* fY = static_cast<const float*>(Y);
   const float* fdY = static_cast<const float*>(dY);
-  cucosma_plan_info pi;
   // Each product's descriptor is resolved against the tuning cache once and
   // that one descriptor gives both the plan (plane offsets, partials region)
-  // and the launch, so the two cannot disagree; the plan must fit the
+  // and the launch, so the two cannot disagree; the plans must fit the
   // caller's workspace (the cache may have changed since it was sized).
-  auto resolve = [&](cucosma_gemm_desc* d, cucosma_gemm_desc* tuned) -> const cucosma_gemm_desc* {
-    const cucosma_gemm_desc* r = apply_tuning(d, tuned, di);
-    tc_plan_info(r, di, &pi, false);  // the planes are prepared here: never the fused kernel
-    return r;
+  struct Product {
+    cucosma_gemm_desc d0, tuned;
+    const cucosma_gemm_desc* d = nullptr;
+    cucosma_plan_info pi;
+    uint8_t* w = nullptr;
+    size_t bytes = 0;  // its part of the workspace
+  } pa, pb;
+  auto resolve = [&](Product& p, int64_t pm, int64_t pn, int64_t pk, int64_t ldc) {
+    sub_desc(f, pm, pn, pk, ldc, &p.d0);
+    p.d = apply_tuning(&p.d0, &p.tuned, di);
+    tc_plan_info(p.d, di, &p.pi, false);  // the planes are prepared here: never the fused kernel
+    p.w = w;
+    p.bytes = part_bytes(p.pi.workspace_bytes);
   };
-  if (dA) {
-    // dA (m x k) = G (m x n) * B^T: K' = n.
-    cucosma_gemm_desc d0, tuned;
-    sub_desc(f, m, k, n, ldda, &d0);
-    const cucosma_gemm_desc* d = resolve(&d0, &tuned);
-    if (pi.workspace_bytes > workspace_bytes) return CUCOSMA_STATUS_WORKSPACE_TOO_SMALL;
-    if (launch_split_bf16(fdY, lddy, (int)m, (int)n, pi.kpad, nt, w + pi.off_a, false, di->sms, st, xf, fY, ldy,
-                          scale) != cudaSuccess ||
-        launch_split_bf16(static_cast<const float*>(B), f->ldb, (int)k, (int)n, pi.kpad, nt, w + pi.off_b, false,
-                          di->sms, st) != cudaSuccess)
-      return CUCOSMA_STATUS_LAUNCH_FAILED;
-    note_launches(2);
-    if ((s = tc_gemm_ex(d, nullptr, nullptr, dA, workspace, workspace_bytes, di, st, 0)) != CUCOSMA_STATUS_SUCCESS) return s;
+  resolve(pa, m, k, n, ldda);  // dA (m x k) = G (m x n) * B^T: K' = n
+  resolve(pb, k, n, m, lddb);  // dB (k x n) = A^T (k x m) * G (m x n): K' = m
+  // (both, whichever gradients are asked for, as the query does)
+  if (std::max(pa.pi.workspace_bytes, pb.pi.workspace_bytes) > workspace_bytes) return CUCOSMA_STATUS_WORKSPACE_TOO_SMALL;
+  auto run = [&](bool da, bool db) -> cucosma_status {
+    SplitJobs jobs{};
+    SplitJob& g = jobs.add(fdY, lddy, (int)m, (int)n, da ? pa.w + pa.pi.off_a : nullptr, da ? pa.pi.kpad : 0,
+                           db ? pb.w + pb.pi.off_b : nullptr, db ? pb.pi.kpad : 0);
+    g.mode = xf;
+    g.scale = scale;
+    g.Y = f->epilogue != CUCOSMA_EPILOGUE_NONE ? fY : nullptr;
+    g.ldy = ldy;
+    if (da) jobs.rows(static_cast<const float*>(B), f->ldb, (int)k, (int)n, pa.w + pa.pi.off_b, pa.pi.kpad);
+    if (db) jobs.cols(static_cast<const float*>(A), f->lda, (int)m, (int)k, pb.w + pb.pi.off_a, pb.pi.kpad);
+    if (launch_split_bf16(jobs, nt, st) != cudaSuccess) return CUCOSMA_STATUS_LAUNCH_FAILED;
+    note_launches(1);
+    cucosma_status e = CUCOSMA_STATUS_SUCCESS;
+    if (da) e = tc_gemm_ex(pa.d, nullptr, nullptr, dA, pa.w, workspace_bytes - (size_t)(pa.w - w), di, st, 0);
+    if (db && e == CUCOSMA_STATUS_SUCCESS)
+      e = tc_gemm_ex(pb.d, nullptr, nullptr, dB, pb.w, workspace_bytes - (size_t)(pb.w - w), di, st, 0);
+    return e;
+  };
+  if (dA && dB && pa.bytes + pb.pi.workspace_bytes > workspace_bytes) {
+    if ((s = run(true, false)) != CUCOSMA_STATUS_SUCCESS) return s;
+    return run(false, true);
   }
-  if (dB) {
-    // dB (k x n) = A^T (k x m) * G (m x n): K' = m.
-    cucosma_gemm_desc d0, tuned;
-    sub_desc(f, k, n, m, lddb, &d0);
-    const cucosma_gemm_desc* d = resolve(&d0, &tuned);
-    if (pi.workspace_bytes > workspace_bytes) return CUCOSMA_STATUS_WORKSPACE_TOO_SMALL;
-    if (launch_split_bf16(static_cast<const float*>(A), f->lda, (int)m, (int)k, pi.kpad, nt, w + pi.off_a, true,
-                          di->sms, st) != cudaSuccess ||
-        launch_split_bf16(fdY, lddy, (int)m, (int)n, pi.kpad, nt, w + pi.off_b, true, di->sms, st, xf, fY, ldy,
-                          scale) != cudaSuccess)
-      return CUCOSMA_STATUS_LAUNCH_FAILED;
-    note_launches(2);
-    if ((s = tc_gemm_ex(d, nullptr, nullptr, dB, workspace, workspace_bytes, di, st, 0)) != CUCOSMA_STATUS_SUCCESS) return s;
-  }
-  return CUCOSMA_STATUS_SUCCESS;
+  if (dA && dB) pb.w = w + pa.bytes;
+  return run(dA != nullptr, dB != nullptr);
 }

@@ -34,107 +34,154 @@ __device__ __forceinline__ void load8(const float* __restrict__ src, int c, int 
   }
 }
 
-// A: rows x cols (ld elements) -> planes [NT][rows][kpad], same layout.
-// Rows stride over grid.y, 8-column groups over grid.x; each thread converts
-// 8 consecutive columns (two 16-byte loads, one 16-byte store per plane).
-// Columns cols..kpad-1 are written as 0 (kpad % 8 == 0).
-template <int MODE, int NT>
-__global__ void __launch_bounds__(256)
-    split_bf16_rows_kernel(const float* __restrict__ A, int64_t lda, int rows, int cols, int64_t kpad,
-                           __nv_bfloat16* __restrict__ out, const float* __restrict__ Y, int64_t ldy, float scale) {
-  const int ng = (int)(kpad / 8);
-  const int64_t plane = (int64_t)rows * kpad;
-  for (int r = blockIdx.y; r < rows; r += gridDim.y) {
-    const float* srow = A + (int64_t)r * lda;
-    __nv_bfloat16* drow = out + (int64_t)r * kpad;
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ng; g += gridDim.x * blockDim.x) {
-      const int c = g * 8;
-      float v[8];
-      load8(srow, c, cols, v);
-      if constexpr (MODE != kXformNone) {
+// NT planes of 8 values: one 16-byte store each.
+template <int NT>
+__device__ __forceinline__ void store_planes8(__nv_bfloat16* dst, int64_t plane, const float (&v)[8]) {
+  uint32_t pk[4][NT];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) split_bf16x2_n<NT>(v[2 * e], v[2 * e + 1], pk[e]);
+#pragma unroll
+  for (int i = 0; i < NT; ++i)
+    *reinterpret_cast<uint4*>(dst + i * plane) = make_uint4(pk[0][i], pk[1][i], pk[2][i], pk[3][i]);
+}
+
+__device__ __forceinline__ float xform_rt(int mode, float v, float y, float scale) {
+  switch (mode) {
+    case kXformScale: return xform<kXformScale>(v, y, scale);
+    case kXformSigmoidGrad: return xform<kXformSigmoidGrad>(v, y, scale);
+    case kXformReluGrad: return xform<kXformReluGrad>(v, y, scale);
+    default: return v;
+  }
+}
+
+// Row planes [NT][rows][kpad] of a source in its own layout: one warp per
+// unit of up to 2048 columns of a row, lanes over 8-column groups (two
+// 16-byte loads, one 16-byte store per plane), two groups in flight.
+// Columns cols .. kpad-1 are written as 0 (kpad % 8 == 0).
+constexpr int kRowUnit = 256;  // 8-column groups per warp
+template <int NT>
+__device__ __forceinline__ void split_rows_unit(const SplitJob& j, int64_t unit) {
+  const int lane = threadIdx.x & 31;
+  const int ng = (int)(j.kpad_r / 8), upr = (ng + kRowUnit - 1) / kRowUnit;
+  const int64_t r = unit / upr;
+  if (r >= j.rows) return;
+  const int g0 = (int)(unit - r * upr) * kRowUnit, g1 = min(ng, g0 + kRowUnit);
+  const float* srow = j.src + r * j.ld;
+  const float* yrow = j.Y + r * j.ldy;
+  __nv_bfloat16* drow = j.out_r + r * j.kpad_r;
+  const int64_t plane = (int64_t)j.rows * j.kpad_r;
+  constexpr int U = 2;
+  for (int g = g0 + lane; g < g1; g += 32 * U) {
+    float v[U][8];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (g + 32 * u < g1) load8(srow, (g + 32 * u) * 8, j.cols, v[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (g + 32 * u >= g1) break;
+      const int c = (g + 32 * u) * 8;
+      if (j.mode != kXformNone) {
         float y[8];
-        load8(Y + (int64_t)r * ldy, c, cols, y);
+        if (j.Y != nullptr) {
+          load8(yrow, c, j.cols, y);
+        } else {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = xform<MODE>(v[e], y[e], scale);
+          for (int e = 0; e < 8; ++e) y[e] = 0.f;
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[u][e] = xform_rt(j.mode, v[u][e], y[e], j.scale);
       }
-      uint32_t pk[NT][4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        __nv_bfloat16 t0[NT], t1[NT];
-        split_bf16_n<NT>(v[2 * e], t0);
-        split_bf16_n<NT>(v[2 * e + 1], t1);
-#pragma unroll
-        for (int i = 0; i < NT; ++i) pk[i][e] = pack_bf16x2(t0[i], t1[i]);
-      }
-#pragma unroll
-      for (int i = 0; i < NT; ++i)
-        *reinterpret_cast<uint4*>(drow + i * plane + c) = make_uint4(pk[i][0], pk[i][1], pk[i][2], pk[i][3]);
+      store_planes8<NT>(drow + c, plane, v[u]);
     }
   }
 }
 
-// B: K x N (ld elements) -> planes [NT][N][kpad] (transposed), through a
-// 64 (k) x 64 (n) shared-memory tile; 256 threads.  Loads: 16 lanes cover a
-// 256-byte row of B (float4 each).  Stores: a lane converts 4 consecutive k
-// of one output row (8 bytes per plane), so 16 lanes write 128 contiguous
-// bytes per plane.
-template <int MODE, int NT>
-__global__ void __launch_bounds__(256)
-    split_bf16_cols_kernel(const float* __restrict__ B, int64_t ldb, int krows, int ncols, int64_t kpad,
-                           __nv_bfloat16* __restrict__ out, const float* __restrict__ Y, int64_t ldy, float scale) {
-  __shared__ float tile[64][65];
-  const int k0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  const int64_t plane = (int64_t)ncols * kpad;
-  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;  // 16 x 16
-#pragma unroll
-  for (int i = ty; i < 64; i += 16) {
-    const int k = k0 + i, n = n0 + 4 * tx;
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
-    if (k < krows) {
-      const float* src = B + (int64_t)k * ldb + n;
-      if (n + 4 <= ncols) {
-        const float4 q = *reinterpret_cast<const float4*>(src);  // n % 4 == 0, ldb % 4 == 0
-        v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) v[e] = n + e < ncols ? src[e] : 0.f;
-      }
-      if constexpr (MODE != kXformNone) {
-        const float* ysrc = Y + (int64_t)k * ldy + n;
-        float y[4] = {0.f, 0.f, 0.f, 0.f};
-        if (n + 4 <= ncols) {
-          const float4 q = *reinterpret_cast<const float4*>(ysrc);
-          y[0] = q.x, y[1] = q.y, y[2] = q.z, y[3] = q.w;
-        } else {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) y[e] = n + e < ncols ? ysrc[e] : 0.f;
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) v[e] = xform<MODE>(v[e], y[e], scale);
-      }
+// One 64 (source rows) x 64 (columns) tile of a source to transposed planes
+// [NT][cols][kpad_c] and, for out_r, to row planes as well (the backward
+// pass's G, needed in both layouts, is read and formed once).  Loads: 16 lanes
+// cover a 256-byte row (float4 each) and write it to shared memory with the
+// 16-byte chunk c of row k at c ^ (k / 8); then a lane converts 8 consecutive
+// k of one column (8 lanes x 4 columns a warp: no bank conflicts, 128
+// contiguous bytes per column and plane).
+template <int NT>
+__device__ __forceinline__ void split_cols_tile(const SplitJob& j, int tk, int tn, float* tile) {
+  const int k0 = tk * 64, n0 = tn * 64;
+  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
+  // columns n .. n + 3 of a row (n % 4 == 0, 16-byte rows), zero past cols
+  auto load4 = [&](const float* row, int n) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (n + 4 <= j.cols) {
+      v = *reinterpret_cast<const float4*>(row + n);
+    } else {
+      if (n < j.cols) v.x = row[n];
+      if (n + 1 < j.cols) v.y = row[n + 1];
+      if (n + 2 < j.cols) v.z = row[n + 2];
     }
+    return v;
+  };
+  const int n = n0 + 4 * tx;
+  const bool use_y = j.mode != kXformNone && j.Y != nullptr;
+  float4 q[4], y[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) tile[i][4 * tx + e] = v[e];
+  for (int p = 0; p < 4; ++p) {  // every load of the tile in flight at once
+    const int k = k0 + ty + 16 * p;
+    q[p] = k < j.rows ? load4(j.src + (int64_t)k * j.ld, n) : make_float4(0.f, 0.f, 0.f, 0.f);
+    y[p] = use_y && k < j.rows ? load4(j.Y + (int64_t)k * j.ldy, n) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const int k = k0 + ty + 16 * p;
+    if (j.mode != kXformNone) {
+      q[p].x = xform_rt(j.mode, q[p].x, y[p].x, j.scale);
+      q[p].y = xform_rt(j.mode, q[p].y, y[p].y, j.scale);
+      q[p].z = xform_rt(j.mode, q[p].z, y[p].z, j.scale);
+      q[p].w = xform_rt(j.mode, q[p].w, y[p].w, j.scale);
+    }
+    const int i = ty + 16 * p;
+    *reinterpret_cast<float4*>(tile + i * 64 + ((tx ^ (i >> 3)) << 2)) = q[p];
+    if (j.out_r != nullptr && k < j.rows && n < j.kpad_r) {  // kpad_r % 8 == 0: n + 3 < kpad_r as well
+      uint32_t lo[NT], hi[NT];
+      split_bf16x2_n<NT>(q[p].x, q[p].y, lo);
+      split_bf16x2_n<NT>(q[p].z, q[p].w, hi);
+      __nv_bfloat16* dst = j.out_r + (int64_t)k * j.kpad_r + n;
+      const int64_t plane = (int64_t)j.rows * j.kpad_r;
+#pragma unroll
+      for (int i2 = 0; i2 < NT; ++i2) *reinterpret_cast<uint2*>(dst + i2 * plane) = make_uint2(lo[i2], hi[i2]);
+    }
   }
   __syncthreads();
-  const int k = k0 + 4 * tx;
+  const int lane = t & 31, kq = lane & 7;
+  const int64_t plane = (int64_t)j.cols * j.kpad_c;
 #pragma unroll
-  for (int i = ty; i < 64; i += 16) {
-    const int n = n0 + i;
-    if (n < ncols && k < kpad) {  // kpad % 8 == 0, so k + 3 < kpad as well
-      uint32_t pk[NT][2];
+  for (int h = 0; h < 2; ++h) {
+    const int nl = (t >> 5) * 8 + h * 4 + (lane >> 3), k = k0 + 8 * kq;
+    if (n0 + nl < j.cols && k < j.kpad_c) {  // kpad_c % 8 == 0: k + 7 < kpad_c as well
+      float v[8];
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        __nv_bfloat16 t0[NT], t1[NT];
-        split_bf16_n<NT>(tile[4 * tx + 2 * e][i], t0);
-        split_bf16_n<NT>(tile[4 * tx + 2 * e + 1][i], t1);
-#pragma unroll
-        for (int j = 0; j < NT; ++j) pk[j][e] = pack_bf16x2(t0[j], t1[j]);
-      }
-      __nv_bfloat16* dst = out + (int64_t)n * kpad + k;
-#pragma unroll
-      for (int j = 0; j < NT; ++j) *reinterpret_cast<uint2*>(dst + j * plane) = make_uint2(pk[j][0], pk[j][1]);
+      for (int e = 0; e < 8; ++e) v[e] = tile[(8 * kq + e) * 64 + (((nl >> 2) ^ kq) << 2) + (nl & 3)];
+      store_planes8<NT>(j.out_c + (int64_t)(n0 + nl) * j.kpad_c + k, plane, v);
     }
+  }
+}
+
+// Every split a call needs in one launch (A and B of a GEMM; G, B and A of a
+// backward pass): the blocks of the jobs follow one another.  HBM-bound at
+// large sizes, launch-bound at small ones.  64 registers, so that four blocks
+// an SM keep their loads in flight; a tile's loads (and Y's) are all issued
+// before the first is used.  B200, against one launch per operand: 8192 x
+// 8192 A and B to three planes 219 -> 208 us (6.4 TB/s), 4096 x 4096 to two
+// 44.4 -> 40.5, 1234 x 777 and 777 x 1111 6.3 -> 4.2 and one launch less; the
+// backward pass's four splits at 4096^3, two planes, sigmoid, 110 -> 84 us.
+template <int NT>
+__global__ void __launch_bounds__(256, 4) split_bf16_kernel(const __grid_constant__ SplitJobs jobs) {
+  __shared__ __align__(16) float tile[64 * 64];
+  int b = blockIdx.x, ji = 0;
+  while (ji + 1 < jobs.count && b >= jobs.job[ji].blocks) b -= jobs.job[ji++].blocks;
+  const SplitJob& j = jobs.job[ji];
+  if (j.out_c == nullptr) {
+    split_rows_unit<NT>(j, (int64_t)b * 8 + (threadIdx.x >> 5));
+  } else {
+    split_cols_tile<NT>(j, b / j.tiles_n, b % j.tiles_n, tile);
   }
 }
 
@@ -459,40 +506,25 @@ static unsigned grid_for(int64_t work, int threads, int sms) {
   return (unsigned)std::max<int64_t>(b, 1);
 }
 
-template <int MODE, int NT>
-static void split_bf16_launch_nt(const float* A, int64_t lda, int rows, int cols, int64_t kpad, void* out,
-                                 bool transpose, int sms, cudaStream_t st, const float* Y, int64_t ldy, float scale) {
-  if (!transpose) {
-    const int64_t gx = std::max<int64_t>(1, std::min<int64_t>(ceil_div(kpad / 8, 256), 16));
-    const int64_t gy = std::max<int64_t>(1, std::min<int64_t>({(int64_t)rows, (int64_t)sms * 16 / gx, 65535}));
-    split_bf16_rows_kernel<MODE, NT><<<dim3((unsigned)gx, (unsigned)gy), 256, 0, st>>>(
-        A, lda, rows, cols, kpad, static_cast<__nv_bfloat16*>(out), Y, ldy, scale);
-  } else {
-    // A is K x N here (krows = rows, ncols = cols); output N x kpad.
-    dim3 grid((unsigned)ceil_div(cols, 64), (unsigned)ceil_div(kpad, 64));
-    split_bf16_cols_kernel<MODE, NT><<<grid, 256, 0, st>>>(A, lda, rows, cols, kpad,
-                                                          static_cast<__nv_bfloat16*>(out), Y, ldy, scale);
+cudaError_t launch_split_bf16(SplitJobs& jobs, int nterms, cudaStream_t st) {
+  int64_t total = 0;
+  for (int i = 0; i < jobs.count; ++i) {
+    SplitJob& j = jobs.job[i];
+    int64_t blocks;
+    if (j.out_c == nullptr) {
+      blocks = ceil_div((int64_t)j.rows * ceil_div(j.kpad_r / 8, kRowUnit), 8);
+    } else {
+      j.tiles_n = (int)ceil_div(j.cols, 64);
+      blocks = ceil_div(j.kpad_c, 64) * j.tiles_n;
+    }
+    total += blocks;
+    if (total > INT32_MAX) return cudaErrorInvalidValue;
+    j.blocks = (int)blocks;
   }
-}
-template <int MODE>
-static void split_bf16_launch(const float* A, int64_t lda, int rows, int cols, int64_t kpad, int nterms, void* out,
-                              bool transpose, int sms, cudaStream_t st, const float* Y, int64_t ldy, float scale) {
   if (nterms == 3)
-    split_bf16_launch_nt<MODE, 3>(A, lda, rows, cols, kpad, out, transpose, sms, st, Y, ldy, scale);
+    split_bf16_kernel<3><<<(unsigned)total, 256, 0, st>>>(jobs);
   else
-    split_bf16_launch_nt<MODE, 2>(A, lda, rows, cols, kpad, out, transpose, sms, st, Y, ldy, scale);
-}
-
-cudaError_t launch_split_bf16(const float* A, int64_t lda, int rows, int cols, int64_t kpad, int nterms, void* out,
-                              bool transpose, int sms, cudaStream_t st, int xform, const float* Y, int64_t ldy,
-                              float scale) {
-  switch (xform) {
-    case kXformNone: split_bf16_launch<kXformNone>(A, lda, rows, cols, kpad, nterms, out, transpose, sms, st, Y, ldy, scale); break;
-    case kXformScale: split_bf16_launch<kXformScale>(A, lda, rows, cols, kpad, nterms, out, transpose, sms, st, Y, ldy, scale); break;
-    case kXformSigmoidGrad: split_bf16_launch<kXformSigmoidGrad>(A, lda, rows, cols, kpad, nterms, out, transpose, sms, st, Y, ldy, scale); break;
-    case kXformReluGrad: split_bf16_launch<kXformReluGrad>(A, lda, rows, cols, kpad, nterms, out, transpose, sms, st, Y, ldy, scale); break;
-    default: return cudaErrorInvalidValue;
-  }
+    split_bf16_kernel<2><<<(unsigned)total, 256, 0, st>>>(jobs);
   return cudaGetLastError();
 }
 

@@ -3,25 +3,64 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include "common.cuh"
 
 namespace cucosma {
 
-// FP32 rows x cols -> nterms BF16 planes.  transpose = false: planes are
-// [nterms][rows][kpad] (A operand, cols = K).  transpose = true: the input is
-// K x N (rows = K, cols = N) and planes are [nterms][N][kpad] (B operand).
+// BF16 split of FP32 sources (rows x cols, row stride ld) into nterms planes.
+// out_r: planes [nterms][rows][kpad_r] in the source's layout (K = cols);
+// out_c: planes [nterms][cols][kpad_c], transposed (K = rows); either or both.
 //
-// xform (backward pass): the value split is not A[i] but
-//   kXformScale:        scale * A[i]
-//   kXformSigmoidGrad:  scale * A[i] * Y[i] * (1 - Y[i])   (A = dY, Y = sigmoid output)
-//   kXformReluGrad:     Y[i] > 0 ? scale * A[i] : 0        (Y = ReLU output)
-// with Y read at the same (row, column) as A (row stride ldy).
+// mode (backward pass): the value split is not src[i] but
+//   kXformScale:        scale * src[i]
+//   kXformSigmoidGrad:  scale * src[i] * Y[i] * (1 - Y[i])   (src = dY, Y = sigmoid output)
+//   kXformReluGrad:     Y[i] > 0 ? scale * src[i] : 0        (Y = ReLU output)
+// with Y read at the same (row, column) as src (row stride ldy).
 enum SplitXform : int { kXformNone = 0, kXformScale = 1, kXformSigmoidGrad = 2, kXformReluGrad = 3 };
-cudaError_t launch_split_bf16(const float* A, int64_t lda, int rows, int cols, int64_t kpad, int nterms, void* out,
-                              bool transpose, int sms, cudaStream_t st, int xform = kXformNone,
-                              const float* Y = nullptr, int64_t ldy = 0, float scale = 1.0f);
+struct SplitJob {
+  const float* src;
+  int64_t ld;
+  int rows, cols;
+  __nv_bfloat16* out_r;
+  int64_t kpad_r;
+  __nv_bfloat16* out_c;
+  int64_t kpad_c;
+  int mode;
+  float scale;
+  const float* Y;
+  int64_t ldy;
+  int blocks, tiles_n;  // set by the launcher
+};
+struct SplitJobs {
+  SplitJob job[3];
+  int count;
+  // Planes in the source's layout (an A operand), and transposed (a B operand).
+  void rows(const float* src, int64_t ld, int nrows, int ncols, void* out, int64_t kpad) {
+    add(src, ld, nrows, ncols, out, kpad, nullptr, 0);
+  }
+  void cols(const float* src, int64_t ld, int nrows, int ncols, void* out, int64_t kpad) {
+    add(src, ld, nrows, ncols, nullptr, 0, out, kpad);
+  }
+  SplitJob& add(const float* src, int64_t ld, int nrows, int ncols, void* out_r, int64_t kpad_r, void* out_c,
+                int64_t kpad_c) {
+    SplitJob& j = job[count++];
+    j = SplitJob{};
+    j.src = src;
+    j.ld = ld;
+    j.rows = nrows;
+    j.cols = ncols;
+    j.out_r = static_cast<__nv_bfloat16*>(out_r);
+    j.kpad_r = kpad_r;
+    j.out_c = static_cast<__nv_bfloat16*>(out_c);
+    j.kpad_c = kpad_c;
+    return j;
+  }
+};
+// All jobs in one launch (count >= 1).
+cudaError_t launch_split_bf16(SplitJobs& jobs, int nterms, cudaStream_t st);
 
 // Statistics of the adaptive Ozaki path (slice count or native FP64 chosen
 // on the device from the operands), kept in the workspace.  The magnitude

@@ -232,7 +232,7 @@ static bool one_chunk(const Tiling& t) { return t.splits == 1 && t.kblocks <= kP
 
 static int plan_launches(const Plan& pl) {
   if (pl.fused) return 1 + (pl.t.splits > 1 ? 1 : 0);
-  if (pl.kind != 2) return 3 + (pl.t.splits > 1 ? 1 : 0);
+  if (pl.kind != 2) return 2 + (pl.t.splits > 1 ? 1 : 0);  // the split of A and B, the GEMM
   if (!pl.adaptive) return 4 + (pl.t.splits > 1 ? 1 : 0);
   // prep B (2), prep A, decision, the three gated kernels and their reductions
   return 7 + (pl.t.splits > 1) + (pl.t9.splits > 1) + (pl.native.splits > 1);
@@ -429,12 +429,11 @@ cucosma_status tc_gemm_ex(const cucosma_gemm_desc* d, const void* A, const void*
     }
   } else if (pl.kind != 2) {
     const int nt = pl.t.slices;
-    if (prep & kPrepA) {
-      e = launch_split_bf16((const float*)A, d->lda, m, k, pl.kpad, nt, w + pl.off_a, false, di->sms, st);
-      launches += 1;
-    }
-    if (e == cudaSuccess && (prep & kPrepB)) {
-      e = launch_split_bf16((const float*)B, d->ldb, k, n, pl.kpad, nt, w + pl.off_b, true, di->sms, st);
+    SplitJobs jobs{};
+    if (prep & kPrepA) jobs.rows((const float*)A, d->lda, m, k, w + pl.off_a, pl.kpad);
+    if (prep & kPrepB) jobs.cols((const float*)B, d->ldb, k, n, w + pl.off_b, pl.kpad);
+    if (jobs.count > 0) {
+      e = launch_split_bf16(jobs, nt, st);
       launches += 1;
     }
     if (e != cudaSuccess) return CUCOSMA_STATUS_LAUNCH_FAILED;
