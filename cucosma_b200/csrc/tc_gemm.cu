@@ -71,7 +71,9 @@ struct Plan {
 
 static size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
-static Tiling make_tiling(const Plan& pl, int slices, int bn, const cucosma_gemm_desc* d, const DeviceInfo* di) {
+// split_k: 0 = chosen here, >= 1 as given (by the caller or the time model).
+static Tiling make_tiling(const Plan& pl, int slices, int bn, const cucosma_gemm_desc* d, int64_t split_k,
+                          const DeviceInfo* di) {
   Tiling t{};
   const int64_t M = d->m, N = d->n, K = d->k;
   t.slices = slices;
@@ -88,14 +90,14 @@ static Tiling make_tiling(const Plan& pl, int slices, int bn, const cucosma_gemm
     kbmax = ((int64_t)2147483647 / ((int64_t)slices * 127 * 127)) / pl.bk;
     min_splits = ceil_div(t.kblocks, kbmax);
   }
-  int64_t splits = d->split_k > 0 ? d->split_k : 1;
-  if (d->split_k <= 0 && tiles < slots) splits = std::max<int64_t>(1, std::min<int64_t>(slots / tiles, t.kblocks / 16));
+  int64_t splits = split_k > 0 ? split_k : 1;
+  if (split_k <= 0 && tiles < slots) splits = std::max<int64_t>(1, std::min<int64_t>(slots / tiles, t.kblocks / 16));
   splits = std::max(splits, min_splits);
   // More splits than one wave of units (the Ozaki exactness bound on long
   // K): as many splits as the same number of waves holds, so that the last
   // wave is full and every unit is shorter (256 x 256 x 1,048,576 at 8
   // slices: 64 splits x 8 tiles = 3.5 waves of 148; 74 splits fill 4).
-  if (d->split_k <= 0 && splits > 1 && tiles * splits > slots) {
+  if (split_k <= 0 && splits > 1 && tiles * splits > slots) {
     const int64_t waves = ceil_div(tiles * splits, (int64_t)slots);
     splits = std::max(splits, waves * slots / tiles);
   }
@@ -109,26 +111,92 @@ static Tiling make_tiling(const Plan& pl, int slices, int bn, const cucosma_gemm
   return t;
 }
 
-// The fused split pays off when the separate pre-pass (read the FP32
+// Operands beyond L2: the fused split pays off when the separate pre-pass (read the FP32
 // operands, write nt BF16 planes) would take more than a quarter of the
 // GEMM's own bound (tensor time at nt products of BF16, or the HBM time of
 // reading the planes and writing -- with beta, also reading -- C): operands
 // read only a few times, as in the large-K and large-N families (measured on
 // B200, beta 0.5, BF16x3 / BF16x6: 256 x 256 x 1,048,576 0.58 / 0.88 ms fused
 // against about 1.2 / 2.6 ms; 256 x 1,048,576 x 256 0.85 / 1.06 against 1.23
-// / 1.19 ms), and not where small operands are re-read by many tiles (16384 x
-// 16384 x 256, BF16x6: 1.01 fused against 0.70 ms with the pre-pass, whose
-// cost there is negligible).
+// / 1.19 ms), and not where operands are re-read by many tiles.
 static bool fused_pays(const cucosma_gemm_desc* d, int nt) {
   const double M = (double)d->m, N = (double)d->n, K = (double)d->k;
   const double hbm = 6.5e12, bf16 = 1.6e15;
   const double products = nt == 2 ? 3.0 : 6.0;
-  const double c_bytes = M * N * 4.0 * (d->beta != 0.0 ? 2.0 : 1.0), ab_bytes = (M * K + K * N) * 4.0;
-  if (ab_bytes < 32.0 * (1 << 20)) return false;  // small operands: the pre-pass costs microseconds
+  const double c_bytes = M * N * 4.0 * (d->beta != 0.0 ? 2.0 : 1.0);
   const double t_pre = (M * K + K * N) * (4.0 + 2.0 * nt) / hbm;
   const double t_mma = 2.0 * M * N * K * products / bf16;
   const double t_mem = ((M * K + K * N) * 2.0 * nt + c_bytes) / hbm;
   return t_pre > 0.25 * std::max(t_mma, t_mem);
+}
+
+// Modelled time (us) of one BF16 call: a tile per variant with
+//   f + (u * k-blocks of a unit + e) * waves   (waves: rho of the whole waves
+//   the units make on the CTAs or pairs, the rest of their plain ratio, since
+//   the last wave runs with less contention; single-CTA tiles lose a tenth
+//   more when they need several waves)
+//   + the pre-pass at 5.5 TB/s, C at 11 TB/s of stores (and loads) beside the
+//   MMAs, and per split-K call 3.1 us and the partials at 13.8 TB/s (L2).
+// Least squares over 2281 measured calls on B200 (60 shapes, 64 to 8192 a
+// side, operands that fit L2; every tile, 1 to 24 splits; CUDA graphs): rms
+// error 5 to 10 %.  On those shapes the model's choice takes 1.017 of the best
+// measured time (geometric mean) and 1/1.24 of the time of the rule it
+// replaced, which took the largest tile, split only below one wave with 16
+// k-blocks left, and fused from 32 MB (1234 x 1111 x 777 BF16x6: 38 us with 25
+// of 74 pairs at work, 25.5 on 128 x 128 tiles; 2048^3 BF16x3: 89 us fused, 48
+// with the pre-pass).
+struct TileModel {
+  int variant, tile_m, bn, fused;
+  double f, u, e, rho;
+};
+constexpr TileModel kModelV3[] = {{kV3Small, 128, 128, 0, 6.5, 0.41, 2.2, 0.8},
+                                  {kV3Pair, 256, 256, 0, 5.8, 0.43, 8.5, 0.76},
+                                  {kV3Fused, 256, 128, 1, 5.6, 0.60, 2.5, 0.9}};
+constexpr TileModel kModelV3Direct = {kV3Pair, 256, 256, 0, 9.3, 0.40, 2.6, 1.0};  // one accumulator chunk
+constexpr TileModel kModelV6[] = {{kV6Single, 128, 128, 0, 7.2, 0.64, 1.8, 0.8},
+                                  {kV6Pair, 256, 128, 0, 7.6, 0.60, 1.7, 0.8},
+                                  {kV6PairWide, 256, 256, 0, 8.1, 1.01, 3.6, 0.92},
+                                  {kV6Fused, 256, 128, 1, 5.8, 0.90, 2.1, 0.92}};
+
+// The (tile, splits) with the smallest modelled time; forced > 0 fixes the splits.
+static void choose_bf16(const cucosma_gemm_desc* d, int kind, const DeviceInfo* di, bool allow_fused, int& variant,
+                        int64_t& splits) {
+  const double M = (double)d->m, N = (double)d->n, K = (double)d->k;
+  const int64_t kblocks = ceil_div(d->k, 32);
+  const TileModel* tm = kind == 1 ? kModelV6 : kModelV3;
+  const int count = kind == 1 ? 4 : 3;
+  const double t_pre = (M * K + K * N) * (kind == 1 ? 10.0 : 8.0) / 5.5e6;
+  const double t_c = M * N * 4.0 * (d->beta != 0.0 ? 2.0 : 1.0) / 11.4e6;
+  double best = 1e300;
+  for (int i = 0; i < count; ++i) {
+    if (tm[i].fused && !allow_fused) continue;
+    const bool pair = tm[i].tile_m == 256;
+    const int64_t tiles = std::max<int64_t>(1, ceil_div(d->m, tm[i].tile_m) * ceil_div(d->n, tm[i].bn));
+    const int64_t slots = pair ? di->sms / 2 : di->sms;
+    auto consider = [&](int64_t s) {
+      const TileModel& v = tm[i].variant == kV3Pair && s == 1 && kblocks <= kPromoteChunk ? kModelV3Direct : tm[i];
+      const double ratio = (double)(tiles * s) / (double)slots, waves = (double)ceil_div(tiles * s, slots);
+      double w = v.rho * waves + (1.0 - v.rho) * std::max(ratio, 1.0);
+      double t = v.f + (v.u * (double)ceil_div(kblocks, s) + v.e) * w * (!pair && waves > 1.0 ? 1.1 : 1.0);
+      if (!v.fused) t += t_pre;
+      if (s > 1) t += 3.1 + (double)s * M * N * 8.0 / 13.8e6;
+      if (t + t_c < best) {
+        best = t + t_c;
+        variant = v.variant;
+        splits = s;
+      }
+    };
+    if (d->split_k > 0) {
+      consider(std::min<int64_t>(d->split_k, kblocks));
+      continue;
+    }
+    consider(1);
+    // at least 4 k-blocks a split, at most two waves of units
+    const int64_t smax = std::min(kblocks / 4, 2 * slots / tiles);
+    for (int64_t s = 2; s <= smax; s += s < 8 ? 1 : s / 4) consider(s);
+    const int64_t full = std::min(smax, slots / tiles);  // one whole wave
+    if (full > 1) consider(full);
+  }
 }
 
 static Plan make_plan(const cucosma_gemm_desc* d, const DeviceInfo* di, bool allow_fused = true) {
@@ -136,6 +204,7 @@ static Plan make_plan(const cucosma_gemm_desc* d, const DeviceInfo* di, bool all
   allow_fused = allow_fused && d->flags == 0;  // the test hooks run the pre-pass path (as does its workspace query)
   const int64_t M = d->m, N = d->n, K = d->k;
   int slices = 0, bn = 0;
+  int64_t splits = d->split_k;
   pl.bk = 32;
   if (d->precision == CUCOSMA_PRECISION_OZAKI) {
     pl.kind = 2;
@@ -149,27 +218,29 @@ static Plan make_plan(const cucosma_gemm_desc* d, const DeviceInfo* di, bool all
     pl.kind = d->precision == CUCOSMA_PRECISION_BF16X6 ? 1 : 0;
     slices = pl.kind == 1 ? 3 : 2;
     pl.layout_slices = slices;
-    // Auto: CTA-pair tiles unless the problem has a single 128-row block.
-    const bool pair_ok = M > 128;
-    if (pl.kind == 0) {
-      switch (d->tile) {
-        case 1: pl.variant = kV3Wide; break;
-        case 2: pl.variant = kV3Small; break;
-        case 3: pl.variant = kV3Promoted; break;
-        case 4: pl.variant = kV3Pair; break;
-        case 5: pl.variant = allow_fused ? kV3Fused : kV3Pair; break;
-        default:
-          pl.variant = !pair_ok ? kV3Promoted : (allow_fused && fused_pays(d, 2)) ? kV3Fused : kV3Pair;
-      }
-    } else {
-      switch (d->tile) {
-        case 1: pl.variant = kV6Single; break;
-        case 2: pl.variant = kV6Pair; break;
-        case 3: pl.variant = kV6PairWide; break;
-        case 4: pl.variant = allow_fused ? kV6Fused : kV6Pair; break;
-        default:
-          pl.variant = !pair_ok ? kV6Single : (allow_fused && fused_pays(d, 3)) ? kV6Fused : kV6PairWide;
-      }
+    switch (d->tile) {
+      case 1: pl.variant = pl.kind == 0 ? kV3Wide : kV6Single; break;
+      case 2: pl.variant = pl.kind == 0 ? kV3Small : kV6Pair; break;
+      case 3: pl.variant = pl.kind == 0 ? kV3Promoted : kV6PairWide; break;
+      case 4: pl.variant = pl.kind == 0 ? kV3Pair : allow_fused ? kV6Fused : kV6Pair; break;
+      case 5:
+        if (pl.kind == 0) {
+          pl.variant = allow_fused ? kV3Fused : kV3Pair;
+          break;
+        }
+        [[fallthrough]];
+      default:
+        // Auto.  Operands that fit L2: the time model.  Larger ones: pair
+        // tiles (unless there is a single 128-row block), fused where the
+        // pre-pass's HBM traffic would show, splits by make_tiling.
+        if (((double)M * K + (double)K * N) * 4.0 <= (double)di->l2_bytes)
+          choose_bf16(d, pl.kind, di, allow_fused, pl.variant, splits);
+        else if (M <= 128)
+          pl.variant = pl.kind == 0 ? kV3Promoted : kV6Single;
+        else if (allow_fused && fused_pays(d, slices))
+          pl.variant = pl.kind == 0 ? kV3Fused : kV6Fused;
+        else
+          pl.variant = pl.kind == 0 ? kV3Pair : kV6PairWide;
     }
     bn = (pl.variant == kV3Small || pl.variant == kV6Single || pl.variant == kV6Pair || pl.variant == kV6Fused ||
           pl.variant == kV3Fused)
@@ -181,9 +252,9 @@ static Plan make_plan(const cucosma_gemm_desc* d, const DeviceInfo* di, bool all
   pl.pair = (pl.variant == kV3Pair || pl.variant == kV6Pair || pl.variant == kV6PairWide || pl.fused) ? 1 : 0;
   pl.tile_m = pl.pair ? 256 : 128;
   pl.bn_local = pl.pair ? bn / 2 : bn;
-  pl.t = make_tiling(pl, slices, bn, d, di);
+  pl.t = make_tiling(pl, slices, bn, d, splits, di);
   if (pl.adaptive) {
-    pl.t9 = make_tiling(pl, 9, ozaki_bn(9), d, di);
+    pl.t9 = make_tiling(pl, 9, ozaki_bn(9), d, splits, di);
     cucosma_gemm_desc nd = *d;
     nd.precision = CUCOSMA_PRECISION_NATIVE;
     nd.slices = 0;

@@ -1218,7 +1218,7 @@ struct Bf16x3 : TraitsBase<3, 256, 64, 2, 2, 1, false, EpiF32, true, kPromoteChu
 struct Bf16x3Wide : TraitsBase<3, 256, 64, 2, 2, 1, false, EpiF32> {
   static constexpr TermTable<3> kTerms{{1, 0, 0}, {0, 1, 0}, {0, 0, 0}, {true, false, false}};
 };
-struct Bf16x3Promoted : TraitsBase<3, 128, 64, 2, 2, 2, false, EpiF32, true, kPromoteChunk> {
+struct Bf16x3Promoted : TraitsBase<3, 128, 64, 2, 2, 2, false, EpiF32, true, kPromoteChunk, 8> {
   static constexpr TermTable<3> kTerms{{1, 0, 0}, {0, 1, 0}, {1, 1, 0}, {true, false, true}};
 };
 
@@ -1227,7 +1227,7 @@ struct Bf16x3Promoted : TraitsBase<3, 128, 64, 2, 2, 2, false, EpiF32, true, kPr
 // hi*hi in accumulator 0, so the main accumulator is rounded only by its own
 // MMAs; both are promoted into FP32 registers every kPromoteChunk k-blocks.
 // Order: smallest first, MMAs that read the same A plane adjacent.
-struct Bf16x6 : TraitsBase<6, 128, 64, 3, 3, 2, false, EpiF32, true, kPromoteChunk> {
+struct Bf16x6 : TraitsBase<6, 128, 64, 3, 3, 2, false, EpiF32, true, kPromoteChunk, 8> {
   static constexpr TermTable<6> kTerms{
       {2, 1, 1, 0, 0, 0}, {0, 1, 0, 2, 1, 0}, {1, 1, 1, 1, 1, 0}, {true, false, false, false, false, true}};
 };

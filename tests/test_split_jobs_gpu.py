@@ -36,11 +36,12 @@ def test_backward_planes_at_edges(cuda, shape, precision, nterms, epilogue):
     d = cc.make_desc(tA, tB, tY, float(alpha), 0.0, precision=precision, epilogue=epilogue)
     need = C.c_size_t(0)
     assert cc.lib().cucosma_gemm_backward_workspace_size(C.byref(d), C.byref(need)) == cc.SUCCESS
-    # the larger product's own part: what the two products need when they share it
+    # the larger product's own part: what the two products need when they share it (the flag's plan is the
+    # backward pass's: never the fused split, whose workspace holds no planes)
     parts = []
     for pm, pn, pk in ((m, k, n), (k, n, m)):
         a, b, c = (torch.empty(r, -(-q // 4) * 4, device="cuda")[:, :q] for r, q in ((pm, pk), (pk, pn), (pm, pn)))
-        parts.append(cc.workspace_size(cc.make_desc(a, b, c, precision=precision)))
+        parts.append(cc.workspace_size(cc.make_desc(a, b, c, precision=precision, flags=cc.FLAG_TEST_SKIP_STAGE)))
     assert need.value >= max(parts)
     for size in (need.value, max(parts)):
         dA, dB = to_dev(np.zeros_like(A)), to_dev(np.zeros_like(B))
