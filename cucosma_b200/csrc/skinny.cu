@@ -8,8 +8,7 @@
 // 4 x 3,000,000 x 4.
 //
 // Kind 2, thin M or N (<= 8) with K > 16: a CTA owns an 8 x 8 output block and
-// one K split; its 256 threads stride over K (coalesced reads of the thin
-// operand's rows and 32-byte rows of the other), each keeping the 64 partial
+// one K split; its 256 threads stride over K, each keeping the 64 partial
 // products, then reduce across the CTA in a fixed order.  Splits write raw
 // partials that a second kernel sums in a fixed order (the split-K reduction
 // of simt_gemm.cu, or one warp per output when there are many splits and few
@@ -39,13 +38,16 @@ __global__ void __launch_bounds__(256)
   __shared__ T As[BMS][skinny::kMaxSmallK + 1];
   __shared__ __align__(16) T Bs[SHARE_B ? skinny::kMaxSmallK : 1][SHARE_B ? BNS : VEC];
   const int tid = threadIdx.x, cg = tid % CG, rg = tid / CG;
+  int tm_loaded = -1;  // the row block As holds
   for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
     const int tm = (int)(t / tiles_n), tn = (int)(t - (int64_t)tm * tiles_n);
     const int m0 = tm * BMS, n0 = tn * BNS;
-    __syncthreads();  // the previous block's reads of As / Bs are done
-    for (int i = tid; i < BMS * k; i += 256) {
-      const int r = i / k, kk = i - r * k;
-      As[r][kk] = m0 + r < m ? A[(int64_t)(m0 + r) * lda + kk] : T(0);
+    if (SHARE_B || tm != tm_loaded) {
+      __syncthreads();  // the previous block's reads of As / Bs are done
+      for (int i = tid; i < BMS * k; i += 256) {
+        const int r = i / k, kk = i - r * k;
+        As[r][kk] = m0 + r < m ? A[(int64_t)(m0 + r) * lda + kk] : T(0);
+      }
     }
     if constexpr (SHARE_B) {
       for (int i = tid; i < k * CG; i += 256) {
@@ -62,33 +64,44 @@ __global__ void __launch_bounds__(256)
         *reinterpret_cast<V*>(&Bs[kk][c]) = v;
       }
     }
-    __syncthreads();
+    if (SHARE_B || tm != tm_loaded) __syncthreads();
+    tm_loaded = tm;
     const int col = n0 + cg * VEC;
     T acc[RPT][VEC];
 #pragma unroll
     for (int r = 0; r < RPT; ++r)
 #pragma unroll
       for (int e = 0; e < VEC; ++e) acc[r][e] = T(0);
-    for (int kk = 0; kk < k; ++kk) {
-      V bv;
-      if constexpr (SHARE_B) {
-        bv = *reinterpret_cast<const V*>(&Bs[kk][cg * VEC]);
-      } else {
-        const T* src = B + (int64_t)kk * ldb + col;
-        T* pb = reinterpret_cast<T*>(&bv);
-        if (col + VEC <= n) {
-          bv = *reinterpret_cast<const V*>(src);
-        } else {
+    // B straight from global memory: four rows' loads in flight at a time
+    constexpr int KU = SHARE_B ? 1 : 4;
+    for (int k0 = 0; k0 < k; k0 += KU) {
+      V bv[KU];
 #pragma unroll
-          for (int e = 0; e < VEC; ++e) pb[e] = col + e < n ? src[e] : T(0);
+      for (int u = 0; u < KU; ++u) {
+        const int kk = k0 + u;
+        if constexpr (SHARE_B) {
+          bv[u] = *reinterpret_cast<const V*>(&Bs[kk][cg * VEC]);
+        } else {
+          T* pb = reinterpret_cast<T*>(&bv[u]);
+          const T* src = B + (int64_t)kk * ldb + col;
+          if (kk < k && col + VEC <= n) {
+            bv[u] = *reinterpret_cast<const V*>(src);
+          } else {
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) pb[e] = kk < k && col + e < n ? src[e] : T(0);
+          }
         }
       }
-      const T* b = reinterpret_cast<const T*>(&bv);
 #pragma unroll
-      for (int r = 0; r < RPT; ++r) {
-        const T a = As[rg * RPT + r][kk];
+      for (int u = 0; u < KU; ++u) {
+        if (KU > 1 && k0 + u >= k) break;
+        const T* b = reinterpret_cast<const T*>(&bv[u]);
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) acc[r][e] = fma(a, b[e], acc[r][e]);
+        for (int r = 0; r < RPT; ++r) {
+          const T a = As[rg * RPT + r][k0 + u];
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) acc[r][e] = fma(a, b[e], acc[r][e]);
+        }
       }
     }
     if (col >= n) continue;
@@ -114,80 +127,95 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Thin kernel: each thread takes KV = VEC consecutive k per step (one
-// 16-byte load per row of the 8-row A block, KV rows of 8 B values).
-template <typename T>
-__global__ void __launch_bounds__(256)
+// Thin kernel: lanes take consecutive k, so a warp's load of a row of the A
+// block is one contiguous line, and its loads of 32 rows of the B block
+// (32-byte FP32 rows) contiguous too when B is as narrow as the block; KU
+// steps of 256 k are loaded before the first product.  HBM-bound: 4 x 8 x
+// 3,000,000 FP32 on B200 39.8 -> 23.8 us (6.1 TB/s); the form it
+// replaced gave each lane four consecutive k, whose B loads lay 128 bytes
+// apart, and was bound by L1 (82 % busy).
+// RS x CS: the part of the 8 x 8 block that exists (4 or 8 rows and columns):
+// fewer accumulators leave registers for loads in flight (4 x 8: 31 us with
+// three CTAs an SM and spills, 28 with two steps in flight, 27 with four and
+// two CTAs an SM, the reduction included).
+template <typename T, int RS, int CS>
+__global__ void __launch_bounds__(256, skinny::thin_ctas<T>(RS, CS))
     thin_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ B, int64_t ldb, T* out, int64_t ldo,
                 int m, int n, int k, int64_t kchunk, int groups_n, T alpha, T beta, int epi, int partial,
                 int64_t split_stride) {
   constexpr int S = skinny::kThin;
-  constexpr int KV = Vec<T>::n;
+  constexpr int VEC = Vec<T>::n;
+  constexpr int KU = RS * CS * (int)sizeof(T) <= 128 ? 4 : 2;
   using V = typename Vec<T>::type;
   const int gm = blockIdx.x / groups_n, gn = blockIdx.x - gm * groups_n;
   const int m0 = gm * S, n0 = gn * S;
-  const int rows = min(S, m - m0), cols = min(S, n - n0);
-  const int64_t kb = (int64_t)blockIdx.y * kchunk, ke = min((int64_t)k, kb + kchunk);  // kchunk % KV == 0
-  T acc[S][S];
+  const int rows = min(RS, m - m0), cols = min(CS, n - n0);
+  const int64_t kb = (int64_t)blockIdx.y * kchunk, ke = min((int64_t)k, kb + kchunk);
+  const T* a0 = A + (int64_t)m0 * lda;
+  const T* b0 = B + n0;
+  T acc[RS][CS];
 #pragma unroll
-  for (int i = 0; i < S; ++i)
+  for (int i = 0; i < RS; ++i)
 #pragma unroll
-    for (int j = 0; j < S; ++j) acc[i][j] = T(0);
-  for (int64_t k0 = kb + (int64_t)KV * threadIdx.x; k0 < ke; k0 += 256 * KV) {
-    T a[S][KV];
-    const bool full = k0 + KV <= ke;
+    for (int j = 0; j < CS; ++j) acc[i][j] = T(0);
+  for (int64_t k0 = kb + threadIdx.x; k0 < ke; k0 += 256 * KU) {
+    T a[KU][RS], b[KU][CS];
 #pragma unroll
-    for (int i = 0; i < S; ++i) {
-      const T* src = A + (int64_t)(m0 + i) * lda + k0;
-      if (i < rows && full) {
-        const V v = *reinterpret_cast<const V*>(src);  // k0 % KV == 0 and 16-byte rows
-        const T* pv = reinterpret_cast<const T*>(&v);
+    for (int u = 0; u < KU; ++u) {
+      const int64_t kk = k0 + 256 * u;
+      const bool in = kk < ke;
 #pragma unroll
-        for (int q = 0; q < KV; ++q) a[i][q] = pv[q];
-      } else {
+      for (int i = 0; i < RS; ++i) a[u][i] = in && i < rows ? a0[(int64_t)i * lda + kk] : T(0);
+      const T* brow = b0 + kk * ldb;
 #pragma unroll
-        for (int q = 0; q < KV; ++q) a[i][q] = (i < rows && k0 + q < ke) ? src[q] : T(0);
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < KV; ++q) {
-      if (k0 + q >= ke) break;
-      T b[S];
-      const T* brow = B + (k0 + q) * ldb + n0;
-      if (cols == S) {
-        // 8 elements from a 16-byte aligned address (n0 % 8 == 0, 16-byte rows)
-#pragma unroll
-        for (int h = 0; h < S / KV; ++h) {
-          const V v = *reinterpret_cast<const V*>(brow + h * KV);
+      for (int h = 0; h < CS / VEC; ++h) {
+        if (in && (h + 1) * VEC <= cols) {  // n0 % 8 == 0 and 16-byte rows
+          const V v = *reinterpret_cast<const V*>(brow + h * VEC);
           const T* pv = reinterpret_cast<const T*>(&v);
 #pragma unroll
-          for (int e = 0; e < KV; ++e) b[h * KV + e] = pv[e];
+          for (int e = 0; e < VEC; ++e) b[u][h * VEC + e] = pv[e];
+        } else {
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) b[u][h * VEC + e] = in && h * VEC + e < cols ? brow[h * VEC + e] : T(0);
         }
-      } else {
-#pragma unroll
-        for (int j = 0; j < S; ++j) b[j] = j < cols ? brow[j] : T(0);
       }
+    }
 #pragma unroll
-      for (int i = 0; i < S; ++i)
+    for (int u = 0; u < KU; ++u)
 #pragma unroll
-        for (int j = 0; j < S; ++j) acc[i][j] = fma(a[i][q], b[j], acc[i][j]);
+      for (int i = 0; i < RS; ++i)
+#pragma unroll
+        for (int j = 0; j < CS; ++j) acc[i][j] = fma(a[u][i], b[u][j], acc[i][j]);
+  }
+  // Fixed-order reduction: within each warp every step halves the outputs a
+  // lane keeps (ending with one or two consecutive ones, or, for fewer outputs
+  // than lanes, one that several lanes hold), then warps 0..7 in order.
+  constexpr int OUT = RS * CS;
+  __shared__ T red[8][OUT];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  T v[OUT];
+#pragma unroll
+  for (int i = 0; i < OUT; ++i) v[i] = acc[i / CS][i % CS];
+  int first = 0;  // the output v[0] is the sum of
+#pragma unroll
+  for (int off = 16, half = OUT / 2; off > 0; off >>= 1, half >>= 1) {
+    if (half > 0) {
+      const bool up = (lane & off) != 0;
+      if (up) first += half;
+#pragma unroll
+      for (int i = 0; i < half; ++i) {
+        const T keep = up ? v[i + half] : v[i], send = up ? v[i] : v[i + half];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+      }
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
     }
   }
-  // Fixed-order reduction: butterfly within each warp, then warps 0..7 in order.
-  __shared__ T red[8][S * S];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int i = 0; i < S; ++i)
-#pragma unroll
-    for (int j = 0; j < S; ++j) {
-      T x = acc[i][j];
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
-      if (lane == 0) red[warp][i * S + j] = x;
-    }
+  if constexpr (OUT == 64) red[warp][first + 1] = v[1];
+  red[warp][first] = v[0];
   __syncthreads();
-  if (threadIdx.x < S * S) {
-    const int i = threadIdx.x / S, j = threadIdx.x % S;
+  if (threadIdx.x < OUT) {
+    const int i = threadIdx.x / CS, j = threadIdx.x % CS;
     T s = red[0][threadIdx.x];
 #pragma unroll
     for (int w = 1; w < 8; ++w) s += red[w][threadIdx.x];
@@ -250,9 +278,12 @@ SkinnyPlan plan_skinny(int64_t m, int64_t n, int64_t k, int dtype_bytes, int spl
   p.kind = 2;
   p.tile_m = p.tile_n = skinny::kThin;
   const int64_t groups = ceil_div(m, skinny::kThin) * ceil_div(n, skinny::kThin);
-  int64_t splits = split_k > 0 ? split_k : ceil_div(4 * (int64_t)sms, groups);
+  // one wave of resident CTAs
+  const int ctas = dtype_bytes == 4 ? skinny::thin_ctas<float>(skinny::thin_side(m), skinny::thin_side(n))
+                                    : skinny::thin_ctas<double>(skinny::thin_side(m), skinny::thin_side(n));
+  int64_t splits = split_k > 0 ? split_k : ceil_div(ctas * (int64_t)sms, groups);
   splits = std::max<int64_t>(1, std::min<int64_t>({splits, ceil_div(k, 256), 65535}));
-  p.kchunk = round_up(ceil_div(k, splits), vec);  // whole 16-byte steps per split
+  p.kchunk = round_up(ceil_div(k, splits), 32);  // whole 128-byte (FP64: 256) lines per split
   p.splits = (int)ceil_div(k, p.kchunk);
   p.ldw = round_up(n, vec);
   p.ws_bytes = p.splits > 1 ? (size_t)p.splits * (size_t)m * (size_t)p.ldw * dtype_bytes : 0;
@@ -278,17 +309,15 @@ cudaError_t launch_skinny(const SkinnyPlan& pl, const T* A, int64_t lda, const T
   const int groups_n = (int)ceil_div(n, skinny::kThin);
   const int64_t groups = ceil_div(m, skinny::kThin) * (int64_t)groups_n;
   const dim3 grid((unsigned)groups, (unsigned)pl.splits);
-  if (pl.splits == 1) {
-    thin_kernel<T><<<grid, 256, 0, st>>>(A, lda, B, ldb, C, ldc, m, n, k, pl.kchunk, groups_n, (T)alpha, (T)beta, epi,
-                                         0, 0);
-    return cudaGetLastError();
-  }
-  T* w = static_cast<T*>(ws);
   const int64_t stride = (int64_t)m * pl.ldw;
-  thin_kernel<T><<<grid, 256, 0, st>>>(A, lda, B, ldb, w, pl.ldw, m, n, k, pl.kchunk, groups_n, (T)alpha, (T)beta, epi,
-                                       1, stride);
+  const bool partial = pl.splits > 1;
+  T* w = static_cast<T*>(ws);
+  auto* kernel = m <= 4 ? (n <= 4 ? thin_kernel<T, 4, 4> : thin_kernel<T, 4, 8>)
+                        : (n <= 4 ? thin_kernel<T, 8, 4> : thin_kernel<T, 8, 8>);
+  kernel<<<grid, 256, 0, st>>>(A, lda, B, ldb, partial ? w : C, partial ? pl.ldw : ldc, m, n, k, pl.kchunk, groups_n,
+                               (T)alpha, (T)beta, epi, partial ? 1 : 0, stride);
   cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess || !partial) return e;
   if (pl.splits >= 32 && (int64_t)m * n <= (int64_t)sms * 64) {
     thin_reduce_kernel<T><<<(unsigned)ceil_div((int64_t)m * n, 8), 256, 0, st>>>(w, stride, pl.ldw, pl.splits, C, ldc,
                                                                                    m, n, (T)alpha, (T)beta, epi);

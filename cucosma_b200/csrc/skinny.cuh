@@ -24,6 +24,13 @@ struct SkinnyPlan {
 namespace skinny {
 constexpr int kMaxSmallK = 16;  // kind 1 when K <= this
 constexpr int kThin = 8;        // kind 2 when M <= this or N <= this
+// Rows (columns) of thin_kernel's block that exist, 4 or 8, and its resident
+// CTAs per SM with that many accumulators a thread.
+constexpr int thin_side(int64_t extent) { return extent <= 4 ? 4 : kThin; }
+template <typename T>
+constexpr int thin_ctas(int rs, int cs) {
+  return rs * cs * (int)sizeof(T) <= 64 ? 4 : rs * cs * (int)sizeof(T) <= 128 ? 2 : rs * cs * (int)sizeof(T) <= 256 ? 2 : 1;
+}
 }  // namespace skinny
 
 // desc must describe a native-precision GEMM with m, n, k > 0.
