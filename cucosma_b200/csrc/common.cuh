@@ -34,6 +34,30 @@ inline cudaError_t debug_cuda(const char* what, cudaError_t e) {
   return e;
 }
 
+// Launches a kernel that begins with pdl_wait(); with `early` its launch and
+// its set-up overlap the end of the kernel before it in the stream (the second
+// kernel of a call; about 2 us on B200: 512^3 BF16x6 18.4 -> 16.4 us, 1024^3
+// FP32 59.7 -> 57).  Not for every second kernel: early CTAs go where there is
+// room, so a reduction of many splits packed itself onto the few SMs its GEMM
+// had left idle (213 x 201 x 19463 BF16x6, 36 splits: 36.8 -> 43.5 us), and a
+// GEMM of several waves lost the CTA order its L2 reuse rests on (grouped
+// batch of 512, BF16x3: 2.89 -> 3.02 ms).
+template <typename... KArgs, typename... Args>
+cudaError_t launch_after(bool early, void (*kernel)(KArgs...), dim3 grid, unsigned threads, size_t smem,
+                         cudaStream_t st, Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 enum Epilogue : int { kEpiNone = 0, kEpiSigmoid = 1, kEpiRelu = 2 };
 
 // Fused activation applied to the final value (cuCOSMAV100.cuh:2466-2476

@@ -45,6 +45,16 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// ------------------------------------------------------- dependent launches
+// A kernel launched by launch_after() (common.cuh) may start while the kernel
+// before it in the stream still runs: pdl_wait() holds until that kernel has
+// completed and its writes are visible (a no-op in a plain launch), so it
+// comes before the first access to anything an earlier kernel of the call
+// wrote or still reads.  pdl_trigger(), once every CTA has issued it, lets the next kernel's
+// CTAs start (in what room is left) instead of at this kernel's end.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ------------------------------------------------------------------ mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");

@@ -88,6 +88,7 @@ template <int BM_>
 __global__ void __launch_bounds__(simt::SgemmShape<BM_>::kThreads, simt::SgemmShape<BM_>::kCtasPerSm)
     simt_sgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const SimtParams p) {
+  pdl_trigger();
   if (p.gate != nullptr && *p.gate != p.gate_value) return;  // path not chosen on the device
   using namespace simt;
   using Shape = SgemmShape<BM_>;
@@ -262,6 +263,7 @@ __device__ __forceinline__ void store_pair(const SimtParams& p, int r, int c, do
 __global__ void __launch_bounds__(simt::kThreads, 1)
     simt_dgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const SimtParams p) {
+  pdl_trigger();
   if (p.gate != nullptr && *p.gate != p.gate_value) return;  // path not chosen on the device
   using namespace simt;
   constexpr int BK = Cfg<double>::BK;  // 16
@@ -391,6 +393,7 @@ template <typename T>
 __global__ void splitk_reduce_kernel(const T* __restrict__ ws, int64_t split_stride, int64_t ldw, int splits, T* C,
                                      int64_t ldc, int m, int n, double alpha_d, double beta_d, int epi,
                                      const int* gate, int gate_value) {
+  pdl_wait();
   if (gate != nullptr && *gate != gate_value) return;  // path not chosen on the device
   constexpr int VEC = Vec<T>::n;
   using V = typename Vec<T>::type;
@@ -511,9 +514,8 @@ cudaError_t launch_reduce(const T* ws, int64_t split_stride, int64_t ldw, int sp
   int64_t blocks = ceil_div(work, threads);
   blocks = std::min<int64_t>(blocks, (int64_t)num_sms * 8);
   if (blocks < 1) blocks = 1;
-  splitk_reduce_kernel<T><<<(unsigned)blocks, threads, 0, stream>>>(ws, split_stride, ldw, splits, C, ldc, m, n, alpha,
-                                                                    beta, epi, gate, gate_value);
-  return cudaGetLastError();
+  return launch_after(splits <= 8, splitk_reduce_kernel<T>, dim3((unsigned)blocks), threads, 0, stream, ws, split_stride, ldw,
+                      splits, C, ldc, m, n, alpha, beta, epi, gate, gate_value);
 }
 
 template <typename T>

@@ -320,7 +320,7 @@ cudaError_t launch_skinny(const SkinnyPlan& pl, const T* A, int64_t lda, const T
   if (e != cudaSuccess || !partial) return e;
   if (pl.splits >= 32 && (int64_t)m * n <= (int64_t)sms * 64) {
     thin_reduce_kernel<T><<<(unsigned)ceil_div((int64_t)m * n, 8), 256, 0, st>>>(w, stride, pl.ldw, pl.splits, C, ldc,
-                                                                                   m, n, (T)alpha, (T)beta, epi);
+                                                                                 m, n, (T)alpha, (T)beta, epi);
     return cudaGetLastError();
   }
   return simt::launch_reduce<T>(w, stride, pl.ldw, pl.splits, C, ldc, m, n, alpha, beta, epi, sms, st);

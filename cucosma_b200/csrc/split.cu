@@ -175,6 +175,7 @@ __device__ __forceinline__ void split_cols_tile(const SplitJob& j, int tk, int t
 template <int NT>
 __global__ void __launch_bounds__(256, 4) split_bf16_kernel(const __grid_constant__ SplitJobs jobs) {
   __shared__ __align__(16) float tile[64 * 64];
+  pdl_trigger();
   int b = blockIdx.x, ji = 0;
   while (ji + 1 < jobs.count && b >= jobs.job[ji].blocks) b -= jobs.job[ji++].blocks;
   const SplitJob& j = jobs.job[ji];

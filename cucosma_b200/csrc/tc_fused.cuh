@@ -207,6 +207,7 @@ __global__ void __maxnreg__((FusedInplaceCfg<Tr, STG>::MAX_REGS))
   constexpr int BN = Tr::BN, NACC = Tr::NACC, NS = F::NS, NBUF = Tr::NBUF, TILE_M = Tr::TILE_M;
   constexpr int A_REGION = Tr::A_REGION;
 
+  pdl_trigger();  // the split-K reduction
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* stages = smem;

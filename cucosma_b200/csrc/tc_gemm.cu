@@ -16,6 +16,7 @@ __global__ void ozaki_reduce_kernel(const double* __restrict__ ws, int64_t split
                                     double* C, int64_t ldc, int m, int n, const int32_t* __restrict__ ea,
                                     const int32_t* __restrict__ eb, double alpha, double beta, int epi,
                                     const int* gate, int gate_value) {
+  pdl_wait();
   if (gate != nullptr && *gate != gate_value) return;
   const int64_t total = (int64_t)m * n;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -439,10 +440,9 @@ cudaError_t run_ozaki(const cucosma_gemm_desc* d, const Plan& pl, const Tiling& 
   if (e == cudaSuccess && t.splits > 1) {
     const int64_t work = (int64_t)m * n;
     const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(work, 256), di->sms * 8));
-    ozaki_reduce_kernel<<<blocks, 256, 0, st>>>((const double*)p.out, p.ws_split_stride, pl.ldw, t.splits,
-                                                (double*)C, d->ldc, m, n, ea, eb, d->alpha, d->beta, d->epilogue, gate,
-                                                s);
-    e = cudaGetLastError();
+    e = launch_after(t.splits <= 8, ozaki_reduce_kernel, dim3(blocks), 256, 0, st, (const double*)p.out, p.ws_split_stride, pl.ldw,
+                     t.splits, (double*)C, d->ldc, m, n, (const int32_t*)ea, (const int32_t*)eb, d->alpha, d->beta,
+                     d->epilogue, gate, s);
     launches += 1;
   }
   return e;

@@ -250,6 +250,7 @@ __global__ void __maxnreg__(Tr::MAX_REGS)
   constexpr bool PAIR = Tr::PAIR;
   constexpr int TILE_M = Tr::TILE_M;
 
+  pdl_trigger();  // the split-K reduction
   // Not the path chosen on the device: every CTA (both of a pair) leaves
   // before touching barriers or TMEM.
   if (p.gate != nullptr && *p.gate != p.gate_value) return;
@@ -313,14 +314,15 @@ __global__ void __maxnreg__(Tr::MAX_REGS)
     __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  if (p.ngroups == 0 && threadIdx.x == 0) {
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+  }
+  pdl_wait();  // the operand planes (set-up above overlaps the pre-pass)
 
   if (warp == 0) {
     // ---------------------------------------------------------- producer
     if (lane == 0) {
-      if (p.ngroups == 0) {
-        tma_prefetch_desc(&tmA);
-        tma_prefetch_desc(&tmB);
-      }
       int it = 0;  // global k-block counter (ring position)
       bool ok = true;
       for (int unit = unit0; unit < units && ok; unit += unit_step) {
@@ -1303,6 +1305,9 @@ struct Ozaki : TraitsBase<S*(S + 1) / 2, OzakiBN<S>::value, 128, S, S, S, true, 
 template <class Tr>
 static cudaError_t launch(const CUtensorMap& a, const CUtensorMap& b, const TcParams& p, int grid, cudaStream_t st) {
   static std::atomic<uint64_t> attr_set{0};  // devices whose context has the limit raised
+  // one wave, and not gated (a gated kernel reads the choice first of all)
+  const bool early = p.gate == nullptr && p.ngroups == 0 &&
+                     p.tiles_m * p.tiles_n * p.splits <= (Tr::PAIR ? grid / 2 : grid);
   cudaError_t e = debug_cuda("smem attribute",
                              ensure_smem_attr(reinterpret_cast<const void*>(tc_gemm_kernel<Tr>), Tr::SMEM, attr_set));
   if (e != cudaSuccess) return e;
@@ -1312,19 +1317,21 @@ static cudaError_t launch(const CUtensorMap& a, const CUtensorMap& b, const TcPa
     cfg.blockDim = dim3(Tr::THREADS, 1, 1);
     cfg.dynamicSmemBytes = Tr::SMEM;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 2;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early ? 2 : 1;
     e = debug_cuda("pair kernel launch", cudaLaunchKernelEx(&cfg, tc_gemm_kernel<Tr>, a, b, p));
     if (e != cudaSuccess) return e;
     return debug_cuda("pair kernel launch (last error)", cudaGetLastError());
   }
-  tc_gemm_kernel<Tr><<<grid, Tr::THREADS, Tr::SMEM, st>>>(a, b, p);
-  return debug_cuda("kernel launch", cudaGetLastError());
+  return debug_cuda("kernel launch", launch_after(early, tc_gemm_kernel<Tr>, dim3((unsigned)grid), Tr::THREADS, Tr::SMEM,
+                                                  st, a, b, p));
 }
 
 // Clusters of two CTAs of a pair kernel that can be resident at once on the
