@@ -118,11 +118,18 @@ def check(status, what=""):
         raise CucosmaError(status, what)
 
 
+_raw_stream = None  # torch's current-stream handle as an integer, without a Stream object (3 us a call)
+
+
 def _stream_handle(stream):
     if stream is None:
+        global _raw_stream
         import torch
 
-        return torch.cuda.current_stream().cuda_stream
+        if _raw_stream is None:
+            _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or \
+                (lambda device: torch.cuda.current_stream(device).cuda_stream)
+        return _raw_stream(torch.cuda.current_device())
     return getattr(stream, "cuda_stream", stream)
 
 
@@ -137,9 +144,11 @@ def _dtype_code(t):
 
 
 def _ld(t):
-    if t.dim() != 2 or t.stride(1) != 1:
+    st = t.stride()
+    if len(st) != 2 or st[1] != 1:
         raise ValueError("cucosma: matrices must be 2-D row-major with unit column stride")
-    return t.stride(0) if t.shape[0] > 1 else max(t.stride(0), t.shape[1])
+    shape = t.shape
+    return st[0] if shape[0] > 1 else max(st[0], shape[1])
 
 
 FLAG_TEST_SKIP_STAGE = 1 << 30  # CUCOSMA_FLAG_TEST_SKIP_STAGE: failure-path test hook
@@ -149,18 +158,13 @@ def make_desc(A, B, Cm, alpha=1.0, beta=0.0, precision="native", epilogue="none"
               slices=0, tile=0, flags=0):
     m, k = A.shape
     k2, n = B.shape
-    if k != k2 or tuple(Cm.shape) != (m, n):
+    if k != k2 or Cm.shape != (m, n):
         raise ValueError("cucosma: shape mismatch A%s B%s C%s" % (tuple(A.shape), tuple(B.shape), tuple(Cm.shape)))
-    d = GemmDesc()
-    lib().cucosma_gemm_desc_init(C.byref(d))
-    d.m, d.n, d.k = m, n, k
-    d.lda, d.ldb, d.ldc = _ld(A), _ld(B), _ld(Cm)
-    d.dtype = _dtype_code(Cm)
-    d.precision = PRECISIONS[precision] if isinstance(precision, str) else int(precision)
-    d.epilogue = EPILOGUES[epilogue] if isinstance(epilogue, str) else int(epilogue)
-    d.alpha, d.beta = float(alpha), float(beta)
-    d.split_k, d.swizzle, d.slices, d.tile, d.flags = int(split_k), int(swizzle), int(slices), int(tile), int(flags)
-    return d
+    # field order of cucosma_gemm_desc; every field is set
+    return GemmDesc(m, n, k, _ld(A), _ld(B), _ld(Cm), _dtype_code(Cm),
+                    PRECISIONS[precision] if isinstance(precision, str) else int(precision), int(slices),
+                    EPILOGUES[epilogue] if isinstance(epilogue, str) else int(epilogue), float(alpha), float(beta),
+                    int(split_k), int(swizzle), int(tile), int(flags))
 
 
 def get_plan(desc):

@@ -328,8 +328,11 @@ cucosma_status gemm(const cucosma_gemm_desc* d, const void* A, const void* B, vo
   return gemm_ex(d, A, B, C, ws, ws_bytes, st, kPrepA | kPrepB);
 }
 
-cucosma_status gemm_ex(const cucosma_gemm_desc* d, const void* A, const void* B, void* C, void* ws, size_t ws_bytes,
-                       cudaStream_t st, int prep) {
+// One validated, tuned and planned call: the native plans are made once (the
+// split search takes microseconds, which small calls would see).  managed: the
+// workspace is the library's buffer for this stream instead of ws.
+static cucosma_status run_gemm(const cucosma_gemm_desc* d, const void* A, const void* B, void* C, void* ws,
+                               size_t ws_bytes, cudaStream_t st, int prep, bool managed) {
   cucosma_status s = validate(d, A, B, C);
   if (s != CUCOSMA_STATUS_SUCCESS) return s;
   if (d->m == 0 || d->n == 0) return CUCOSMA_STATUS_SUCCESS;
@@ -347,21 +350,35 @@ cucosma_status gemm_ex(const cucosma_gemm_desc* d, const void* A, const void* B,
     note_launches(1);
     return e == cudaSuccess ? CUCOSMA_STATUS_SUCCESS : CUCOSMA_STATUS_LAUNCH_FAILED;
   }
+  const bool native = d->precision == CUCOSMA_PRECISION_NATIVE;
+  SkinnyPlan sp{};
+  NativePlan pl{};
   size_t need = 0;
-  s = workspace_size(d, &need, di);
-  if (s != CUCOSMA_STATUS_SUCCESS) return s;
+  if (native) {
+    sp = plan_skinny_for(d, di->sms);
+    if (!sp.kind) pl = plan_native(d, di->sms);
+    need = sp.kind ? sp.ws_bytes : pl.ws_bytes;
+  } else if ((s = tc_workspace_size(d, &need, di)) != CUCOSMA_STATUS_SUCCESS) {
+    return s;
+  }
+  if (managed && need > 0) {
+    ws = managed_workspace(need, st);
+    if (!ws) return CUCOSMA_STATUS_ALLOC_FAILED;
+    ws_bytes = need;
+  }
   if (need > 0 && (ws == nullptr || ws_bytes < need)) return CUCOSMA_STATUS_WORKSPACE_TOO_SMALL;
   if (need > 0 && !aligned16(ws)) return CUCOSMA_STATUS_MISALIGNED;
-  if (d->precision == CUCOSMA_PRECISION_NATIVE) {
-    const SkinnyPlan sp = plan_skinny_for(d, di->sms);
-    if (sp.kind)
-      return fp32 ? run_skinny<float>(d, sp, (const float*)A, (const float*)B, (float*)C, ws, di, st)
-                  : run_skinny<double>(d, sp, (const double*)A, (const double*)B, (double*)C, ws, di, st);
-    const NativePlan pl = plan_native(d, di->sms);
-    return fp32 ? run_native<float>(d, pl, (const float*)A, (const float*)B, (float*)C, ws, di, st)
-                : run_native<double>(d, pl, (const double*)A, (const double*)B, (double*)C, ws, di, st);
-  }
-  return tc_gemm_ex(d, A, B, C, ws, ws_bytes, di, st, prep);
+  if (!native) return tc_gemm_ex(d, A, B, C, ws, ws_bytes, di, st, prep);
+  if (sp.kind)
+    return fp32 ? run_skinny<float>(d, sp, (const float*)A, (const float*)B, (float*)C, ws, di, st)
+                : run_skinny<double>(d, sp, (const double*)A, (const double*)B, (double*)C, ws, di, st);
+  return fp32 ? run_native<float>(d, pl, (const float*)A, (const float*)B, (float*)C, ws, di, st)
+              : run_native<double>(d, pl, (const double*)A, (const double*)B, (double*)C, ws, di, st);
+}
+
+cucosma_status gemm_ex(const cucosma_gemm_desc* d, const void* A, const void* B, void* C, void* ws, size_t ws_bytes,
+                       cudaStream_t st, int prep) {
+  return run_gemm(d, A, B, C, ws, ws_bytes, st, prep, false);
 }
 
 // ---------------------------------------------- launch count and profiling
@@ -498,17 +515,7 @@ extern "C" cucosma_status cucosma_gemm(const cucosma_gemm_desc* d, const void* A
 
 extern "C" cucosma_status cucosma_gemm_managed(const cucosma_gemm_desc* d, const void* A, const void* B, void* C,
                                                void* stream) {
-  cucosma_status s = validate(d, A, B, C);
-  if (s != CUCOSMA_STATUS_SUCCESS) return s;
-  size_t need = 0;
-  s = cucosma_gemm_workspace_size(d, &need);
-  if (s != CUCOSMA_STATUS_SUCCESS) return s;
-  void* ws = nullptr;
-  if (need) {
-    ws = managed_workspace(need, static_cast<cudaStream_t>(stream));
-    if (!ws) return CUCOSMA_STATUS_ALLOC_FAILED;
-  }
-  return gemm(d, A, B, C, ws, need, static_cast<cudaStream_t>(stream));
+  return run_gemm(d, A, B, C, nullptr, 0, static_cast<cudaStream_t>(stream), kPrepA | kPrepB, true);
 }
 
 template <typename T>
