@@ -16,142 +16,85 @@
 #include <vector>
 
 #include "split_device.cuh"
+#include "split_tiles.cuh"
 #include "tc_kernel.cuh"
 
 struct cucosma_grouped_plan_st {
   cucosma_gemm_desc desc;
-  int count = 0, kind = 0, slices = 0, total_tiles = 0;
+  int count = 0, kind = 0, slices = 0, total_tiles = 0, grid = 0;
   int tile = 1, tile_m = 128, tile_n = 128, pair = 0, from_cache = 0;
   int pre_a_blocks = 0, pre_b_blocks = 0, exp_a_blocks = 0, exp_b_blocks = 0;
   int device = 0;
   void* workspace = nullptr;
   cucosma::tc::GroupEntry* table = nullptr;  // device copy inside the workspace
+  const int* starts = nullptr;      // [4][count]: pre-pass blocks (A, B), exponent blocks (A, B) before each problem
+  const int2* unit_list = nullptr;  // the GEMM's work list (TcParams::unit_list)
 };
 
 namespace cucosma {
 namespace tc {
 
-// Problem owning pre-pass block b: last entry whose start field is <= b.
-template <int FIELD>
-__device__ __forceinline__ int find_entry(const GroupEntry* g, int count, int b) {
-  auto start = [&](int i) {
-    return FIELD == 0 ? g[i].pre_a_start : FIELD == 1 ? g[i].pre_b_start : FIELD == 2 ? g[i].exp_a_start
-                                                                                      : g[i].exp_b_start;
-  };
-  int lo = 0, hi = count - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (start(mid) <= b)
-      lo = mid;
-    else
-      hi = mid - 1;
+// Problem owning pre-pass block b: the number of starts <= b, less one.  The
+// block counts the (ascending) starts together -- one load latency, where a
+// binary search by every thread was nine in a row.
+__device__ __forceinline__ int find_entry(const int* __restrict__ starts, int count, int b) {
+  int n = 0;
+  for (int i = 0; i < count; i += 256) {
+    const int j = i + (int)threadIdx.x;
+    n += __syncthreads_count(j < count && starts[j] <= b);
   }
-  return lo;
+  return n - 1;
 }
 
-// BF16 split of every problem (NT terms).  Blocks [0, a_blocks): 8 rows of
-// some A per block, one warp per row, lanes over 8-column groups (two 16-byte
-// loads, one 16-byte store per plane).  Blocks after that: one 64 (k) x 64 (n)
-// tile of some B, transposed: 16 lanes load 64 floats of a row; a lane then
-// converts 4 consecutive k of one column (one 8-byte store per plane).
+// BF16 split of every problem (NT terms).  Blocks [0, a_blocks): kRowsPerBlock
+// row units of some A; blocks after that: up to kStripTiles 64 x 64 tiles of
+// one column strip of some B, transposed.  Several units a block, because each
+// block first waits for its problem's table entry.
+constexpr int kRowsPerBlock = 32, kStripTiles = 4;
 template <int NT>
-__global__ void __launch_bounds__(256) grouped_split_bf16_kernel(const GroupEntry* __restrict__ g, int count,
-                                                                 int a_blocks) {
-  __shared__ float tile[64][65];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+__global__ void __launch_bounds__(256, 4)
+    grouped_split_bf16_kernel(const GroupEntry* __restrict__ g, const int* __restrict__ starts, int count,
+                              int a_blocks) {
+  __shared__ __align__(16) float tile[64 * 64];
   int b = blockIdx.x;
+  SplitJob j{};
   if (b < a_blocks) {
-    const GroupEntry& e = g[find_entry<0>(g, count, b)];
-    const int r = (b - e.pre_a_start) * 8 + warp;
-    if (r >= e.m) return;
-    const float* src = static_cast<const float*>(e.A) + (int64_t)r * e.lda;
-    __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(e.planes_a) + (int64_t)r * e.kpad;
-    const int64_t plane = (int64_t)e.m * e.kpad;
-    const int nc8 = (int)(e.kpad / 8);
-    for (int gi = lane; gi < nc8; gi += 32) {
-      const int c = gi * 8;
-      float v[8];
-      if (c + 8 <= e.k) {
-        const float4 q0 = *reinterpret_cast<const float4*>(src + c);  // 16-byte rows, c % 8 == 0
-        const float4 q1 = *reinterpret_cast<const float4*>(src + c + 4);
-        v[0] = q0.x, v[1] = q0.y, v[2] = q0.z, v[3] = q0.w, v[4] = q1.x, v[5] = q1.y, v[6] = q1.z, v[7] = q1.w;
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = c + j < e.k ? src[c + j] : 0.f;
-      }
-      uint32_t pk[NT][4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        __nv_bfloat16 t0[NT], t1[NT];
-        split_bf16_n<NT>(v[2 * j], t0);
-        split_bf16_n<NT>(v[2 * j + 1], t1);
-#pragma unroll
-        for (int i = 0; i < NT; ++i) pk[i][j] = pack_bf16x2(t0[i], t1[i]);
-      }
-#pragma unroll
-      for (int i = 0; i < NT; ++i)
-        *reinterpret_cast<uint4*>(dst + i * plane + c) = make_uint4(pk[i][0], pk[i][1], pk[i][2], pk[i][3]);
-    }
-    return;
-  }
-  b -= a_blocks;
-  const GroupEntry& e = g[find_entry<1>(g, count, b)];
-  const int t = b - e.pre_b_start;
-  const int tiles_n64 = (e.n + 63) / 64;
-  const int k0 = (t / tiles_n64) * 64, n0 = (t % tiles_n64) * 64;
-  const float* B = static_cast<const float*>(e.B);
-#pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    const int i = p * 16 + tid / 16, c = (tid % 16) * 4;
-    const int k = k0 + i, n = n0 + c;
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
-    if (k < e.k) {
-      const float* src = B + (int64_t)k * e.ldb + n;
-      if (n + 4 <= e.n) {
-        const float4 q = *reinterpret_cast<const float4*>(src);  // n % 4 == 0, 16-byte rows
-        v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = n + j < e.n ? src[j] : 0.f;
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) tile[i][c + j] = v[j];
-  }
-  __syncthreads();
-  const int64_t plane = (int64_t)e.n * e.kpad;
-  __nv_bfloat16* out = static_cast<__nv_bfloat16*>(e.planes_b);
-#pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    const int item = p * 256 + tid, nl = item / 16, kq = item % 16;
-    const int n = n0 + nl, k = k0 + kq * 4;
-    if (n < e.n && k < e.kpad) {  // kpad % 8 == 0: k + 3 < kpad as well
-      uint32_t pk[NT][2];
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        __nv_bfloat16 t0[NT], t1[NT];
-        split_bf16_n<NT>(tile[kq * 4 + 2 * j][nl], t0);
-        split_bf16_n<NT>(tile[kq * 4 + 2 * j + 1][nl], t1);
-#pragma unroll
-        for (int i = 0; i < NT; ++i) pk[i][j] = pack_bf16x2(t0[i], t1[i]);
-      }
-      __nv_bfloat16* dst = out + (int64_t)n * e.kpad + k;
-#pragma unroll
-      for (int i = 0; i < NT; ++i) *reinterpret_cast<uint2*>(dst + i * plane) = make_uint2(pk[i][0], pk[i][1]);
-    }
+    const GroupEntry& e = g[find_entry(starts, count, b)];
+    j.src = static_cast<const float*>(e.A);
+    j.ld = e.lda;
+    j.rows = e.m;
+    j.cols = e.k;
+    j.out_r = static_cast<__nv_bfloat16*>(e.planes_a);
+    j.kpad_r = e.kpad;
+    const int64_t u0 = (int64_t)(b - e.pre_a_start) * kRowsPerBlock + (threadIdx.x >> 5);
+#pragma unroll 1
+    for (int i = 0; i < kRowsPerBlock; i += 8) split_rows_unit<NT>(j, u0 + i);
+  } else {
+    b -= a_blocks;
+    const GroupEntry& e = g[find_entry(starts + count, count, b)];
+    const int t = b - e.pre_b_start, tiles_n = (e.n + 63) / 64;
+    j.src = static_cast<const float*>(e.B);
+    j.ld = e.ldb;
+    j.rows = e.k;
+    j.cols = e.n;
+    j.out_c = static_cast<__nv_bfloat16*>(e.planes_b);
+    j.kpad_c = e.kpad;
+    const int tk0 = t / tiles_n * kStripTiles, tk1 = min(tk0 + kStripTiles, (int)((e.kpad + 63) / 64));
+    split_cols_strip<NT>(j, tk0, tk1, t % tiles_n, tile);
   }
 }
 
 // Ozaki exponents of every problem: blocks [0, a_blocks) take 8 rows of some
 // A (warp per row); the rest take 32 columns of some B (8 thread rows
 // striding over K).
-__global__ void __launch_bounds__(256) grouped_ozaki_exp_kernel(const GroupEntry* __restrict__ g, int count,
+__global__ void __launch_bounds__(256) grouped_ozaki_exp_kernel(const GroupEntry* __restrict__ g,
+                                                                const int* __restrict__ starts, int count,
                                                                 int a_blocks) {
   __shared__ double red[8][33];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int b = blockIdx.x;
   if (b < a_blocks) {
-    const GroupEntry& e = g[find_entry<2>(g, count, b)];
+    const GroupEntry& e = g[find_entry(starts + 2 * count, count, b)];
     const int r = (b - e.exp_a_start) * 8 + warp;
     if (r >= e.m) return;
     const double* src = static_cast<const double*>(e.A) + (int64_t)r * e.lda;
@@ -163,7 +106,7 @@ __global__ void __launch_bounds__(256) grouped_ozaki_exp_kernel(const GroupEntry
     return;
   }
   b -= a_blocks;
-  const GroupEntry& e = g[find_entry<3>(g, count, b)];
+  const GroupEntry& e = g[find_entry(starts + 3 * count, count, b)];
   const int n = (b - e.exp_b_start) * 32 + lane;
   const double* B = static_cast<const double*>(e.B);
   double m = 0.0;
@@ -181,13 +124,14 @@ __global__ void __launch_bounds__(256) grouped_ozaki_exp_kernel(const GroupEntry
 // 8 rows of some A (warp per row, lanes over 4-column groups); the rest take
 // one 32 (k) x 64 (n) tile of some B, transposed.
 template <int S>
-__global__ void __launch_bounds__(256) grouped_ozaki_slice_kernel(const GroupEntry* __restrict__ g, int count,
+__global__ void __launch_bounds__(256) grouped_ozaki_slice_kernel(const GroupEntry* __restrict__ g,
+                                                                  const int* __restrict__ starts, int count,
                                                                   int a_blocks) {
   __shared__ double tile[32][65];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int b = blockIdx.x;
   if (b < a_blocks) {
-    const GroupEntry& e = g[find_entry<0>(g, count, b)];
+    const GroupEntry& e = g[find_entry(starts, count, b)];
     const int r = (b - e.pre_a_start) * 8 + warp;
     if (r >= e.m) return;
     const double* src = static_cast<const double*>(e.A) + (int64_t)r * e.lda;
@@ -215,7 +159,7 @@ __global__ void __launch_bounds__(256) grouped_ozaki_slice_kernel(const GroupEnt
   // one 32 (k) x 64 (n) tile of some B: 16 lanes load 64 doubles of a row; a
   // lane slices 4 consecutive k of one column (one 4-byte store per slice)
   b -= a_blocks;
-  const GroupEntry& e = g[find_entry<1>(g, count, b)];
+  const GroupEntry& e = g[find_entry(starts + count, count, b)];
   const int t = b - e.pre_b_start;
   const int tiles_n64 = (e.n + 63) / 64;
   const int k0 = (t / tiles_n64) * 32, n0 = (t % tiles_n64) * 64;
@@ -261,17 +205,21 @@ namespace {
 size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Tile of a grouped launch (descriptor tile id, 0 = the tuner's cached choice
-// for this batch, else 1):
-//   BF16X3  1 = 128 x 128 promoted, 2 = 128 x 256 promoted, 3 = 256 x 256 CTA pair
+// for this batch, else automatic_tile()):
+//   BF16X3  1 = 128 x 128 promoted, 2 = 128 x 256 promoted, 3 = 256 x 256 CTA pair;
+//           4 / 5 = 256 x 128 / 256 x 256 CTA pair, bit-identical to 1
 //   BF16X6  1 = 128 x 128, 2 = 256 x 256 CTA pair (split release)
 //   OZAKI   1 = 128 x ozaki_bn(slices)
 struct GTile {
   int id, tile_m, bn, pair;
 };
 bool grouped_tile(int kind, int slices, int id, GTile& g) {
-  if (id == 0) id = 1;
-  if (kind == 0 && id >= 1 && id <= 3) {
-    g = id == 1 ? GTile{1, 128, 128, 0} : id == 2 ? GTile{2, 128, 256, 0} : GTile{3, 256, 256, 1};
+  if (kind == 0 && id >= 1 && id <= 5) {
+    g = id == 1   ? GTile{1, 128, 128, 0}
+        : id == 2 ? GTile{2, 128, 256, 0}
+        : id == 3 ? GTile{3, 256, 256, 1}
+        : id == 4 ? GTile{4, 256, 128, 1}
+                  : GTile{5, 256, 256, 1};
     return true;
   }
   if (kind == 1 && id >= 1 && id <= 2) {
@@ -287,13 +235,90 @@ bool grouped_tile(int kind, int slices, int id, GTile& g) {
 
 struct Layout {
   int kind, slices, bn, tile_m, pair, tile;
-  size_t table_bytes, total_bytes;
+  size_t table_bytes, total_bytes, off_starts, off_units;
   std::vector<GroupEntry> entries;  // pointers relative to the workspace base (offsets)
   std::vector<size_t> off_a, off_b, off_ea, off_eb;
-  int total_tiles, pre_a, pre_b, exp_a, exp_b;
+  std::vector<int2> units;  // work list
+  int slots;                // CTAs (pairs) that walk it
+  int pre_a, pre_b, exp_a, exp_b;
 };
 
-cucosma_status layout(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr, int count, Layout& L,
+// Work list of a tile: the units (tiles of the problems, longest K first) in
+// rounds of one per slot, each round's longest to the slot with the least work
+// so far, work being k-blocks plus a constant for the epilogue.  Handing them
+// out round-robin left the busiest slot a third above the mean on 64 problems
+// of the benchmark's distribution (601 against 452 k-blocks of 32).  Loads less
+// than one unit apart count as equal and keep the slots in order, so that
+// neighbouring tiles of a problem still run on neighbouring SMs (sorted by the
+// exact loads, the 512-problem batch lost 8 % to L2).  Returns the busiest
+// slot's work.
+constexpr int kUnitOverhead = 4;  // k-blocks
+int64_t work_list(const cucosma_gemm_problem* pr, const std::vector<int>& order, int tile_m, int bn, int slots,
+                  std::vector<int2>* list) {
+  std::vector<int64_t> load(slots, 0);
+  std::vector<std::pair<int64_t, int>> round(slots);  // (load in units, slot), least first
+  int next = slots;                                   // slots of this round served so far
+  for (int e = 0; e < (int)order.size(); ++e) {
+    const cucosma_gemm_problem& p = pr[order[e]];
+    const int tiles = (int)(ceil_div(p.m, tile_m) * ceil_div(p.n, bn));
+    const int64_t work = ceil_div(p.k, 32) + kUnitOverhead;
+    for (int t = 0; t < tiles; ++t) {
+      if (next == slots) {
+        const int64_t least = *std::min_element(load.begin(), load.end());
+        for (int s = 0; s < slots; ++s) round[s] = {(load[s] - least) / work, s};
+        std::sort(round.begin(), round.end());
+        if (list) list->resize(list->size() + slots, int2{-1, 0});
+        next = 0;
+      }
+      const int s = round[next++].second;
+      load[s] += work;
+      if (list) (*list)[list->size() - slots + s] = int2{e, t};
+    }
+  }
+  return *std::max_element(load.begin(), load.end());
+}
+
+// CTAs (pairs) of a grouped launch with `units` units.
+int launch_slots(int64_t units, int pair, int sms) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(units, pair ? max_pair_clusters<Bf16x3PairSmall>(sms) : sms));
+}
+
+int64_t unit_count(const cucosma_gemm_problem* pr, int count, int tile_m, int bn) {
+  int64_t n = 0;
+  for (int i = 0; i < count; ++i) n += ceil_div(pr[i].m, tile_m) * ceil_div(pr[i].n, bn);
+  return n;
+}
+
+// Automatic tile: of the tiles that give bit-identical results, the one whose
+// busiest slot finishes first at these times per k-block of a slot (us, fitted
+// to batches of 16, 64 and 512 of the benchmark's distribution on B200: GEMM
+// kernel 2.69 ms on 128 x 128 tiles, 2.50 on 256 x 128 pairs, 2.39 on
+// 256 x 256 for the 512; L2 feeds the SMs about 7 TB/s, which bounds the
+// narrower tiles).  Batches of at most two waves keep the 128 x 128 tile.
+int automatic_tile(int kind, const cucosma_gemm_problem* pr, const std::vector<int>& order, int sms) {
+  struct Option {
+    int id, tile_m, bn, pair;
+    double us;
+  };
+  static constexpr Option kV3[] = {{1, 128, 128, 0, 0.60}, {4, 256, 128, 1, 0.50}, {5, 256, 256, 1, 0.83}};
+  static constexpr Option kV6[] = {{1, 128, 128, 0, 0.90}, {2, 256, 256, 1, 1.30}};
+  if (kind == 2) return 1;
+  const int count = (int)order.size();
+  if (unit_count(pr, count, 128, 128) <= 2 * (int64_t)sms) return 1;
+  int best = 1;
+  double t_best = 1e300;
+  for (const Option* o = kind == 0 ? kV3 : kV6, *end = o + (kind == 0 ? 3 : 2); o != end; ++o) {
+    const int slots = launch_slots(unit_count(pr, count, o->tile_m, o->bn), o->pair, sms);
+    const double t = o->us * (double)work_list(pr, order, o->tile_m, o->bn, slots, nullptr);
+    if (t < t_best) {
+      t_best = t;
+      best = o->id;
+    }
+  }
+  return best;
+}
+
+cucosma_status layout(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr, int count, int sms, Layout& L,
                       int tile = -1) {
   if (!d || !pr || count <= 0) return CUCOSMA_STATUS_INVALID_VALUE;
   if (d->flags != 0 || d->epilogue < 0 || d->epilogue > CUCOSMA_EPILOGUE_RELU) return CUCOSMA_STATUS_INVALID_VALUE;
@@ -309,8 +334,20 @@ cucosma_status layout(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr
   } else {
     return CUCOSMA_STATUS_NOT_SUPPORTED;  // the grouped launch is a tensor-core path
   }
+  for (int i = 0; i < count; ++i) {
+    const cucosma_gemm_problem& q = pr[i];
+    if (q.m <= 0 || q.n <= 0 || q.k <= 0) return CUCOSMA_STATUS_INVALID_VALUE;
+    if (q.m > INT32_MAX || q.n > INT32_MAX || q.k > INT32_MAX) return CUCOSMA_STATUS_INVALID_VALUE;
+  }
+  // Table order: K descending (stable): the long-K tiles are dealt out first
+  // and the short ones even out the end.
+  std::vector<int> order(count);
+  for (int i = 0; i < count; ++i) order[i] = i;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return pr[a].k > pr[b].k; });
+  if (tile < 0) tile = d->tile;
   GTile g{};
-  if (!grouped_tile(L.kind, L.slices, tile >= 0 ? tile : d->tile, g)) return CUCOSMA_STATUS_NOT_SUPPORTED;
+  if (!grouped_tile(L.kind, L.slices, tile > 0 ? tile : automatic_tile(L.kind, pr, order, sms), g))
+    return CUCOSMA_STATUS_NOT_SUPPORTED;
   L.bn = g.bn;
   L.tile_m = g.tile_m;
   L.pair = g.pair;
@@ -318,24 +355,23 @@ cucosma_status layout(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr
   const int es_in = L.kind == 2 ? 8 : 4;
   const int es_pl = L.kind == 2 ? 1 : 2;
   const int64_t kmax_exact = ((int64_t)2147483647 / ((int64_t)L.slices * 127 * 127)) / 32 * 32;
-  L.table_bytes = al256(sizeof(GroupEntry) * (size_t)count);
+  const int64_t units = unit_count(pr, count, L.tile_m, L.bn);
+  if (units > (1 << 26)) return CUCOSMA_STATUS_NOT_SUPPORTED;  // (the work list: 2^26 tiles are 8 bytes each)
+  L.slots = launch_slots(units, L.pair, sms);
+  L.units.clear();
+  work_list(pr, order, L.tile_m, L.bn, L.slots, &L.units);
+  L.off_starts = al256(sizeof(GroupEntry) * (size_t)count);
+  L.off_units = L.off_starts + al256(sizeof(int) * 4 * (size_t)count);
+  L.table_bytes = L.off_units + al256(sizeof(int2) * L.units.size());
   size_t off = L.table_bytes;
   L.entries.assign(count, GroupEntry{});
   L.off_a.resize(count);
   L.off_b.resize(count);
   L.off_ea.resize(count);
   L.off_eb.resize(count);
-  // Table order: K descending (stable).  The persistent kernel hands units out
-  // round-robin in table order, so the long-K tiles are spread over the CTAs
-  // first and the short ones even out the end.
-  std::vector<int> order(count);
-  for (int i = 0; i < count; ++i) order[i] = i;
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return pr[a].k > pr[b].k; });
-  int tiles = 0, pa = 0, pb = 0, xa = 0, xb = 0;
+  int pa = 0, pb = 0, xa = 0, xb = 0;
   for (int i = 0; i < count; ++i) {
     const cucosma_gemm_problem& q = pr[order[i]];
-    if (q.m <= 0 || q.n <= 0 || q.k <= 0) return CUCOSMA_STATUS_INVALID_VALUE;
-    if (q.m > INT32_MAX || q.n > INT32_MAX || q.k > INT32_MAX) return CUCOSMA_STATUS_INVALID_VALUE;
     if (q.lda < q.k || q.ldb < q.n || q.ldc < q.n || !q.A || !q.B || !q.C) return CUCOSMA_STATUS_INVALID_VALUE;
     if ((reinterpret_cast<uintptr_t>(q.A) | reinterpret_cast<uintptr_t>(q.B) | reinterpret_cast<uintptr_t>(q.C)) & 15)
       return CUCOSMA_STATUS_MISALIGNED;
@@ -349,8 +385,6 @@ cucosma_status layout(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr
     e.kblocks = (int)ceil_div(q.k, 32);
     e.tiles_m = (int)ceil_div(q.m, L.tile_m);
     e.tiles_n = (int)ceil_div(q.n, L.bn);
-    e.tile_start = tiles;
-    tiles += e.tiles_m * e.tiles_n;
     e.C = q.C;
     e.ldc = q.ldc;
     e.A = q.A;
@@ -358,9 +392,9 @@ cucosma_status layout(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr
     e.lda = q.lda;
     e.ldb = q.ldb;
     e.pre_a_start = pa;
-    pa += (int)ceil_div(q.m, 8);
+    pa += (int)(L.kind == 2 ? ceil_div(q.m, 8) : ceil_div(q.m * ceil_div(e.kpad / 8, kRowUnit), kRowsPerBlock));
     e.pre_b_start = pb;
-    pb += L.kind == 2 ? (int)(ceil_div(e.kpad, 32) * ceil_div(q.n, 64)) : (int)(ceil_div(e.kpad, 64) * ceil_div(q.n, 64));
+    pb += L.kind == 2 ? (int)(ceil_div(e.kpad, 32) * ceil_div(q.n, 64)) : (int)(ceil_div(e.kpad, 64 * kStripTiles) * ceil_div(q.n, 64));
     e.exp_a_start = xa;
     xa += (int)ceil_div(q.m, 8);
     e.exp_b_start = xb;
@@ -376,7 +410,6 @@ cucosma_status layout(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr
       off = al256(off + (size_t)q.n * 4);
     }
   }
-  L.total_tiles = tiles;
   L.pre_a = pa;
   L.pre_b = pb;
   L.exp_a = xa;
@@ -396,10 +429,16 @@ extern "C" cucosma_status cucosma_grouped_workspace_size(const cucosma_gemm_desc
                                                          const cucosma_gemm_problem* problems, int count,
                                                          size_t* bytes) {
   if (!bytes) return CUCOSMA_STATUS_INVALID_VALUE;
+  const DeviceInfo* di = device_info();
+  const int sms = di ? di->sms : 148;  // (sizes can be asked for without a device)
   Layout L;
-  cucosma_status s = layout(d, problems, count, L);
+  cucosma_status s = layout(d, problems, count, sms, L);
   if (s != CUCOSMA_STATUS_SUCCESS) return s;
   *bytes = L.total_bytes;
+  // a plan with tile 0 may take the tuner's tile, whose work list can be longer
+  const int tuned = d->tile == 0 && di ? grouped_tuned_tile(d, problems, count, di) : 0;
+  if (tuned > 0 && layout(d, problems, count, sms, L, tuned) == CUCOSMA_STATUS_SUCCESS)
+    *bytes = std::max(*bytes, L.total_bytes);
   return CUCOSMA_STATUS_SUCCESS;
 }
 
@@ -419,7 +458,7 @@ extern "C" cucosma_status cucosma_grouped_plan_create(const cucosma_gemm_desc* d
     from_cache = tile > 0;
   }
   Layout L;
-  cucosma_status s = layout(d, problems, count, L, tile);
+  cucosma_status s = layout(d, problems, count, di->sms, L, tile);
   if (s != CUCOSMA_STATUS_SUCCESS) return s;
   if (!workspace || workspace_bytes < L.total_bytes) return CUCOSMA_STATUS_WORKSPACE_TOO_SMALL;
   if (reinterpret_cast<uintptr_t>(workspace) & 255) return CUCOSMA_STATUS_MISALIGNED;
@@ -446,15 +485,26 @@ extern "C" cucosma_status cucosma_grouped_plan_create(const cucosma_gemm_desc* d
     }
     if (!ok) return CUCOSMA_STATUS_LAUNCH_FAILED;
   }
-  if (cudaMemcpy(workspace, L.entries.data(), sizeof(GroupEntry) * (size_t)count, cudaMemcpyHostToDevice) !=
-      cudaSuccess)
+  std::vector<uint8_t> image(L.table_bytes, 0);
+  std::memcpy(image.data(), L.entries.data(), sizeof(GroupEntry) * (size_t)count);
+  int* starts = reinterpret_cast<int*>(image.data() + L.off_starts);
+  for (int i = 0; i < count; ++i) {
+    const GroupEntry& e = L.entries[i];
+    starts[i] = e.pre_a_start;
+    starts[count + i] = e.pre_b_start;
+    starts[2 * count + i] = e.exp_a_start;
+    starts[3 * count + i] = e.exp_b_start;
+  }
+  std::memcpy(image.data() + L.off_units, L.units.data(), sizeof(int2) * L.units.size());
+  if (cudaMemcpy(workspace, image.data(), L.table_bytes, cudaMemcpyHostToDevice) != cudaSuccess)
     return CUCOSMA_STATUS_LAUNCH_FAILED;
   auto* p = new cucosma_grouped_plan_st;
   p->desc = *d;
   p->count = count;
   p->kind = L.kind;
   p->slices = L.slices;
-  p->total_tiles = L.total_tiles;
+  p->total_tiles = (int)L.units.size();
+  p->grid = L.slots * (L.pair ? 2 : 1);
   p->tile = L.tile;
   p->tile_m = L.tile_m;
   p->tile_n = L.bn;
@@ -467,6 +517,8 @@ extern "C" cucosma_status cucosma_grouped_plan_create(const cucosma_gemm_desc* d
   cudaGetDevice(&p->device);
   p->workspace = workspace;
   p->table = reinterpret_cast<GroupEntry*>(workspace);
+  p->starts = reinterpret_cast<const int*>(w + L.off_starts);
+  p->unit_list = reinterpret_cast<const int2*>(w + L.off_units);
   *plan = p;
   return CUCOSMA_STATUS_SUCCESS;
 }
@@ -489,8 +541,8 @@ extern "C" cucosma_status cucosma_grouped_plan_get_tile(cucosma_grouped_plan pla
 template <int S>
 static cudaError_t launch_ozaki_grouped(const cucosma_grouped_plan_st& pl, const TcParams& p, const CUtensorMap& dummy,
                                         int grid, cudaStream_t st) {
-  grouped_ozaki_slice_kernel<S><<<pl.pre_a_blocks + pl.pre_b_blocks, 256, 0, st>>>(pl.table, pl.count,
-                                                                                   pl.pre_a_blocks);
+  grouped_ozaki_slice_kernel<S><<<pl.pre_a_blocks + pl.pre_b_blocks, 256, 0, st>>>(pl.table, pl.starts,
+                                                                                   pl.count, pl.pre_a_blocks);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   prof_begin(st);
@@ -510,37 +562,41 @@ extern "C" cucosma_status cucosma_gemm_grouped(cucosma_grouped_plan plan, void* 
   p.alpha = plan->desc.alpha;
   p.beta = plan->desc.beta;
   p.groups = plan->table;
+  p.unit_list = plan->unit_list;
   p.ngroups = plan->count;
   p.total_tiles = plan->total_tiles;
   p.splits = 1;
   wait_ctl(di, &p.ctl.status, &p.ctl.timeout_ns);
-  const int grid = std::min(plan->total_tiles, di->sms);
+  const int grid = plan->grid;  // the CTAs the work list was made for
   CUtensorMap dummy;
   std::memset(&dummy, 0, sizeof(dummy));
   cudaError_t e;
   if (plan->kind != 2) {
     const unsigned blocks = (unsigned)(plan->pre_a_blocks + plan->pre_b_blocks);
     if (plan->slices == 3)
-      grouped_split_bf16_kernel<3><<<blocks, 256, 0, st>>>(plan->table, plan->count, plan->pre_a_blocks);
+      grouped_split_bf16_kernel<3><<<blocks, 256, 0, st>>>(plan->table, plan->starts, plan->count, plan->pre_a_blocks);
     else
-      grouped_split_bf16_kernel<2><<<blocks, 256, 0, st>>>(plan->table, plan->count, plan->pre_a_blocks);
+      grouped_split_bf16_kernel<2><<<blocks, 256, 0, st>>>(plan->table, plan->starts, plan->count, plan->pre_a_blocks);
     e = cudaGetLastError();
     if (e != cudaSuccess) return CUCOSMA_STATUS_LAUNCH_FAILED;
-    auto pair_grid = [&](int clusters) { return 2 * std::max(1, std::min(plan->total_tiles, clusters)); };
     prof_begin(st);
     if (plan->kind == 1)
       e = plan->tile == 2
-              ? launch<Bf16x6PairWide>(dummy, dummy, p, pair_grid(max_pair_clusters<Bf16x6PairWide>(di->sms)), st)
+              ? launch<Bf16x6PairWide>(dummy, dummy, p, grid, st)
               : launch<Bf16x6>(dummy, dummy, p, grid, st);
     else
-      e = plan->tile == 3   ? launch<Bf16x3Pair>(dummy, dummy, p, pair_grid(max_pair_clusters<Bf16x3Pair>(di->sms)), st)
+      e = plan->tile == 5
+              ? launch<Bf16x3PairSplit>(dummy, dummy, p, grid, st)
+          : plan->tile == 4
+              ? launch<Bf16x3PairSmall>(dummy, dummy, p, grid, st)
+          : plan->tile == 3 ? launch<Bf16x3Pair>(dummy, dummy, p, grid, st)
           : plan->tile == 2 ? launch<Bf16x3>(dummy, dummy, p, grid, st)
                             : launch<Bf16x3Promoted>(dummy, dummy, p, grid, st);
     prof_end(st);
     note_launches(2);
   } else {
-    grouped_ozaki_exp_kernel<<<plan->exp_a_blocks + plan->exp_b_blocks, 256, 0, st>>>(plan->table, plan->count,
-                                                                                      plan->exp_a_blocks);
+    grouped_ozaki_exp_kernel<<<plan->exp_a_blocks + plan->exp_b_blocks, 256, 0, st>>>(plan->table, plan->starts,
+                                                                                      plan->count, plan->exp_a_blocks);
     e = cudaGetLastError();
     if (e != cudaSuccess) return CUCOSMA_STATUS_LAUNCH_FAILED;
     switch (plan->slices) {

@@ -21,8 +21,7 @@ namespace tc {
 
 // One problem of a grouped launch, stored in the workspace.  The tensor maps
 // describe this problem's operand planes (they live in global memory; the
-// TMA unit reads them there).  Tiles of all problems are numbered
-// consecutively: this problem owns [tile_start, tile_start + tiles_m*tiles_n).
+// TMA unit reads them there).
 struct alignas(64) GroupEntry {
   CUtensorMap tmA, tmB;
   void* C;
@@ -30,7 +29,7 @@ struct alignas(64) GroupEntry {
   const int32_t* ea;  // Ozaki exponents of this problem (null for BF16)
   const int32_t* eb;
   int m, n, k, kblocks;
-  int tiles_m, tiles_n, tile_start, pad0;
+  int tiles_m, tiles_n;
   // operand pre-pass: sources, destination planes, first pre-pass block of
   // this problem for the A rows / B tiles / exponent passes
   const void* A;
@@ -73,9 +72,12 @@ struct TcParams {
   WaitCtl ctl;
   int skip_stage;  // test hook: ring position whose loads the producer omits (-1: none)
   // Grouped launch: when ngroups > 0 the problems come from groups[] (all
-  // other per-problem fields above are ignored) and units = total_tiles.
+  // other per-problem fields above are ignored).
   const GroupEntry* groups;
-  int ngroups, total_tiles;
+  // Work list: position i * slots + s is the i-th unit of CTA (pair) s, as
+  // {problem, tile of the problem}; problem -1 where a slot has no more.
+  const int2* unit_list;
+  int ngroups, total_tiles;  // total_tiles: positions
   // Optional device-side gate: the kernel runs only if *gate == gate_value
   // (the adaptive Ozaki call's slice count, chosen on the device).
   const int* gate;

@@ -67,10 +67,11 @@ __device__ __forceinline__ void unit_coords(int unit, int tiles, int tiles_m, in
 }
 
 // Unit -> (operand descriptors, tile, K range).  Single problem: banded
-// raster over tiles x K splits.  Grouped: the problem owning the unit is
-// found by binary search over the tile_start column of the problem table;
-// its tiles are visited down M first, then across N.
-__device__ __forceinline__ void resolve_unit(const TcParams& p, const CUtensorMap* tmA, const CUtensorMap* tmB,
+// raster over tiles x K splits.  Grouped: the plan's work list names the
+// problem and the tile (finding the problem here by binary search was nine
+// dependent loads for every role and unit); tiles are numbered down M first,
+// then across N.  Returns false at an empty position of the work list.
+__device__ __forceinline__ bool resolve_unit(const TcParams& p, const CUtensorMap* tmA, const CUtensorMap* tmB,
                                              int unit, Unit& u) {
   if (p.ngroups == 0) {
     unit_coords(unit, p.tiles_m * p.tiles_n, p.tiles_m, p.tiles_n, p.band, u.z, u.tm, u.tn);
@@ -80,16 +81,10 @@ __device__ __forceinline__ void resolve_unit(const TcParams& p, const CUtensorMa
     u.tb = tmB;
     u.group = -1;
   } else {
-    int lo = 0, hi = p.ngroups - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (p.groups[mid].tile_start <= unit)
-        lo = mid;
-      else
-        hi = mid - 1;
-    }
-    const GroupEntry& e = p.groups[lo];
-    const int local = unit - e.tile_start;
+    const int2 item = p.unit_list[unit];
+    if (item.x < 0) return false;
+    const GroupEntry& e = p.groups[item.x];
+    const int local = item.y;
     u.tm = local % e.tiles_m;
     u.tn = local / e.tiles_m;
     u.z = 0;
@@ -97,8 +92,9 @@ __device__ __forceinline__ void resolve_unit(const TcParams& p, const CUtensorMa
     u.kb1 = e.kblocks;
     u.ta = &e.tmA;
     u.tb = &e.tmB;
-    u.group = lo;
+    u.group = item.x;
   }
+  return true;
 }
 
 // With beta != 0: L2 prefetch of the C block an epilogue warp will read
@@ -327,7 +323,7 @@ __global__ void __maxnreg__(Tr::MAX_REGS)
       bool ok = true;
       for (int unit = unit0; unit < units && ok; unit += unit_step) {
         Unit u;
-        resolve_unit(p, &tmA, &tmB, unit, u);
+        if (!resolve_unit(p, &tmA, &tmB, unit, u)) continue;
         const int tm = u.tm, tn = u.tn;
         for (int kb = u.kb0; kb < u.kb1; ++kb, ++it) {
           const int s = it % ST;
@@ -380,7 +376,7 @@ __global__ void __maxnreg__(Tr::MAX_REGS)
       bool ok = true;
       for (int unit = unit0; unit < units && ok; unit += unit_step) {
         Unit u;
-        resolve_unit(p, &tmA, &tmB, unit, u);
+        if (!resolve_unit(p, &tmA, &tmB, unit, u)) continue;
         const int kb1 = u.kb1;
         for (int cs = u.kb0; cs < kb1 && ok; cs += chunk, ++ci) {
           const int ce = min(kb1, cs + chunk);
@@ -448,7 +444,7 @@ __global__ void __maxnreg__(Tr::MAX_REGS)
       bool ok = true;
       for (int unit = unit0; unit < units && ok; unit += unit_step) {
         Unit u;
-        resolve_unit(p, &tmA, &tmB, unit, u);
+        if (!resolve_unit(p, &tmA, &tmB, unit, u)) continue;
         if constexpr (Tr::PROMOTE) {
           for (int cs = u.kb0; cs < u.kb1 && ok; cs += chunk, ++ci) {
             if constexpr (Tr::SPLIT)
@@ -484,7 +480,7 @@ __global__ void __maxnreg__(Tr::MAX_REGS)
     bool ok = true;
     for (int unit = unit0; unit < units && ok; unit += unit_step) {
       Unit u;
-      resolve_unit(p, &tmA, &tmB, unit, u);
+      if (!resolve_unit(p, &tmA, &tmB, unit, u)) continue;
       const int z = u.z;
       const int row0 = u.tm * TILE_M + (int)rank * 128 + 32 * q;
       const int col0 = u.tn * BN;
@@ -493,7 +489,7 @@ __global__ void __maxnreg__(Tr::MAX_REGS)
       auto prefetch_unit = [&](int un) {
         if (un >= units) return;
         Unit v;
-        resolve_unit(p, &tmA, &tmB, un, v);
+        if (!resolve_unit(p, &tmA, &tmB, un, v)) return;
         prefetch_c_block(out_ctx(p, v), v.tm * TILE_M + (int)rank * 128 + 32 * q,
                          v.tn * BN + colsub, W, Tr::kInt8 ? 8 : 4, lane);
       };
@@ -1260,6 +1256,15 @@ struct Bf16x3PairDirect : TraitsBase<3, 256, 64, 2, 2, 1, false, EpiF32, false, 
 };
 struct Bf16x3Pair128 : TraitsBase<3, 128, 64, 2, 2, 1, false, EpiF32, true, kPromoteChunk, 8, 0, true> {
   static constexpr TermTable<3> kTerms{{1, 0, 0}, {0, 1, 0}, {0, 0, 0}, {true, false, false}};
+};
+// The 256 x 128 pair with Bf16x3Promoted's two accumulators (bit-identical
+// results): the pair reads each B column from one CTA's shared memory, which
+// bounds the 128 x 128 tile.
+struct Bf16x3PairSmall : TraitsBase<3, 128, 64, 2, 2, 2, false, EpiF32, true, kPromoteChunk, 8, 0, true> {
+  static constexpr TermTable<3> kTerms{{1, 0, 0}, {0, 1, 0}, {1, 1, 0}, {true, false, true}};
+};
+struct Bf16x3PairSplit : TraitsBase<3, 256, 64, 2, 2, 2, false, EpiF32, true, kPromoteChunk, 8, 0, true, true> {
+  static constexpr TermTable<3> kTerms{{1, 0, 0}, {0, 1, 0}, {1, 1, 0}, {true, false, true}};
 };
 struct Bf16x6Pair : TraitsBase<6, 128, 64, 3, 3, 2, false, EpiF32, true, kPromoteChunk, 8, 0, true> {
   static constexpr TermTable<6> kTerms{

@@ -263,10 +263,12 @@ CUCOSMA_API cucosma_status cucosma_grouped_plan_create(const cucosma_gemm_desc* 
 CUCOSMA_API cucosma_status cucosma_gemm_grouped(cucosma_grouped_plan plan, void* stream);
 CUCOSMA_API cucosma_status cucosma_grouped_plan_destroy(cucosma_grouped_plan plan);
 /* The plan's tile: descriptor tile id (BF16X3 1 = 128 x 128 promoted,
- * 2 = 128 x 256 promoted, 3 = 256 x 256 CTA pair; BF16X6 1 = 128 x 128,
+ * 2 = 128 x 256 promoted, 3 = 256 x 256 CTA pair, 4 / 5 = 256 x 128 / 256 x
+ * 256 CTA pair with the results of 1 bit for bit; BF16X6 1 = 128 x 128,
  * 2 = 256 x 256 pair; Ozaki 1), its rows and columns, and whether it came
  * from the tuning cache (descriptor tile 0 with a cucosma_tune_grouped entry
- * for this batch; otherwise tile 0 means 1). */
+ * for this batch; otherwise tile 0 takes the fastest expected of the tiles
+ * whose results equal tile 1's: BF16X3 1, 4 or 5, BF16X6 1 or 2). */
 CUCOSMA_API cucosma_status cucosma_grouped_plan_get_tile(cucosma_grouped_plan plan, int32_t* tile, int32_t* tile_m,
                                                          int32_t* tile_n, int32_t* from_cache);
 
