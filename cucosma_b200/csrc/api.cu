@@ -141,8 +141,8 @@ static int simt_bk(int dtype) { return dtype == CUCOSMA_R_32F ? simt::Cfg<float>
 
 // Modelled time (us) of the tile kernel with bm-row CTA tiles, `tiles` output
 // tiles and `s` K splits of `kblocks` 16-deep k-blocks in all, plus the
-// split-K reduction (s partial planes of per_split bytes in and out at HBM
-// speed, and a launch).  Fitted to B200 measurements of both FP32 tile
+// split-K reduction (inside a cluster where cluster_splits(); else s partial
+// planes of per_split bytes in and out at HBM speed, and a launch).  Fitted to B200 measurements of both FP32 tile
 // heights over square, flat, large-N and large-K shapes:
 //   * a 128 x 128 x 16 k-block step takes kUnitUs of an SM holding 16 warps
 //     (FP64: kUnitUsF64 a CTA, one CTA an SM);
@@ -154,12 +154,13 @@ static int simt_bk(int dtype) { return dtype == CUCOSMA_R_32F ? simt::Cfg<float>
 //   * whole waves of resident CTAs run at full occupancy, and the last,
 //     partial wave at the occupancy it leaves.
 namespace {
-constexpr double kUnitUs = 1.45, kUnitUsF64 = 2.4, kTile64Factor = 0.95;
+constexpr double kUnitUs = 1.45, kUnitUsF64 = 2.4, kTile64Factor = 0.95, kClusterUs = 1.75;
 double occupancy_rate(int warps) {
   return warps >= 16 ? 1.0 : warps >= 14 ? 0.99 : warps >= 12 ? 0.97 : warps >= 10 ? 0.95 : warps >= 8 ? 0.91
                        : warps >= 6 ? 0.8 : 0.71;
 }
-double native_time_us(int bm, bool fp32, int64_t tiles, int64_t s, int64_t kblocks, int sms, size_t per_split) {
+double native_time_us(int bm, bool fp32, int64_t tiles, int64_t s, int64_t kblocks, int sms, size_t per_split,
+                      bool clusters) {
   const int per_sm = fp32 ? (bm == 64 ? simt::SgemmShape<64>::kCtasPerSm : simt::SgemmShape<128>::kCtasPerSm)
                           : simt::Cfg<double>::CTAS_PER_SM;
   const int warps_per_cta = fp32 ? bm / 16 : 16;  // FP64: one CTA fills its SM's FP64 rate
@@ -172,7 +173,7 @@ double native_time_us(int bm, bool fp32, int64_t tiles, int64_t s, int64_t kbloc
     const int r = (int)ceil_div(rest, (int64_t)sms);  // CTAs on the busiest SM of the last wave
     t += kbs * r * step / occupancy_rate(r * warps_per_cta);
   }
-  if (s > 1) t += 2.0 + 2.0 * (double)s * (double)per_split / 6.0e6;
+  if (s > 1) t += clusters && simt::cluster_splits(tiles, s) ? kClusterUs : 2.0 + 2.0 * (double)s * (double)per_split / 6.0e6;
   return t;
 }
 }  // namespace
@@ -191,20 +192,24 @@ NativePlan plan_native(const cucosma_gemm_desc* d, int sms, size_t max_ws) {
   if (fp32 && d->tile == 2) heights[0] = 64;
   else if (fp32 && d->tile == 0) nh = 2;
   const int64_t tiles_n = ceil_div(d->n, simt::BN);
+  const bool clusters = max_ws == SIZE_MAX;
   int64_t splits = d->split_k;
   int bm = heights[0];
   if (splits <= 0) {
     // The (height, split) pair with the smallest modelled time wins; splits
-    // keep >= 4 k-blocks each and fit max_ws, and a candidate must beat the
-    // best so far by 2 % (ties keep the taller tile and the smaller split).
-    const int64_t smax = std::max<int64_t>(1, std::min<int64_t>(kblocks / 4, 512));
+    // keep >= 4 k-blocks each (inside a cluster one is enough) and fit max_ws,
+    // and a candidate must beat the best so far by 2 % (ties keep the taller
+    // tile and the smaller split).
+    const int64_t smax = std::max<int64_t>(clusters ? std::min<int64_t>(kblocks, simt::kMaxCluster) : 1,
+                                           std::min<int64_t>(kblocks / 4, 512));
     double best = 1e300;
     splits = 1;
     for (int h = 0; h < nh; ++h) {
       const int64_t tiles = ceil_div(d->m, heights[h]) * tiles_n;
       for (int64_t s = 1; s <= smax; ++s) {
         if (s > 1 && (size_t)s * per_split > max_ws) break;
-        const double t = native_time_us(heights[h], fp32, tiles, s, kblocks, sms, per_split);
+        if (s > 1 && s > kblocks / 4 && !simt::cluster_splits(tiles, s)) break;
+        const double t = native_time_us(heights[h], fp32, tiles, s, kblocks, sms, per_split, clusters);
         if (t < best * 0.98) {
           best = t;
           splits = s;
@@ -215,8 +220,8 @@ NativePlan plan_native(const cucosma_gemm_desc* d, int sms, size_t max_ws) {
   } else if (nh == 2) {
     // forced split: the height with the smaller modelled time
     const int64_t s = std::min<int64_t>(splits, kblocks);
-    const double t128 = native_time_us(128, fp32, ceil_div(d->m, 128) * tiles_n, s, kblocks, sms, per_split);
-    const double t64 = native_time_us(64, fp32, ceil_div(d->m, 64) * tiles_n, s, kblocks, sms, per_split);
+    const double t128 = native_time_us(128, fp32, ceil_div(d->m, 128) * tiles_n, s, kblocks, sms, per_split, clusters);
+    const double t64 = native_time_us(64, fp32, ceil_div(d->m, 64) * tiles_n, s, kblocks, sms, per_split, clusters);
     bm = t64 < t128 * 0.98 ? 64 : 128;
   }
   p.bm = bm;
@@ -231,7 +236,8 @@ NativePlan plan_native(const cucosma_gemm_desc* d, int sms, size_t max_ws) {
   int sw = d->swizzle > 0 ? d->swizzle : 1;
   p.swizzle = sw;
   p.ldw = round_up(d->n, vec);
-  p.ws_bytes = p.splits > 1 ? (size_t)p.splits * (size_t)d->m * (size_t)p.ldw * es : 0;
+  p.cluster = clusters && simt::cluster_splits((int64_t)p.tiles_m * p.tiles_n, p.splits);
+  p.ws_bytes = p.splits > 1 && !p.cluster ? (size_t)p.splits * (size_t)d->m * (size_t)p.ldw * es : 0;
   return p;
 }
 
@@ -262,7 +268,9 @@ static cucosma_status run_native(const cucosma_gemm_desc* d, const NativePlan& p
   p.gate = gate;
   p.gate_value = gate_value;
   wait_ctl(di, &p.ctl.status, &p.ctl.timeout_ns);
-  if (pl.splits > 1) {
+  const bool partial = pl.splits > 1 && !pl.cluster;
+  p.cluster = pl.cluster;
+  if (partial) {
     p.partial = 1;
     p.out = ws;
     p.ldo = pl.ldw;
@@ -275,8 +283,8 @@ static cucosma_status run_native(const cucosma_gemm_desc* d, const NativePlan& p
   if (profile) prof_begin(st);
   if (simt::launch_gemm<T>(tmA, tmB, p, pl.bm, st) != cudaSuccess) return CUCOSMA_STATUS_LAUNCH_FAILED;
   if (profile) prof_end(st);
-  note_launches(pl.splits > 1 ? 2 : 1);
-  if (pl.splits > 1) {
+  note_launches(partial ? 2 : 1);
+  if (partial) {
     if (simt::launch_reduce<T>(static_cast<const T*>(ws), p.ws_split_stride, pl.ldw, pl.splits, C, d->ldc, p.m, p.n,
                                d->alpha, d->beta, d->epilogue, di->sms, st, gate, gate_value) != cudaSuccess)
       return CUCOSMA_STATUS_LAUNCH_FAILED;
@@ -498,7 +506,7 @@ extern "C" cucosma_status cucosma_gemm_get_plan(const cucosma_gemm_desc* d, cuco
     info->splits = pl.splits;
     info->band = pl.swizzle;
     info->slices = 1;
-    info->launches = pl.splits > 1 ? 2 : 1;
+    info->launches = pl.splits > 1 && !pl.cluster ? 2 : 1;
     info->kchunk = pl.kchunk;
     info->kpad = d->k;
     info->workspace_bytes = pl.ws_bytes;

@@ -27,11 +27,13 @@ enum : int { kPrepA = 1, kPrepB = 2, kNoFused = 4 };
 struct NativePlan {
   int bm;  // CTA tile rows: 128, or 64 (FP32 only); 128 columns either way
   int tiles_m, tiles_n, splits, swizzle;
+  int cluster;  // 1: the splits are a cluster that reduces through shared memory (no workspace, no second kernel)
   int64_t kchunk, ldw;
   size_t ws_bytes;
 };
 // Plan of the tile kernel (tile height and split-K factor); an automatic
-// split-K factor is chosen so that its partial sums fit max_ws bytes.
+// split-K factor is chosen so that its partial sums fit max_ws bytes.  A plan
+// made for a limited workspace keeps all partial sums there (no clusters).
 NativePlan plan_native(const cucosma_gemm_desc* d, int sms, size_t max_ws = SIZE_MAX);
 
 cucosma_status validate(const cucosma_gemm_desc* d, const void* A, const void* B, const void* C);

@@ -12,9 +12,11 @@
 //   * FP64 (simt_dgemm_kernel) runs on FP64 tensor-core MMAs with a 64x32
 //     warp tile;
 //   * 8 warps hold a 128x128 CTA tile;
-//   * split-K writes raw partial tiles to a caller-provided workspace and a
-//     separate kernel reduces them in ascending split order (deterministic),
-//     then applies alpha/beta and the epilogue, like cosmaSplitKReduce;
+//   * the K splits of a small launch are a cluster that adds its partial tiles
+//     through distributed shared memory; others write raw partial tiles to a
+//     caller-provided workspace and a separate kernel reduces them.  Both add
+//     in ascending split order (deterministic), then apply alpha/beta and the
+//     epilogue, like cosmaSplitKReduce;
 //   * the block-index swizzle follows the reference's remap
 //     (cuCOSMAV100.cuh:2586-2603).
 #include <type_traits>
@@ -74,6 +76,57 @@ __device__ __forceinline__ void simt_store(const T (&acc)[8][8], const SimtParam
   }
 }
 
+template <typename T>
+__device__ __forceinline__ typename Vec<T>::type ld_cluster_vec(uint32_t a) {
+  if constexpr (sizeof(T) == 4) return ld_cluster_f4(a);
+  else return ld_cluster_d2(a);
+}
+
+// Split-K reduction inside a cluster (one CTA per split, rank = split): every
+// CTA has put its rows x BN partial tile in shared memory; CTA r sums the r-th
+// share of the tile's 16-byte vectors over the ranks in ascending order (the
+// order and rounding of splitk_reduce_kernel) and stores epi(alpha * sum +
+// beta * C): no trip through the workspace, no second kernel.
+template <typename T, int ROWS, int THREADS>
+__device__ __forceinline__ void cluster_reduce(const SimtParams& p, const T* tile, int m0, int n0) {
+  constexpr int VEC = Vec<T>::n, VPR = simt::BN / VEC;  // vectors per row
+  using V = typename Vec<T>::type;
+  const T alpha = (T)p.alpha, beta = (T)p.beta;
+  cluster_sync_all();  // every rank's tile is written
+  const uint32_t base = smem_u32(tile);
+  for (int v = (int)cluster_ctarank() * THREADS + (int)threadIdx.x; v < ROWS * VPR; v += p.splits * THREADS) {
+    const int r = m0 + v / VPR, c = n0 + (v % VPR) * VEC;
+    if (r >= p.m || c >= p.n) continue;
+    V part[simt::kMaxCluster];
+#pragma unroll
+    for (int z = 0; z < simt::kMaxCluster; ++z)
+      if (z < p.splits) part[z] = ld_cluster_vec<T>(mapa_shared(base + (uint32_t)(v * 16), (uint32_t)z));
+    T* sum = reinterpret_cast<T*>(&part[0]);
+#pragma unroll
+    for (int z = 1; z < simt::kMaxCluster; ++z)
+      if (z < p.splits) {
+        const T* t = reinterpret_cast<const T*>(&part[z]);
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) sum[e] += t[e];
+      }
+    T* o = reinterpret_cast<T*>(p.out) + (int64_t)r * p.ldo + c;
+    if (c + VEC <= p.n) {
+      V cv;
+      if (beta != T(0)) cv = *reinterpret_cast<const V*>(o);
+      const T* pc = reinterpret_cast<const T*>(&cv);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) sum[e] = apply_epi(combine(sum[e], alpha, beta, pc + e), p.epilogue);
+      *reinterpret_cast<V*>(o) = part[0];
+    } else {
+#pragma unroll
+      for (int e = 0; e < VEC; ++e)
+        if (c + e < p.n) o[e] = apply_epi(combine(sum[e], alpha, beta, o + e), p.epilogue);
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();  // no rank leaves while another may read its tile
+}
+
 // FP32 kernel, CTA tile BM_ x 128 with BM_ = 128 (8 warps, 4 stages, two
 // CTAs per SM) or 64 (4 warps, 3 stages, four CTAs per SM: twice the tiles
 // for shapes that leave SMs idle at 128 rows).  A TMA ring of stages; every A
@@ -84,7 +137,7 @@ __device__ __forceinline__ void simt_store(const T (&acc)[8][8], const SimtParam
 // also proves that every warp finished the previous stage, so thread 0
 // refills that stage right after it: no empty barriers, no producer wait on
 // the critical path.  128 registers a thread either way.
-template <int BM_>
+template <int BM_, bool CLUSTER>
 __global__ void __launch_bounds__(simt::SgemmShape<BM_>::kThreads, simt::SgemmShape<BM_>::kCtasPerSm)
     simt_sgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const SimtParams p) {
@@ -204,6 +257,24 @@ __global__ void __launch_bounds__(simt::SgemmShape<BM_>::kThreads, simt::SgemmSh
     if (tid == 0)
       for (int kb = max(0, issued - STAGES); kb < issued; ++kb)
         mbar_wait(&full[kb % STAGES], (kb / STAGES) & 1, kErrTimeoutDrain, p.ctl);
+    if constexpr (CLUSTER) {  // the other ranks still read this CTA's shared memory
+      __syncthreads();
+      cluster_sync_all();
+      cluster_sync_all();
+    }
+    return;
+  }
+  if constexpr (CLUSTER) {
+    __syncthreads();  // every warp has read the last stage: its memory holds the tile now
+    float* tile = reinterpret_cast<float*>(smem);  // [BM][BN] over the stages
+    static_assert(BM * BN * 4 <= STAGES * (A_STAGE + B_STAGE), "the tile fits the stages");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float* row = tile + (a_col + (i & 3) + (i >> 2) * 16) * BN + b_col;
+      *reinterpret_cast<float4*>(row) = make_float4(acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y);
+      *reinterpret_cast<float4*>(row + 32) = make_float4(acc[i][2].x, acc[i][2].y, acc[i][3].x, acc[i][3].y);
+    }
+    cluster_reduce<float, BM, Shape::kThreads>(p, tile, m0, n0);
     return;
   }
   int rows[8];
@@ -260,6 +331,7 @@ __device__ __forceinline__ void store_pair(const SimtParams& p, int r, int c, do
   }
 }
 
+template <bool CLUSTER>
 __global__ void __launch_bounds__(simt::kThreads, 1)
     simt_dgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const SimtParams p) {
@@ -375,6 +447,23 @@ __global__ void __launch_bounds__(simt::kThreads, 1)
     if (tid == 0)
       for (int kb = max(0, issued - S); kb < issued; ++kb)
         mbar_wait(&full[kb % S], (kb / S) & 1, kErrTimeoutDrain, p.ctl);
+    if constexpr (!CLUSTER) return;
+  }
+  if constexpr (CLUSTER) {
+    // (a failed CTA's tile holds sums it did not finish; the status word says so)
+    __syncwarp();
+    __syncthreads();  // every warp has read the last stage: its memory holds the tile now
+    double* tile = reinterpret_cast<double*>(smem);  // [BM][BN] over the stages
+    static_assert(BM * BN * 8 <= S * (A_STAGE + B_STAGE), "the tile fits the stages");
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          *reinterpret_cast<double2*>(tile + (wm * 64 + mt * 16 + g + 8 * h) * BN + wn * 32 + nt * 8 + 2 * t) =
+              make_double2(acc[mt][nt][2 * h], acc[mt][nt][2 * h + 1]);
+    cluster_reduce<double, BM, kThreads>(p, tile, m0, n0);
     return;
   }
 #pragma unroll
@@ -477,9 +566,13 @@ size_t smem_bytes(int bm) {
 // The GEMM kernel of each arithmetic type and CTA tile height.
 using GemmKernel = void (*)(const CUtensorMap, const CUtensorMap, const SimtParams);
 template <typename T>
-GemmKernel gemm_kernel(int bm) {
-  if constexpr (std::is_same<T, float>::value) return bm == 64 ? simt_sgemm_kernel<64> : simt_sgemm_kernel<128>;
-  else return simt_dgemm_kernel;
+GemmKernel gemm_kernel(int bm, bool cluster = false) {
+  if constexpr (std::is_same<T, float>::value) {
+    if (bm == 64) return cluster ? simt_sgemm_kernel<64, true> : simt_sgemm_kernel<64, false>;
+    return cluster ? simt_sgemm_kernel<128, true> : simt_sgemm_kernel<128, false>;
+  } else {
+    return cluster ? simt_dgemm_kernel<true> : simt_dgemm_kernel<false>;
+  }
 }
 template <typename T>
 int threads_of(int bm) {
@@ -490,16 +583,32 @@ template <typename T>
 cudaError_t launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const SimtParams& p, int bm,
                         cudaStream_t stream) {
   if (!tile_rows_supported<T>(bm)) return cudaErrorInvalidValue;
-  static std::atomic<uint64_t> attr_set[2];  // devices done, per tile height (one kernel each)
+  static std::atomic<uint64_t> attr_set[2][2];  // devices done, per tile height and cluster form (one kernel each)
   const size_t smem = smem_bytes<T>(bm);
-  cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(gemm_kernel<T>(bm)), (int)smem,
-                                   attr_set[bm == 64 ? 1 : 0]);
+  const bool cluster = p.cluster != 0;
+  cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(gemm_kernel<T>(bm, cluster)), (int)smem,
+                                   attr_set[bm == 64 ? 1 : 0][cluster ? 1 : 0]);
   if (e != cudaSuccess) return e;
   dim3 grid;
   if (p.swizzle > 1) {
     grid = dim3(p.tiles_n * p.swizzle, (unsigned)ceil_div(p.tiles_m, p.swizzle), p.splits);
   } else {
     grid = dim3(p.tiles_n, p.tiles_m, p.splits);
+  }
+  if (cluster) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads_of<T>(bm), 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = (unsigned)p.splits;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, gemm_kernel<T>(bm, true), tmA, tmB, p);
   }
   gemm_kernel<T>(bm)<<<grid, threads_of<T>(bm), smem, stream>>>(tmA, tmB, p);
   return cudaGetLastError();

@@ -307,7 +307,7 @@ static int plan_launches(const Plan& pl) {
   if (pl.kind != 2) return 2 + (pl.t.splits > 1 ? 1 : 0);  // the split of A and B, the GEMM
   if (!pl.adaptive) return 4 + (pl.t.splits > 1 ? 1 : 0);
   // prep B (2), prep A, decision, the three gated kernels and their reductions
-  return 7 + (pl.t.splits > 1) + (pl.t9.splits > 1) + (pl.native.splits > 1);
+  return 7 + (pl.t.splits > 1) + (pl.t9.splits > 1) + (pl.native.splits > 1 && !pl.native.cluster);
 }
 
 }  // namespace tc
