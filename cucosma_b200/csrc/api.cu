@@ -155,6 +155,8 @@ static int simt_bk(int dtype) { return dtype == CUCOSMA_R_32F ? simt::Cfg<float>
 //     partial wave at the occupancy it leaves.
 namespace {
 constexpr double kUnitUs = 1.45, kUnitUsF64 = 2.4, kTile64Factor = 0.95, kClusterUs = 1.75;
+constexpr double kTile64F64 = 1.0;  // the 64 x 64 FP64 CTA: a quarter of the 128 x 128 step (2000^3: 0.588 us of 0.6)
+constexpr int kWarpsF64 = 8;  // its occupancy counts as 8 warps: one DMMA warp a scheduler nearly fills the pipe
 double occupancy_rate(int warps) {
   return warps >= 16 ? 1.0 : warps >= 14 ? 0.99 : warps >= 12 ? 0.97 : warps >= 10 ? 0.95 : warps >= 8 ? 0.91
                        : warps >= 6 ? 0.8 : 0.71;
@@ -162,9 +164,10 @@ double occupancy_rate(int warps) {
 double native_time_us(int bm, bool fp32, int64_t tiles, int64_t s, int64_t kblocks, int sms, size_t per_split,
                       bool clusters) {
   const int per_sm = fp32 ? (bm == 64 ? simt::SgemmShape<64>::kCtasPerSm : simt::SgemmShape<128>::kCtasPerSm)
-                          : simt::Cfg<double>::CTAS_PER_SM;
-  const int warps_per_cta = fp32 ? bm / 16 : 16;  // FP64: one CTA fills its SM's FP64 rate
-  const double step = fp32 ? kUnitUs * (bm == 64 ? 0.5 * kTile64Factor : 1.0) : kUnitUsF64;  // one CTA k-block, full SM
+                          : bm == 64 ? 4 : 1;
+  const int warps_per_cta = fp32 ? bm / 16 : bm == 64 ? kWarpsF64 : 16;  // FP64 128 x 128: one CTA fills its SM's rate
+  const double step = fp32 ? kUnitUs * (bm == 64 ? 0.5 * kTile64Factor : 1.0)
+                           : kUnitUsF64 * (bm == 64 ? 0.25 * kTile64F64 : 1.0);  // one CTA k-block, full SM
   const int64_t ctas = tiles * s, slots = (int64_t)sms * per_sm;
   const double kbs = (double)ceil_div(kblocks, s);
   const int64_t waves = ctas / slots, rest = ctas - waves * slots;
@@ -186,12 +189,12 @@ NativePlan plan_native(const cucosma_gemm_desc* d, int sms, size_t max_ws) {
   const int vec = 16 / es;
   const int64_t kblocks = std::max<int64_t>(1, ceil_div(d->k, bk));
   const size_t per_split = (size_t)d->m * (size_t)round_up(d->n, vec) * es;
-  // Tile heights to consider: tile id 1 = 128 rows, 2 = 64 rows (FP32), 0 = both.
+  // Tile heights to consider: tile id 1 = 128 rows, 2 = 64 rows (FP32), 0 = both (FP64: tile ids 1, 2 = 128).
   int heights[2] = {simt::BM, 64};
   int nh = 1;
   if (fp32 && d->tile == 2) heights[0] = 64;
-  else if (fp32 && d->tile == 0) nh = 2;
-  const int64_t tiles_n = ceil_div(d->n, simt::BN);
+  else if (d->tile == 0) nh = 2;
+  auto tiles_of = [&](int bm) { return ceil_div(d->m, bm) * ceil_div(d->n, simt::tile_cols(fp32, bm)); };
   const bool clusters = max_ws == SIZE_MAX;
   int64_t splits = d->split_k;
   int bm = heights[0];
@@ -205,7 +208,7 @@ NativePlan plan_native(const cucosma_gemm_desc* d, int sms, size_t max_ws) {
     double best = 1e300;
     splits = 1;
     for (int h = 0; h < nh; ++h) {
-      const int64_t tiles = ceil_div(d->m, heights[h]) * tiles_n;
+      const int64_t tiles = tiles_of(heights[h]);
       for (int64_t s = 1; s <= smax; ++s) {
         if (s > 1 && (size_t)s * per_split > max_ws) break;
         if (s > 1 && s > kblocks / 4 && !simt::cluster_splits(tiles, s)) break;
@@ -220,13 +223,13 @@ NativePlan plan_native(const cucosma_gemm_desc* d, int sms, size_t max_ws) {
   } else if (nh == 2) {
     // forced split: the height with the smaller modelled time
     const int64_t s = std::min<int64_t>(splits, kblocks);
-    const double t128 = native_time_us(128, fp32, ceil_div(d->m, 128) * tiles_n, s, kblocks, sms, per_split, clusters);
-    const double t64 = native_time_us(64, fp32, ceil_div(d->m, 64) * tiles_n, s, kblocks, sms, per_split, clusters);
+    const double t128 = native_time_us(128, fp32, tiles_of(128), s, kblocks, sms, per_split, clusters);
+    const double t64 = native_time_us(64, fp32, tiles_of(64), s, kblocks, sms, per_split, clusters);
     bm = t64 < t128 * 0.98 ? 64 : 128;
   }
   p.bm = bm;
   p.tiles_m = (int)ceil_div(d->m, bm);
-  p.tiles_n = (int)tiles_n;
+  p.tiles_n = (int)ceil_div(d->n, simt::tile_cols(fp32, bm));
   splits = std::max<int64_t>(1, std::min<int64_t>(splits, kblocks));
   splits = std::min<int64_t>(splits, 65535);
   int64_t kchunk = round_up(ceil_div(std::max<int64_t>(d->k, 1), splits), bk);
@@ -251,7 +254,10 @@ static cucosma_status run_native(const cucosma_gemm_desc* d, const NativePlan& p
   CUtensorMap tmA, tmB;
   if (!encode_2d(&tmA, dt, sizeof(T), A, d->k, d->m, d->lda, BK, pl.bm, simt::Cfg<T>::A_SWIZZLE))
     return CUCOSMA_STATUS_LAUNCH_FAILED;
-  if (!encode_2d(&tmB, dt, sizeof(T), B, d->n, d->k, d->ldb, simt::BN, BK, CU_TENSOR_MAP_SWIZZLE_NONE))
+  // FP64, 64 columns: 16-column boxes (128-byte rows) with the 128-byte swizzle
+  const bool swizzle_b = sizeof(T) == 8 && pl.bm == 64;
+  if (!encode_2d(&tmB, dt, sizeof(T), B, d->n, d->k, d->ldb, swizzle_b ? 16 : simt::BN, BK,
+                 swizzle_b ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE))
     return CUCOSMA_STATUS_LAUNCH_FAILED;
   SimtParams p{};
   p.m = (int)d->m;
@@ -501,7 +507,7 @@ extern "C" cucosma_status cucosma_gemm_get_plan(const cucosma_gemm_desc* d, cuco
     const NativePlan pl = plan_native(d, di->sms);
     info->path = 0;
     info->tile_m = pl.bm;
-    info->tile_n = simt::BN;
+    info->tile_n = simt::tile_cols(d->dtype == CUCOSMA_R_32F, pl.bm);
     info->tile_k = simt_bk(d->dtype);
     info->splits = pl.splits;
     info->band = pl.swizzle;

@@ -83,13 +83,13 @@ __device__ __forceinline__ typename Vec<T>::type ld_cluster_vec(uint32_t a) {
 }
 
 // Split-K reduction inside a cluster (one CTA per split, rank = split): every
-// CTA has put its rows x BN partial tile in shared memory; CTA r sums the r-th
+// CTA has put its partial tile in shared memory; CTA r sums the r-th
 // share of the tile's 16-byte vectors over the ranks in ascending order (the
 // order and rounding of splitk_reduce_kernel) and stores epi(alpha * sum +
 // beta * C): no trip through the workspace, no second kernel.
-template <typename T, int ROWS, int THREADS>
+template <typename T, int ROWS, int COLS, int THREADS>
 __device__ __forceinline__ void cluster_reduce(const SimtParams& p, const T* tile, int m0, int n0) {
-  constexpr int VEC = Vec<T>::n, VPR = simt::BN / VEC;  // vectors per row
+  constexpr int VEC = Vec<T>::n, VPR = COLS / VEC;  // vectors per row
   using V = typename Vec<T>::type;
   const T alpha = (T)p.alpha, beta = (T)p.beta;
   cluster_sync_all();  // every rank's tile is written
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(simt::SgemmShape<BM_>::kThreads, simt::SgemmSh
       *reinterpret_cast<float4*>(row) = make_float4(acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y);
       *reinterpret_cast<float4*>(row + 32) = make_float4(acc[i][2].x, acc[i][2].y, acc[i][3].x, acc[i][3].y);
     }
-    cluster_reduce<float, BM, Shape::kThreads>(p, tile, m0, n0);
+    cluster_reduce<float, BM, BN, Shape::kThreads>(p, tile, m0, n0);
     return;
   }
   int rows[8];
@@ -293,14 +293,29 @@ __global__ void __launch_bounds__(simt::SgemmShape<BM_>::kThreads, simt::SgemmSh
 
 // FP64 kernel on the FP64 tensor-core MMA (mma.sync m16n8k8 .f64, the
 // DMMA path: same peak as DFMA on B200, but one instruction does 32 FMAs a
-// lane, so fragment loads and issue slots stop mattering).  8 warps in a 2x4
-// grid, warp tile 64x32 = 4x4 MMA tiles, 64 FP64 accumulators a thread.  A
-// stages (128 rows x 16 k, 128-byte rows) land with the 128-byte TMA swizzle;
-// B stages (16 k x 128 n) unswizzled.  Thread 0 refills a stage two stages
-// after it was consumed, so its wait on the stage's empty barrier rarely
-// blocks.
+// lane, so fragment loads and issue slots stop mattering).  CTA tile EDGE x
+// EDGE: 128 (8 warps in a 2x4 grid, warp tile 64x32, one CTA an SM) or 64 (4
+// warps in a 2x2 grid, warp tile 32x32, four CTAs an SM: a quarter of the
+// padding, and units small enough to spread evenly).  Every output adds its k
+// in the same order either way.  A stages (EDGE rows x 16 k, 128-byte rows)
+// land with the 128-byte TMA swizzle; so do the 64-column tile's B stages, in
+// boxes of 16 k x 16 columns (unswizzled rows of B put the four k a half-warp
+// reads into the same banks: 1000 x 777 x 1531 95.5 -> 91.8 us; the 128-column
+// tile reads half as much a product and lost 0.6 % to the eight boxes).
+// Thread 0 refills a stage two stages after it was consumed, so its wait on
+// the stage's empty barrier rarely blocks.  Bound by the FP64 pipe (37.2
+// TFLOP/s): 35.4 at 4096^3 on 128 x 128; on 64 x 64 31.4 at 2000^3 (30.1 on 128
+// x 128), 1000 x 777 x 1531 101 -> 92 us, 256^3 16.2 -> 8.6.
 namespace simt {
-constexpr int kDStages = 5;
+template <int EDGE>
+struct DgemmShape {
+  static constexpr int kThreads = EDGE == 128 ? 256 : 128;
+  static constexpr int kCtasPerSm = EDGE == 128 ? 1 : 4;
+  static constexpr int kStages = EDGE == 128 ? 5 : 3;
+  static constexpr int kWarpsN = EDGE / 32;   // warps across N, 32 columns each
+  static constexpr int kMt = EDGE == 128 ? 4 : 2;  // 16-row MMA tiles of a warp (two warps down M)
+  static constexpr bool kSwizzleB = EDGE == 64;
+};
 }
 
 __device__ __forceinline__ void dmma_m16n8k8(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
@@ -331,15 +346,17 @@ __device__ __forceinline__ void store_pair(const SimtParams& p, int r, int c, do
   }
 }
 
-template <bool CLUSTER>
-__global__ void __launch_bounds__(simt::kThreads, 1)
+template <int EDGE, bool CLUSTER>
+__global__ void __launch_bounds__(simt::DgemmShape<EDGE>::kThreads, simt::DgemmShape<EDGE>::kCtasPerSm)
     simt_dgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const SimtParams p) {
   pdl_trigger();
   if (p.gate != nullptr && *p.gate != p.gate_value) return;  // path not chosen on the device
   using namespace simt;
+  using Shape = DgemmShape<EDGE>;
+  constexpr int BM = EDGE, BN = EDGE, MT = Shape::kMt;
   constexpr int BK = Cfg<double>::BK;  // 16
-  constexpr int S = kDStages;
+  constexpr int S = Shape::kStages;
   constexpr int A_STAGE = BM * BK * 8, B_STAGE = BK * BN * 8;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -365,7 +382,7 @@ __global__ void __launch_bounds__(simt::kThreads, 1)
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], kComputeWarps);
+      mbar_init(&empty[s], Shape::kThreads / 32);
     }
     fence_mbar_init();
   }
@@ -378,7 +395,12 @@ __global__ void __launch_bounds__(simt::kThreads, 1)
     mbar_arrive_expect_tx(&full[s], A_STAGE + B_STAGE);
     const int kx = (int)(kbeg + (int64_t)kb * BK);
     tma_load_2d(As + s * A_STAGE, &tmA, kx, m0, &full[s]);
-    tma_load_2d(Bs + s * B_STAGE, &tmB, n0, kx, &full[s]);
+    if constexpr (Shape::kSwizzleB) {
+#pragma unroll
+      for (int c = 0; c < BN / 16; ++c) tma_load_2d(Bs + s * B_STAGE + c * 16 * BK * 8, &tmB, n0 + 16 * c, kx, &full[s]);
+    } else {
+      tma_load_2d(Bs + s * B_STAGE, &tmB, n0, kx, &full[s]);
+    }
     issued = kb + 1;
     return true;
   };
@@ -390,20 +412,28 @@ __global__ void __launch_bounds__(simt::kThreads, 1)
   }
 
   const int g = lane >> 2, t = lane & 3;
-  const int wm = warp >> 2, wn = warp & 3;
+  const int wm = warp / Shape::kWarpsN, wn = warp % Shape::kWarpsN;
   // A element (r, k) of a stage sits at r * 128 + (((k >> 1) ^ (r & 7)) << 4) + (k & 1) * 8;
   // every row this thread reads has r & 7 == g.
-  const uint8_t* a_rows = As + (wm * 64 + g) * 128 + (t & 1) * 8;
+  const uint8_t* a_rows = As + (wm * 16 * MT + g) * 128 + (t & 1) * 8;
   int a_off[2][2];  // [k-step][k = t or t + 4]
 #pragma unroll
   for (int ks = 0; ks < 2; ++ks)
 #pragma unroll
     for (int h = 0; h < 2; ++h) a_off[ks][h] = ((((ks * 8 + t + 4 * h) >> 1) ^ g) << 4);
-  const uint8_t* b_cols = Bs + t * BN * 8 + (wn * 32 + g) * 8;
-
-  double acc[4][4][4];
+  // B element (k, n), swizzled: box n / 16 of [16 k][16 columns] at 128 bytes a
+  // k, 16-byte chunk (n % 16) / 2 at its position ^ (k & 7); else row k of BN.
+  const uint8_t* b_cols = Shape::kSwizzleB ? Bs + wn * 2 * (16 * BK * 8) + t * 128 + (g & 1) * 8
+                                           : Bs + t * BN * 8 + (wn * 32 + g) * 8;
+  int b_off[2][2];  // swizzled: [n tile & 1][k = t or t + 4]
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int o = 0; o < 2; ++o)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) b_off[o][h] = h * 4 * 128 + (((o * 4 + (g >> 1)) ^ (t + 4 * h)) << 4);
+
+  double acc[MT][4][4];
+#pragma unroll
+  for (int i = 0; i < MT; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
@@ -418,9 +448,9 @@ __global__ void __launch_bounds__(simt::kThreads, 1)
     const uint8_t* bs = b_cols + s * B_STAGE;
 #pragma unroll
     for (int ks = 0; ks < 2; ++ks) {
-      double af[4][4], bf[4][2];
+      double af[MT][4], bf[4][2];
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt) {
+      for (int mt = 0; mt < MT; ++mt) {
         const uint8_t* r0 = as + mt * 16 * 128;
         af[mt][0] = *reinterpret_cast<const double*>(r0 + a_off[ks][0]);
         af[mt][1] = *reinterpret_cast<const double*>(r0 + 8 * 128 + a_off[ks][0]);
@@ -429,12 +459,18 @@ __global__ void __launch_bounds__(simt::kThreads, 1)
       }
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
-        const uint8_t* c0 = bs + (ks * 8) * BN * 8 + nt * 64;
-        bf[nt][0] = *reinterpret_cast<const double*>(c0);
-        bf[nt][1] = *reinterpret_cast<const double*>(c0 + 4 * BN * 8);
+        if constexpr (Shape::kSwizzleB) {
+          const uint8_t* c0 = bs + (nt >> 1) * (16 * BK * 8) + ks * 8 * 128;
+          bf[nt][0] = *reinterpret_cast<const double*>(c0 + b_off[nt & 1][0]);
+          bf[nt][1] = *reinterpret_cast<const double*>(c0 + b_off[nt & 1][1]);
+        } else {
+          const uint8_t* c0 = bs + (ks * 8) * BN * 8 + nt * 64;
+          bf[nt][0] = *reinterpret_cast<const double*>(c0);
+          bf[nt][1] = *reinterpret_cast<const double*>(c0 + 4 * BN * 8);
+        }
       }
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
+      for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) dmma_m16n8k8(acc[mt][nt], af[mt], bf[nt]);
     }
@@ -456,23 +492,23 @@ __global__ void __launch_bounds__(simt::kThreads, 1)
     double* tile = reinterpret_cast<double*>(smem);  // [BM][BN] over the stages
     static_assert(BM * BN * 8 <= S * (A_STAGE + B_STAGE), "the tile fits the stages");
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
+    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
         for (int h = 0; h < 2; ++h)
-          *reinterpret_cast<double2*>(tile + (wm * 64 + mt * 16 + g + 8 * h) * BN + wn * 32 + nt * 8 + 2 * t) =
+          *reinterpret_cast<double2*>(tile + (wm * 16 * MT + mt * 16 + g + 8 * h) * BN + wn * 32 + nt * 8 + 2 * t) =
               make_double2(acc[mt][nt][2 * h], acc[mt][nt][2 * h + 1]);
-    cluster_reduce<double, BM, kThreads>(p, tile, m0, n0);
+    cluster_reduce<double, BM, BN, Shape::kThreads>(p, tile, m0, n0);
     return;
   }
 #pragma unroll
-  for (int mt = 0; mt < 4; ++mt)
+  for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
       for (int h = 0; h < 2; ++h)
-        store_pair(p, m0 + wm * 64 + mt * 16 + g + 8 * h, n0 + wn * 32 + nt * 8 + 2 * t, acc[mt][nt][2 * h],
+        store_pair(p, m0 + wm * 16 * MT + mt * 16 + g + 8 * h, n0 + wn * 32 + nt * 8 + 2 * t, acc[mt][nt][2 * h],
                    acc[mt][nt][2 * h + 1]);
 }
 
@@ -559,7 +595,8 @@ size_t smem_bytes(int bm) {
     return 1024 + (size_t)stages * (bm * BK + BK * BN) * sizeof(float) + 2 * BK * (bm + 4) * sizeof(float) +
            2 * stages * sizeof(uint64_t);
   } else {
-    return 1024 + kDStages * (BM * BK + BK * BN) * sizeof(T) + 2 * kDStages * sizeof(uint64_t);
+    const int stages = bm == 64 ? DgemmShape<64>::kStages : DgemmShape<128>::kStages;
+    return 1024 + (size_t)stages * 2 * bm * BK * sizeof(T) + 2 * stages * sizeof(uint64_t);
   }
 }
 
@@ -571,12 +608,13 @@ GemmKernel gemm_kernel(int bm, bool cluster = false) {
     if (bm == 64) return cluster ? simt_sgemm_kernel<64, true> : simt_sgemm_kernel<64, false>;
     return cluster ? simt_sgemm_kernel<128, true> : simt_sgemm_kernel<128, false>;
   } else {
-    return cluster ? simt_dgemm_kernel<true> : simt_dgemm_kernel<false>;
+    if (bm == 64) return cluster ? simt_dgemm_kernel<64, true> : simt_dgemm_kernel<64, false>;
+    return cluster ? simt_dgemm_kernel<128, true> : simt_dgemm_kernel<128, false>;
   }
 }
 template <typename T>
 int threads_of(int bm) {
-  return std::is_same<T, float>::value ? 2 * bm : kThreads;
+  return 2 * bm;
 }
 
 template <typename T>

@@ -54,13 +54,11 @@ struct Cfg;
 template <>
 struct Cfg<float> {
   static constexpr int BK = 16;  // 64-byte A rows
-  static constexpr int CTAS_PER_SM = 2;
   static constexpr CUtensorMapSwizzle A_SWIZZLE = CU_TENSOR_MAP_SWIZZLE_64B;
 };
 template <>
 struct Cfg<double> {
   static constexpr int BK = 16;  // 128-byte A rows
-  static constexpr int CTAS_PER_SM = 1;
   static constexpr CUtensorMapSwizzle A_SWIZZLE = CU_TENSOR_MAP_SWIZZLE_128B;
 };
 
@@ -74,11 +72,13 @@ struct SgemmShape {
   static constexpr int kStages = BM_ == 128 ? 4 : 3;
   static constexpr int kLdT = BM_ + 4;  // k-major A row pitch (floats): 16-byte aligned rows
 };
-// CTA tile rows the native kernel of type T can run with (FP64: 128 only).
+// CTA tile rows the native kernel of type T can run with, and the columns
+// that go with them (FP32: 128 x 128 or 64 x 128; FP64: 128 x 128 or 64 x 64).
 template <typename T>
 inline bool tile_rows_supported(int bm) {
-  return bm == BM || (sizeof(T) == 4 && bm == 64);
+  return bm == BM || bm == 64;
 }
+constexpr int tile_cols(bool fp32, int bm) { return fp32 ? BN : bm; }
 
 // Dynamic shared memory of the GEMM kernel with bm-row CTA tiles.
 template <typename T>

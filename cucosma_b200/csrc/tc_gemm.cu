@@ -259,7 +259,7 @@ static Plan make_plan(const cucosma_gemm_desc* d, const DeviceInfo* di, bool all
     cucosma_gemm_desc nd = *d;
     nd.precision = CUCOSMA_PRECISION_NATIVE;
     nd.slices = 0;
-    nd.tile = 0;
+    nd.tile = 1;  // the 128 x 128 kernel: the fallback equals a native call with that tile bit for bit
     pl.native = plan_native(&nd, di->sms);
   }
   const int es_in = pl.kind == 2 ? 1 : 2;
