@@ -45,8 +45,8 @@ __global__ void __launch_bounds__(256, 4) split_bf16_kernel(const __grid_constan
 }
 
 // ----------------------------------------------------------------- Ozaki
-// Column exponents of B start at this sentinel (a byte memset); columns that
-// are all zero keep it until ozaki_rows_kernel turns it into exp_of(0) = 0.
+// Exponents start at this sentinel; all-zero columns and long rows keep it
+// until the slicing turns it into exp_of(0) = 0.
 constexpr int32_t kExpSentinel = (int32_t)0x80808080;
 
 // Column exponents of B (K x N): a block covers 64 rows of K and 512 columns
@@ -54,10 +54,10 @@ constexpr int32_t kExpSentinel = (int32_t)0x80808080;
 // atomicMax of their exponents -- exact, since the exponent of a maximum is
 // the maximum of the exponents (frexp is monotonic in |x|); zero maxima stay
 // out so that they cannot raise a column's exponent.
-__global__ void __launch_bounds__(256)
-    ozaki_col_exp_kernel(const double* __restrict__ B, int64_t ldb, int krows, int ncols, int32_t* eb) {
-  const int c = (blockIdx.x * 256 + threadIdx.x) * 2;
-  const int k0 = blockIdx.y * 64, k1 = min(krows, k0 + 64);
+__device__ __forceinline__ void ozaki_col_exp_block(const double* __restrict__ B, int64_t ldb, int krows, int ncols,
+                                                    int32_t* eb, int bx, int by) {
+  const int c = (bx * 256 + threadIdx.x) * 2;
+  const int k0 = by * 64, k1 = min(krows, k0 + 64);
   if (c >= ncols) return;
   double m0 = 0.0, m1 = 0.0;
   if (c + 1 < ncols) {
@@ -110,14 +110,14 @@ __device__ __forceinline__ unsigned long long store_slices4(int8_t* __restrict__
 }
 
 template <int S>
-__global__ void __launch_bounds__(256)
-    ozaki_rows_kernel(const double* __restrict__ A, int64_t lda, int rows, int cols, int64_t kpad,
-                      int32_t* __restrict__ ea, int8_t* __restrict__ out, unsigned long long* __restrict__ rowsum) {
+__device__ __forceinline__ void ozaki_rows_block(const double* __restrict__ A, int64_t lda, int rows, int cols,
+                                                 int64_t kpad, int32_t* __restrict__ ea, int8_t* __restrict__ out,
+                                                 unsigned long long* __restrict__ rowsum, int b, int blocks) {
   const bool stats = rowsum != nullptr;
   __shared__ double red[8];
   __shared__ unsigned long long red_sum[8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+  for (int r = b; r < rows; r += blocks) {
     const double* src = A + (int64_t)r * lda;
     double v[kRowSteps][4];
     double m = 0.0;
@@ -177,12 +177,12 @@ __global__ void __launch_bounds__(256)
 // independent of the order of the blocks).  Rows that are all zero keep the
 // sentinel until the second kernel's first chunk turns it into 0; every
 // block reads the sentinel as 0.
-__global__ void __launch_bounds__(256)
-    ozaki_row_exp_kernel(const double* __restrict__ A, int64_t lda, int rows, int cols, int32_t* __restrict__ ea) {
+__device__ __forceinline__ void ozaki_row_exp_block(const double* __restrict__ A, int64_t lda, int rows, int cols,
+                                                    int32_t* __restrict__ ea, int chunk, int r0, int rstep) {
   __shared__ double red[8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int c0 = blockIdx.x * kRowRegK;
-  for (int r = blockIdx.y; r < rows; r += gridDim.y) {
+  const int c0 = chunk * kRowRegK;
+  for (int r = r0; r < rows; r += rstep) {
     const double* src = A + (int64_t)r * lda;
     double m = 0.0;
 #pragma unroll
@@ -208,18 +208,19 @@ __global__ void __launch_bounds__(256)
 }
 
 template <int S>
-__global__ void __launch_bounds__(256)
-    ozaki_row_slice_kernel(const double* __restrict__ A, int64_t lda, int rows, int cols, int64_t kpad,
-                           int32_t* __restrict__ ea, int8_t* __restrict__ out, unsigned long long* __restrict__ rowsum) {
+__device__ __forceinline__ void ozaki_row_slice_block(const double* __restrict__ A, int64_t lda, int rows, int cols,
+                                                      int64_t kpad, int32_t* __restrict__ ea, int8_t* __restrict__ out,
+                                                      unsigned long long* __restrict__ rowsum, int chunk, int r0,
+                                                      int rstep) {
   __shared__ unsigned long long red_sum[8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int c0 = blockIdx.x * kRowRegK;
-  for (int r = blockIdx.y; r < rows; r += gridDim.y) {
+  const int c0 = chunk * kRowRegK;
+  for (int r = r0; r < rows; r += rstep) {
     const double* src = A + (int64_t)r * lda;
     int e = ea[r];
     if (e == kExpSentinel) {
       e = 0;
-      if (blockIdx.x == 0 && tid == 0) ea[r] = 0;
+      if (chunk == 0 && tid == 0) ea[r] = 0;
     }
     unsigned long long sum = 0;
 #pragma unroll
@@ -263,11 +264,11 @@ __global__ void __launch_bounds__(256)
 constexpr int kColTileK = 64;
 
 template <int S>
-__global__ void __launch_bounds__(256)
-    ozaki_slice_cols_kernel(const double* __restrict__ B, int64_t ldb, int krows, int ncols, int64_t kpad,
-                            int32_t* __restrict__ eb, int8_t* __restrict__ out, unsigned long long* __restrict__ colsum) {
+__device__ __forceinline__ void ozaki_slice_cols_block(const double* __restrict__ B, int64_t ldb, int krows, int ncols,
+                                                       int64_t kpad, int32_t* __restrict__ eb, int8_t* __restrict__ out,
+                                                       unsigned long long* __restrict__ colsum, int bx, int by) {
   __shared__ double tile[kColTileK][65];
-  const int k0 = blockIdx.y * kColTileK, n0 = blockIdx.x * 64, t = threadIdx.x;
+  const int k0 = by * kColTileK, n0 = bx * 64, t = threadIdx.x;
 #pragma unroll
   for (int p = 0; p < kColTileK / 16; ++p) {
     const int i = p * 16 + t / 16, c = (t % 16) * 4;
@@ -299,7 +300,7 @@ __global__ void __launch_bounds__(256)
       int e = eb[n];
       if (e == kExpSentinel) {
         e = 0;
-        if (blockIdx.y == 0 && kl == 0) eb[n] = 0;
+        if (by == 0 && kl == 0) eb[n] = 0;
       }
       const double v[4] = {tile[kl][nl], tile[kl + 1][nl], tile[kl + 2][nl], tile[kl + 3][nl]};
       uint32_t w[S];
@@ -314,6 +315,83 @@ __global__ void __launch_bounds__(256)
       for (int o = 1; o < 8; o <<= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
       if (kq == 0 && n < ncols && part) atomicAdd(&colsum[n], part);
     }
+  }
+}
+
+// The pre-pass of both operands in three launches (either operand can be left
+// out: its block count is 0): the exponents and sums at their start values;
+// B's column exponents beside A's rows (short rows complete, long rows'
+// exponents); B's slices beside long rows' slices.  Replaces six memsets and
+// four kernels in a row (B200, whole calls: 256^3 60 -> 46 us, 2624 x 511 x 395
+// 113 -> 94, 2000^3 338 -> 308).  The slicing is bound by the integer ALUs, the
+// exponents by HBM: B's exponents run beside A's rows.
+struct OzakiPrep {
+  const double* A;
+  int64_t lda;
+  int m;
+  const double* B;
+  int64_t ldb;
+  int n, k;
+  int64_t kpad;
+  int32_t *ea, *eb;
+  int8_t *sa, *sb;
+  unsigned long long *rowsum, *colsum;  // null: no sums
+  OzakiStats* stats;                    // null: not adaptive
+  int a_chunks;                         // 0: short rows
+  int b1, a1, b2, a2;                   // blocks of B and A in the second and third launch
+  int tiles_exp, tiles_n;               // blocks across N of B's exponents and slices
+  int do_a, do_b;
+};
+
+__global__ void __launch_bounds__(256) ozaki_init_kernel(const __grid_constant__ OzakiPrep p) {
+  pdl_trigger();
+  const int i0 = blockIdx.x * 256 + threadIdx.x, step = gridDim.x * 256;
+  if (p.do_b)
+    for (int i = i0; i < p.n; i += step) {
+      p.eb[i] = kExpSentinel;
+      if (p.colsum) p.colsum[i] = 0;
+    }
+  if (p.do_a)
+    for (int i = i0; i < p.m; i += step) {
+      p.ea[i] = kExpSentinel;
+      if (p.rowsum) p.rowsum[i] = 0;
+    }
+  if (p.stats && i0 == 0) {
+    if (p.do_b) p.stats->min_col = ~0ull;
+    if (p.do_a) {  // min_row, done_blocks and choice restart for every A (min_col belongs to B)
+      p.stats->min_row = ~0ull;
+      p.stats->done_blocks = 0;
+      p.stats->choice = -1;
+    }
+  }
+}
+
+template <int S>
+__global__ void __launch_bounds__(256) ozaki_prep1_kernel(const __grid_constant__ OzakiPrep p) {
+  pdl_trigger();
+  pdl_wait();
+  const int b = blockIdx.x;
+  if (b < p.b1) {
+    ozaki_col_exp_block(p.B, p.ldb, p.k, p.n, p.eb, b % p.tiles_exp, b / p.tiles_exp);
+  } else if (p.a_chunks == 0) {
+    ozaki_rows_block<S>(p.A, p.lda, p.m, p.k, p.kpad, p.ea, p.sa, p.rowsum, b - p.b1, p.a1);
+  } else {
+    const int i = b - p.b1;
+    ozaki_row_exp_block(p.A, p.lda, p.m, p.k, p.ea, i % p.a_chunks, i / p.a_chunks, p.a1 / p.a_chunks);
+  }
+}
+
+template <int S>
+__global__ void __launch_bounds__(256) ozaki_prep2_kernel(const __grid_constant__ OzakiPrep p) {
+  pdl_trigger();
+  pdl_wait();
+  const int b = blockIdx.x;
+  if (b < p.b2) {
+    ozaki_slice_cols_block<S>(p.B, p.ldb, p.k, p.n, p.kpad, p.eb, p.sb, p.colsum, b % p.tiles_n, b / p.tiles_n);
+  } else {
+    const int i = b - p.b2;
+    ozaki_row_slice_block<S>(p.A, p.lda, p.m, p.k, p.kpad, p.ea, p.sa, p.rowsum, i % p.a_chunks, i / p.a_chunks,
+                             p.a2 / p.a_chunks);
   }
 }
 
@@ -342,6 +420,7 @@ __device__ __forceinline__ unsigned long long block_min_nonzero(const unsigned l
 __global__ void __launch_bounds__(256) ozaki_decide_kernel(const unsigned long long* __restrict__ rowsum, int nrows,
                                                            const unsigned long long* __restrict__ colsum, int ncols,
                                                            int64_t k, OzakiStats* stats) {
+  pdl_wait();
   __shared__ unsigned long long red[8];
   const unsigned long long mrow = block_min_nonzero(rowsum, nrows, red);
   const unsigned long long m = block_min_nonzero(colsum, ncols, red);
@@ -388,80 +467,80 @@ cudaError_t launch_split_bf16(SplitJobs& jobs, int nterms, cudaStream_t st) {
 }
 
 template <int S>
-static cudaError_t prep_b_s(const double* B, int64_t ldb, int k, int n, int64_t kpad, int32_t* eb, int8_t* sb,
-                            unsigned long long* colsum, cudaStream_t st) {
-  dim3 grid((unsigned)ceil_div(n, 64), (unsigned)ceil_div(kpad, kColTileK));
-  ozaki_slice_cols_kernel<S><<<grid, 256, 0, st>>>(B, ldb, k, n, kpad, eb, sb, colsum);
-  return cudaGetLastError();
+static cudaError_t prep_s(const OzakiPrep& p, cudaStream_t st) {
+  cudaError_t e = cudaSuccess;
+  if (p.b1 + p.a1 > 0)
+    e = launch_after(true, ozaki_prep1_kernel<S>, dim3((unsigned)(p.b1 + p.a1)), 256, 0, st, p);
+  if (e == cudaSuccess && p.b2 + p.a2 > 0)
+    e = launch_after(true, ozaki_prep2_kernel<S>, dim3((unsigned)(p.b2 + p.a2)), 256, 0, st, p);
+  return e;
 }
 
-template <int S>
-static cudaError_t prep_a_s(const double* A, int64_t lda, int m, int k, int64_t kpad, int32_t* ea, int8_t* sa,
-                            unsigned long long* rowsum, int sms, cudaStream_t st) {
-  if (kpad <= kRowRegK) {
-    const unsigned rows_grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(m, (int64_t)sms * 8));
-    ozaki_rows_kernel<S><<<rows_grid, 256, 0, st>>>(A, lda, m, k, kpad, ea, sa, rowsum);
-    return cudaGetLastError();
+cudaError_t launch_ozaki_prep(int s, const OzakiOperands& o, bool do_a, bool do_b, OzakiStats* stats, int sms,
+                              cudaStream_t st, int* launches) {
+  OzakiPrep p{};
+  p.A = o.A;
+  p.lda = o.lda;
+  p.m = o.m;
+  p.B = o.B;
+  p.ldb = o.ldb;
+  p.n = o.n;
+  p.k = o.k;
+  p.kpad = o.kpad;
+  p.ea = o.ea;
+  p.eb = o.eb;
+  p.sa = o.sa;
+  p.sb = o.sb;
+  p.rowsum = stats ? o.rowsum : nullptr;
+  p.colsum = stats ? o.colsum : nullptr;
+  p.stats = stats;
+  p.do_a = do_a;
+  p.do_b = do_b;
+  int64_t b1 = 0, b2 = 0, a1 = 0, a2 = 0;
+  if (do_b) {
+    p.tiles_exp = (int)ceil_div(o.n, 512);
+    p.tiles_n = (int)ceil_div(o.n, 64);
+    b1 = p.tiles_exp * ceil_div(o.k, 64);
+    b2 = p.tiles_n * ceil_div(o.kpad, kColTileK);
   }
-  cudaError_t e = cudaMemsetAsync(ea, 0x80, (size_t)m * sizeof(int32_t), st);
-  if (e == cudaSuccess && rowsum) e = cudaMemsetAsync(rowsum, 0, (size_t)m * sizeof(unsigned long long), st);
-  if (e != cudaSuccess) return e;
-  const dim3 grid((unsigned)ceil_div(kpad, kRowRegK), (unsigned)std::min<int64_t>(m, 65535));
-  ozaki_row_exp_kernel<<<grid, 256, 0, st>>>(A, lda, m, k, ea);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  ozaki_row_slice_kernel<S><<<grid, 256, 0, st>>>(A, lda, m, k, kpad, ea, sa, rowsum);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_ozaki_prep_b(int s, const double* B, int64_t ldb, int k, int n, int64_t kpad, int32_t* eb,
-                                int8_t* sb, unsigned long long* colsum, OzakiStats* stats, int sms, cudaStream_t st) {
-  (void)sms;
-  cudaError_t e = cudaMemsetAsync(eb, 0x80, (size_t)n * sizeof(int32_t), st);
-  if (e == cudaSuccess && colsum) e = cudaMemsetAsync(colsum, 0, (size_t)n * sizeof(unsigned long long), st);
-  if (e == cudaSuccess && stats) e = cudaMemsetAsync(&stats->min_col, 0xFF, sizeof(stats->min_col), st);
-  if (e != cudaSuccess) return e;
-  if (k > 0) {
-    const dim3 grid((unsigned)ceil_div(n, 512), (unsigned)ceil_div(k, 64));
-    ozaki_col_exp_kernel<<<grid, 256, 0, st>>>(B, ldb, k, n, eb);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if (do_a) {
+    if (o.kpad <= kRowRegK) {
+      a1 = std::max<int64_t>(1, std::min<int64_t>(o.m, (int64_t)sms * 8));
+    } else {
+      p.a_chunks = (int)ceil_div(o.kpad, kRowRegK);
+      // rows over as many blocks per chunk as one launch takes
+      const int64_t rows = std::min<int64_t>(o.m, std::max<int64_t>(1, ((int64_t)1 << 30) / p.a_chunks));
+      a1 = a2 = rows * p.a_chunks;
+    }
   }
+  if (b1 + a1 > INT32_MAX || b2 + a2 > INT32_MAX) return cudaErrorInvalidValue;
+  p.b1 = (int)b1;
+  p.b2 = (int)b2;
+  p.a1 = (int)a1;
+  p.a2 = (int)a2;
+  const int cells = std::max(do_a ? o.m : 0, do_b ? o.n : 0);
+  const unsigned init_blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(cells, 256), (int64_t)sms * 2));
+  ozaki_init_kernel<<<init_blocks, 256, 0, st>>>(p);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
   switch (s) {
-    case 4: return prep_b_s<4>(B, ldb, k, n, kpad, eb, sb, colsum, st);
-    case 5: return prep_b_s<5>(B, ldb, k, n, kpad, eb, sb, colsum, st);
-    case 6: return prep_b_s<6>(B, ldb, k, n, kpad, eb, sb, colsum, st);
-    case 7: return prep_b_s<7>(B, ldb, k, n, kpad, eb, sb, colsum, st);
-    case 8: return prep_b_s<8>(B, ldb, k, n, kpad, eb, sb, colsum, st);
-    case 9: return prep_b_s<9>(B, ldb, k, n, kpad, eb, sb, colsum, st);
+    case 4: e = prep_s<4>(p, st); break;
+    case 5: e = prep_s<5>(p, st); break;
+    case 6: e = prep_s<6>(p, st); break;
+    case 7: e = prep_s<7>(p, st); break;
+    case 8: e = prep_s<8>(p, st); break;
+    case 9: e = prep_s<9>(p, st); break;
     default: return cudaErrorInvalidValue;
   }
-}
-
-cudaError_t launch_ozaki_prep_a(int s, const double* A, int64_t lda, int m, int k, int64_t kpad, int32_t* ea,
-                                int8_t* sa, unsigned long long* rowsum, OzakiStats* stats, int sms, cudaStream_t st) {
-  if (stats) {
-    // min_row, done_blocks and choice restart for every A (min_col belongs to B)
-    cudaError_t e = cudaMemsetAsync(&stats->min_row, 0xFF, sizeof(stats->min_row), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(&stats->done_blocks, 0, sizeof(stats->done_blocks), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(&stats->choice, 0xFF, sizeof(stats->choice), st);
-    if (e != cudaSuccess) return e;
-  }
-  switch (s) {
-    case 4: return prep_a_s<4>(A, lda, m, k, kpad, ea, sa, stats ? rowsum : nullptr, sms, st);
-    case 5: return prep_a_s<5>(A, lda, m, k, kpad, ea, sa, stats ? rowsum : nullptr, sms, st);
-    case 6: return prep_a_s<6>(A, lda, m, k, kpad, ea, sa, stats ? rowsum : nullptr, sms, st);
-    case 7: return prep_a_s<7>(A, lda, m, k, kpad, ea, sa, stats ? rowsum : nullptr, sms, st);
-    case 8: return prep_a_s<8>(A, lda, m, k, kpad, ea, sa, stats ? rowsum : nullptr, sms, st);
-    case 9: return prep_a_s<9>(A, lda, m, k, kpad, ea, sa, stats ? rowsum : nullptr, sms, st);
-    default: return cudaErrorInvalidValue;
-  }
+  *launches += 1 + (p.b1 + p.a1 > 0) + (p.b2 + p.a2 > 0);
+  return e;
 }
 
 cudaError_t launch_ozaki_decide(const unsigned long long* rowsum, int m, const unsigned long long* colsum, int n,
                                 int64_t k, OzakiStats* stats, int sms, cudaStream_t st) {
   const unsigned blocks =
       (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(std::max(m, n), 256), (int64_t)sms * 2));
-  ozaki_decide_kernel<<<blocks, 256, 0, st>>>(rowsum, m, colsum, n, k, stats);
-  return cudaGetLastError();
+  return launch_after(true, ozaki_decide_kernel, dim3(blocks), 256, 0, st, rowsum, m, colsum, n, k, stats);
 }
 
 }  // namespace cucosma

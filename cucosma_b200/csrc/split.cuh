@@ -102,20 +102,28 @@ constexpr int kOzakiLayoutAdaptive = 9;  // slices produced when the count is ch
 // one kernel that holds the row in registers.
 constexpr int kOzakiRowChunk = 8192;
 
+// Operands of an Ozaki GEMM and where their pre-pass results go.
+struct OzakiOperands {
+  const double* A;  // m x k
+  int64_t lda;
+  const double* B;  // k x n
+  int64_t ldb;
+  int m, n, k;
+  int64_t kpad;     // k rounded up to 32
+  int32_t *ea, *eb; // exponents
+  int8_t *sa, *sb;  // slices
+  unsigned long long *rowsum, *colsum;  // magnitude sums (with stats)
+};
 // B (k x n) -> per-column exponents eb (|b_kn| < 2^eb_n, 0 for zero columns)
 // and s INT8 slices of the columns, stacked: byte (n, k, p) at
-// ((k / 32) * s + p) * n * 32 + n * 32 + k % 32.  With colsum (n entries)
-// also the columns' magnitude sums, and stats->min_col is reset.
-cudaError_t launch_ozaki_prep_b(int s, const double* B, int64_t ldb, int k, int n, int64_t kpad, int32_t* eb,
-                                int8_t* sb, unsigned long long* colsum, OzakiStats* stats, int sms, cudaStream_t st);
-
-// A (m x k) -> row exponents ea and s INT8 slices of the rows, packed (four
-// slices' 32-byte k-blocks per 128-byte row): byte (r, k, p) at
-// r * kpad * s + (k / 32) * 32 * s + p * 32 + k % 32; kpad a multiple of 32.
-// With stats, also the rows' magnitude sums into rowsum (m entries; the
-// decision fields of stats are reset first).
-cudaError_t launch_ozaki_prep_a(int s, const double* A, int64_t lda, int m, int k, int64_t kpad, int32_t* ea,
-                                int8_t* sa, unsigned long long* rowsum, OzakiStats* stats, int sms, cudaStream_t st);
+// ((k / 32) * s + p) * n * 32 + n * 32 + k % 32; A (m x k) -> row exponents ea
+// and s slices of the rows, packed (four slices' 32-byte k-blocks per 128-byte
+// row): byte (r, k, p) at r * kpad * s + (k / 32) * 32 * s + p * 32 + k % 32.
+// do_a / do_b choose the operands.  With stats, also the magnitude sums
+// (min_col is reset with B, the decision's other fields with A).  Adds the
+// kernels enqueued to *launches.
+cudaError_t launch_ozaki_prep(int s, const OzakiOperands& o, bool do_a, bool do_b, OzakiStats* stats, int sms,
+                              cudaStream_t st, int* launches);
 
 // After both preparations: stats->min_row / min_col from rowsum and colsum,
 // then stats->choice.

@@ -306,7 +306,7 @@ static int plan_launches(const Plan& pl) {
   if (pl.fused) return 1 + (pl.t.splits > 1 ? 1 : 0);
   if (pl.kind != 2) return 2 + (pl.t.splits > 1 ? 1 : 0);  // the split of A and B, the GEMM
   if (!pl.adaptive) return 4 + (pl.t.splits > 1 ? 1 : 0);
-  // prep B (2), prep A, decision, the three gated kernels and their reductions
+  // pre-pass (3), decision, the three gated kernels and their reductions
   return 7 + (pl.t.splits > 1) + (pl.t9.splits > 1) + (pl.native.splits > 1 && !pl.native.cluster);
 }
 
@@ -548,15 +548,23 @@ cucosma_status tc_gemm_ex(const cucosma_gemm_desc* d, const void* A, const void*
     OzakiStats* stats = pl.adaptive ? reinterpret_cast<OzakiStats*>(w + pl.off_stats) : nullptr;
     unsigned long long* colsum = pl.adaptive ? reinterpret_cast<unsigned long long*>(w + pl.off_colsum) : nullptr;
     unsigned long long* rowsum = pl.adaptive ? reinterpret_cast<unsigned long long*>(w + pl.off_rowsum) : nullptr;
-    if (prep & kPrepB) {
-      e = launch_ozaki_prep_b(ls, (const double*)B, d->ldb, k, n, pl.kpad, eb, reinterpret_cast<int8_t*>(w + pl.off_b),
-                              colsum, stats, di->sms, st);
-      launches += 2;
-    }
-    if (e == cudaSuccess && (prep & kPrepA)) {
-      e = launch_ozaki_prep_a(ls, (const double*)A, d->lda, m, k, pl.kpad, ea, reinterpret_cast<int8_t*>(w + pl.off_a),
-                              rowsum, stats, di->sms, st);
-      launches += pl.kpad > kOzakiRowChunk ? 2 : 1;  // long rows: exponent and slicing kernels
+    if (prep & (kPrepA | kPrepB)) {
+      OzakiOperands o{};
+      o.A = (const double*)A;
+      o.lda = d->lda;
+      o.B = (const double*)B;
+      o.ldb = d->ldb;
+      o.m = m;
+      o.n = n;
+      o.k = k;
+      o.kpad = pl.kpad;
+      o.ea = ea;
+      o.eb = eb;
+      o.sa = reinterpret_cast<int8_t*>(w + pl.off_a);
+      o.sb = reinterpret_cast<int8_t*>(w + pl.off_b);
+      o.rowsum = rowsum;
+      o.colsum = colsum;
+      e = launch_ozaki_prep(ls, o, (prep & kPrepA) != 0, (prep & kPrepB) != 0, stats, di->sms, st, &launches);
     }
     if (e == cudaSuccess && pl.adaptive) {
       e = launch_ozaki_decide(rowsum, m, colsum, n, k, stats, di->sms, st);

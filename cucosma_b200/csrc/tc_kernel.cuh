@@ -1310,7 +1310,9 @@ struct Ozaki : TraitsBase<S*(S + 1) / 2, OzakiBN<S>::value, 128, S, S, S, true, 
 template <class Tr>
 static cudaError_t launch(const CUtensorMap& a, const CUtensorMap& b, const TcParams& p, int grid, cudaStream_t st) {
   static std::atomic<uint64_t> attr_set{0};  // devices whose context has the limit raised
-  // one wave, and not gated (a gated kernel reads the choice first of all)
+  // one wave, and not gated (a gated kernel reads the choice first of all;
+  // started early behind the decision it also lost CTA order: Ozaki 4096^3
+  // 1.61 -> 1.66 ms)
   const bool early = p.gate == nullptr && p.ngroups == 0 &&
                      p.tiles_m * p.tiles_n * p.splits <= (Tr::PAIR ? grid / 2 : grid);
   cudaError_t e = debug_cuda("smem attribute",
