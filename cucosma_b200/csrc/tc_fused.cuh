@@ -265,7 +265,7 @@ __global__ void __maxnreg__((FusedInplaceCfg<Tr, STG>::MAX_REGS))
       bool ok = true;
       for (int unit = unit0; unit < units && ok; unit += unit_step) {
         Unit u;
-        resolve_unit(p, &tmA, &tmB, unit, u);
+        resolve_unit<false>(p, &tmA, &tmB, unit, u);
         for (int kb = u.kb0; kb < u.kb1; kb += F::KB, ++sj) {
           const int st = sj % NS;
           if (!mbar_wait(&empty[st], ((sj / NS) & 1) ^ 1, kErrTimeoutEmpty, p.ctl)) {
@@ -289,7 +289,7 @@ __global__ void __maxnreg__((FusedInplaceCfg<Tr, STG>::MAX_REGS))
       bool ok = true;
       for (int unit = unit0; unit < units && ok; unit += unit_step) {
         Unit u;
-        resolve_unit(p, &tmA, &tmB, unit, u);
+        resolve_unit<false>(p, &tmA, &tmB, unit, u);
         for (int cs = u.kb0; cs < u.kb1 && ok; cs += chunk, ++ci) {
           const int ce = min(u.kb1, cs + chunk);
           const int buf = ci % NBUF;
@@ -329,7 +329,7 @@ __global__ void __maxnreg__((FusedInplaceCfg<Tr, STG>::MAX_REGS))
       bool ok = true;
       for (int unit = unit0; unit < units && ok; unit += unit_step) {
         Unit u;
-        resolve_unit(p, &tmA, &tmB, unit, u);
+        resolve_unit<false>(p, &tmA, &tmB, unit, u);
         for (int kb = u.kb0; kb < u.kb1 && ok; kb += F::KB, ++sj) {
           const int st = sj % NS;
           ok = forward_planes(&fwd[st], (sj / NS) & 1, full_rank0 + (uint32_t)(st * sizeof(uint64_t)), p.ctl);
@@ -348,20 +348,20 @@ __global__ void __maxnreg__((FusedInplaceCfg<Tr, STG>::MAX_REGS))
     uint32_t cph = 0;  // phase of this warp's C-load barrier
     for (int unit = unit0; unit < units; unit += unit_step) {
       Unit u;
-      resolve_unit(p, &tmA, &tmB, unit, u);
+      resolve_unit<false>(p, &tmA, &tmB, unit, u);
       const int row0 = u.tm * TILE_M + (int)rank * 128 + 32 * q;
       const int col0 = u.tn * BN;
       // C prefetched into L2 one unit ahead (this unit's only for the first)
       auto prefetch_unit = [&](int un) {
         if (un >= units) return;
         Unit v;
-        resolve_unit(p, &tmA, &tmB, un, v);
-        prefetch_c_block(out_ctx(p, v), v.tm * TILE_M + (int)rank * 128 + 32 * q, v.tn * BN + colsub, W, 4, lane);
+        resolve_unit<false>(p, &tmA, &tmB, un, v);
+        prefetch_c_block(out_ctx<TILE_M, BN, false>(p, v), v.tm * TILE_M + (int)rank * 128 + 32 * q, v.tn * BN + colsub, W, 4, lane);
       };
       if (unit == unit0) prefetch_unit(unit);
       const int nchunks = (u.kb1 - u.kb0 + chunk - 1) / chunk;
       auto octx = [&]() {
-        OutCtx o = out_ctx(p, u);
+        OutCtx o = out_ctx<TILE_M, BN, false>(p, u);
         o.tbar = &ebar[STG * (warp - 2)];
         return o;
       };
@@ -419,7 +419,7 @@ __global__ void __maxnreg__((FusedInplaceCfg<Tr, STG>::MAX_REGS))
     bool ok = true;
     for (int unit = unit0; unit < units && ok; unit += unit_step) {
       Unit u;
-      resolve_unit(p, &tmA, &tmB, unit, u);
+      resolve_unit<false>(p, &tmA, &tmB, unit, u);
       for (int kb = u.kb0; kb < u.kb1; kb += F::KB, ++sj) {
         const int st = sj % NS;
         uint8_t* stage = stages + st * F::STAGE;

@@ -33,6 +33,44 @@ __global__ void ozaki_reduce_kernel(const double* __restrict__ ws, int64_t split
   }
 }
 
+// C = epi(alpha * sum of a tile's partials + beta * C) for the tiles of a
+// K-split last wave (TcParams::tail_ws), splits in ascending order; four
+// columns a thread.  The partials lie in L2: bound by it and by launch latency.
+__global__ void __launch_bounds__(256) tail_reduce_kernel(const __grid_constant__ TailReduce t) {
+  pdl_wait();
+  const int per_tile = t.tile_m * t.bn / 4, vpr = t.bn / 4;
+  const int64_t split_stride = (int64_t)t.count * t.tile_m * t.bn;
+  for (int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x; idx < (int64_t)t.count * per_tile;
+       idx += (int64_t)gridDim.x * 256) {
+    const int i = (int)(idx / per_tile), v = (int)(idx - (int64_t)i * per_tile);
+    int z, tm, tn;
+    unit_coords(t.tile0 + i, t.tiles_m * t.tiles_n, t.tiles_m, t.tiles_n, t.band, z, tm, tn);
+    const int r = tm * t.tile_m + v / vpr, c = tn * t.bn + (v % vpr) * 4;
+    if (r >= t.m || c >= t.n) continue;
+    const float* w = t.ws + idx * 4;
+    float4 s = *reinterpret_cast<const float4*>(w);  // (columns past n: read, never used)
+    for (int q = 1; q < t.splits; ++q) {
+      const float4 a = *reinterpret_cast<const float4*>(w + q * split_stride);
+      s.x += a.x, s.y += a.y, s.z += a.z, s.w += a.w;
+    }
+    float* o = t.C + (int64_t)r * t.ldc + c;
+    const float acc[4] = {s.x, s.y, s.z, s.w};
+    if (c + 4 <= t.n) {  // c % 4 == 0, 16-byte rows
+      float4 cv = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (t.beta != 0.f) cv = *reinterpret_cast<const float4*>(o);
+      cv.x = apply_epi(combine(acc[0], t.alpha, t.beta, &cv.x), t.epilogue);
+      cv.y = apply_epi(combine(acc[1], t.alpha, t.beta, &cv.y), t.epilogue);
+      cv.z = apply_epi(combine(acc[2], t.alpha, t.beta, &cv.z), t.epilogue);
+      cv.w = apply_epi(combine(acc[3], t.alpha, t.beta, &cv.w), t.epilogue);
+      *reinterpret_cast<float4*>(o) = cv;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (c + e < t.n) o[e] = apply_epi(combine(acc[e], t.alpha, t.beta, o + e), t.epilogue);
+    }
+  }
+}
+
 // ------------------------------------------------------------ planning
 // BF16 kernel variants (the descriptor's tile id selects one; 0 = auto).
 enum Variant : int {
@@ -48,9 +86,11 @@ enum Variant : int {
   kV6Fused = 11,     // BF16x6 256 x 128 pair, split fused into the kernel (tile id 4)
 };
 
-// Tiling of one kernel: tiles, K blocks and splits, raster band.
+// Tiling of one kernel: tiles, K blocks and splits, raster band; tiles from
+// tail_tile0 on (the last wave) run as tail_splits K splits (1: none).
 struct Tiling {
   int slices, bn, tiles_m, tiles_n, kblocks, kb_per_split, splits, band;
+  int tail_tile0, tail_splits, tail_kb;
 };
 
 struct Plan {
@@ -159,6 +199,41 @@ constexpr TileModel kModelV6[] = {{kV6Single, 128, 128, 0, 7.2, 0.64, 1.8, 0.8},
                                   {kV6PairWide, 256, 256, 0, 8.1, 1.01, 3.6, 0.92},
                                   {kV6Fused, 256, 128, 1, 5.8, 0.90, 2.1, 0.92}};
 
+// us a k-block of a 256 x 256 pair takes in a thin last wave (BF16x3, BF16x6)
+constexpr double kTailUnitUs[2] = {0.33, 0.93};
+
+// The last wave of `tiles` unsplit units on `slots` CTAs or pairs, when it is
+// partial: its K in `splits` parts of kb k-blocks, so that most slots have work
+// for a shorter time.  unit_us: the modelled time of one k-block of a unit.
+// Returns the modelled time saved: the k-blocks a slot no longer walks, less
+// the reduction (a launch, and every partial tile out of and back into the SMs
+// through L2); 0 (leave it whole) below 5.5 % of the units' time, where B200
+// showed no gain beyond the runs' differences (BF16x6 8192^3, 62 tiles left,
+// modelled 0.4 %; 2600^3 4.8 %; 4700 x 6100 x 520 2.7 %).  Above it, back to
+// back: 1900 x 2500 x 4000 (a few tiles more than one wave) BF16x3 153..177 ->
+// 122..127 us, BF16x6 325 -> 246; 4096^3 (half a wave left) BF16x3 325 -> 318,
+// BF16x6 877..915 -> 762..829; 3000 x 5000 x 2000 BF16x3 162 -> 157; 5000^3
+// BF16x3 734 -> 706.  kb is a whole number of promotion chunks, so a part's
+// sums are the chunk sums of the whole.
+struct Tail {
+  int splits, kb;
+  double saved;
+};
+static Tail plan_tail(int64_t tiles, int64_t slots, int64_t kblocks, double unit_us, double tile_elems) {
+  Tail best{1, 0, 0.0};
+  const int64_t r = tiles % slots;
+  if (tiles < slots || r == 0) return best;
+  const double least = 0.055 * (double)(ceil_div(tiles, slots) * kblocks) * unit_us;
+  for (int64_t s = 2; s <= 8; ++s) {
+    const int64_t kb = round_up(ceil_div(kblocks, s), kPromoteChunk);
+    if (ceil_div(kblocks, kb) != s) continue;
+    const double saved = ((double)kblocks - (double)(ceil_div(r * s, slots) * kb)) * unit_us -
+                         (4.0 + (double)(r * s) * tile_elems * 8.0 / 13.8e6);
+    if (saved > least && saved > best.saved * 1.02) best = {(int)s, (int)kb, saved};
+  }
+  return best;
+}
+
 // The (tile, splits) with the smallest modelled time; forced > 0 fixes the splits.
 static void choose_bf16(const cucosma_gemm_desc* d, int kind, const DeviceInfo* di, bool allow_fused, int& variant,
                         int64_t& splits) {
@@ -181,6 +256,8 @@ static void choose_bf16(const cucosma_gemm_desc* d, int kind, const DeviceInfo* 
       double t = v.f + (v.u * (double)ceil_div(kblocks, s) + v.e) * w * (!pair && waves > 1.0 ? 1.1 : 1.0);
       if (!v.fused) t += t_pre;
       if (s > 1) t += 3.1 + (double)s * M * N * 8.0 / 13.8e6;
+      if (s == 1 && d->split_k <= 0 && d->flags == 0 && (v.variant == kV3Pair || v.variant == kV6PairWide))
+        t -= plan_tail(tiles, slots, kblocks, kTailUnitUs[kind], 256.0 * v.bn).saved;
       if (t + t_c < best) {
         best = t + t_c;
         variant = v.variant;
@@ -254,6 +331,22 @@ static Plan make_plan(const cucosma_gemm_desc* d, const DeviceInfo* di, bool all
   pl.tile_m = pl.pair ? 256 : 128;
   pl.bn_local = pl.pair ? bn / 2 : bn;
   pl.t = make_tiling(pl, slices, bn, d, splits, di);
+  pl.t.tail_tile0 = pl.t.tiles_m * pl.t.tiles_n;
+  pl.t.tail_splits = 1;
+  // Automatic calls (a given tile or split count is run as given; the test
+  // hooks too) on pair tiles: a partial last wave is split along K.
+  if (pl.kind != 2 && d->tile == 0 && d->split_k <= 0 && d->flags == 0 && pl.t.splits == 1 &&
+      (pl.variant == kV3Pair || pl.variant == kV6PairWide)) {
+    const int slots =
+        pl.variant == kV3Pair ? max_pair_clusters<Bf16x3Pair>(di->sms) : max_pair_clusters<Bf16x6PairWide>(di->sms);
+    const Tail tail = plan_tail(pl.t.tail_tile0, slots, pl.t.kblocks, kTailUnitUs[pl.kind],
+                                (double)pl.tile_m * bn);
+    if (tail.splits > 1) {
+      pl.t.tail_tile0 -= pl.t.tail_tile0 % slots;
+      pl.t.tail_splits = tail.splits;
+      pl.t.tail_kb = tail.kb;
+    }
+  }
   if (pl.adaptive) {
     pl.t9 = make_tiling(pl, 9, ozaki_bn(9), d, splits, di);
     cucosma_gemm_desc nd = *d;
@@ -289,6 +382,8 @@ static Plan make_plan(const cucosma_gemm_desc* d, const DeviceInfo* di, bool all
   pl.ldw = round_up(N, 4);
   pl.off_part = off;
   size_t part = pl.t.splits > 1 ? (size_t)pl.t.splits * M * pl.ldw * es_out : 0;
+  if (pl.t.tail_splits > 1)
+    part = (size_t)pl.t.tail_splits * (pl.t.tiles_m * pl.t.tiles_n - pl.t.tail_tile0) * pl.tile_m * bn * es_out;
   if (pl.adaptive) {
     if (pl.t9.splits > 1) part = std::max(part, (size_t)pl.t9.splits * M * pl.ldw * es_out);
     part = std::max(part, pl.native.ws_bytes);
@@ -304,7 +399,7 @@ static bool one_chunk(const Tiling& t) { return t.splits == 1 && t.kblocks <= kP
 
 static int plan_launches(const Plan& pl) {
   if (pl.fused) return 1 + (pl.t.splits > 1 ? 1 : 0);
-  if (pl.kind != 2) return 2 + (pl.t.splits > 1 ? 1 : 0);  // the split of A and B, the GEMM
+  if (pl.kind != 2) return 2 + (pl.t.splits > 1 || pl.t.tail_splits > 1 ? 1 : 0);  // the split of A and B, the GEMM
   if (!pl.adaptive) return 4 + (pl.t.splits > 1 ? 1 : 0);
   // pre-pass (3), decision, the three gated kernels and their reductions
   return 7 + (pl.t.splits > 1) + (pl.t9.splits > 1) + (pl.native.splits > 1 && !pl.native.cluster);
@@ -359,6 +454,10 @@ TcParams tc_params(const cucosma_gemm_desc* d, const Tiling& t, const Plan& pl, 
   p.kblocks = t.kblocks;
   p.kb_per_split = t.kb_per_split;
   p.splits = t.splits;
+  p.tail_tile0 = t.tail_tile0;
+  p.tail_splits = t.tail_splits;
+  p.tail_kb = t.tail_kb;
+  p.tail_ws = t.tail_splits > 1 ? reinterpret_cast<float*>(w + pl.off_part) : nullptr;
   p.band = t.band;
   p.epilogue = d->epilogue;
   p.alpha = d->alpha;
@@ -515,7 +614,9 @@ cucosma_status tc_gemm_ex(const cucosma_gemm_desc* d, const void* A, const void*
                    pl.bk, pl.bn_local, nt, CU_TENSOR_MAP_SWIZZLE_64B))
       return CUCOSMA_STATUS_LAUNCH_FAILED;
     const TcParams p = tc_params(d, pl.t, pl, C, w, di, pl.variant == kV3Wide);
-    const int units = pl.t.tiles_m * pl.t.tiles_n * pl.t.splits;
+    const int tail_tiles = pl.t.tiles_m * pl.t.tiles_n - pl.t.tail_tile0;
+    const int units = pl.t.tail_splits > 1 ? pl.t.tail_tile0 + tail_tiles * pl.t.tail_splits
+                                           : pl.t.tiles_m * pl.t.tiles_n * pl.t.splits;
     const int grid = std::min(units, di->sms);
     auto pair_grid = [&](int clusters) { return 2 * std::max(1, std::min(units, clusters)); };
     prof_begin(st);
@@ -523,15 +624,21 @@ cucosma_status tc_gemm_ex(const cucosma_gemm_desc* d, const void* A, const void*
       case kV6Single: e = launch<Bf16x6>(ta, tb, p, grid, st); break;
       case kV6Pair: e = launch<Bf16x6Pair>(ta, tb, p, pair_grid(max_pair_clusters<Bf16x6Pair>(di->sms)), st); break;
       case kV6PairWide:
-        e = launch<Bf16x6PairWide>(ta, tb, p, pair_grid(max_pair_clusters<Bf16x6PairWide>(di->sms)), st);
+        if (pl.t.tail_splits > 1)
+          e = launch<WithTail<Bf16x6PairWide>>(ta, tb, p, pair_grid(max_pair_clusters<Bf16x6PairWide>(di->sms)), st);
+        else
+          e = launch<Bf16x6PairWide>(ta, tb, p, pair_grid(max_pair_clusters<Bf16x6PairWide>(di->sms)), st);
         break;
       case kV3Small: e = launch<Bf16x3Promoted>(ta, tb, p, grid, st); break;
       case kV3Wide: e = launch<Bf16x3Wide>(ta, tb, p, grid, st); break;
       case kV3Pair:
         if (one_chunk(pl.t))
           e = launch<Bf16x3PairDirect>(ta, tb, p, pair_grid(max_pair_clusters<Bf16x3PairDirect>(di->sms)), st);
+        else if (pl.t.tail_splits > 1)
+          e = launch<WithTail<Bf16x3Pair>>(ta, tb, p, pair_grid(max_pair_clusters<Bf16x3Pair>(di->sms)), st);
         else
-          e = launch<Bf16x3Pair>(ta, tb, p, pair_grid(max_pair_clusters<Bf16x3Pair>(di->sms)), st); break;
+          e = launch<Bf16x3Pair>(ta, tb, p, pair_grid(max_pair_clusters<Bf16x3Pair>(di->sms)), st);
+        break;
       default: e = launch<Bf16x3>(ta, tb, p, grid, st);
     }
     prof_end(st);
@@ -539,6 +646,15 @@ cucosma_status tc_gemm_ex(const cucosma_gemm_desc* d, const void* A, const void*
     if (e == cudaSuccess && pl.t.splits > 1) {
       e = simt::launch_reduce<float>((const float*)p.out, p.ws_split_stride, pl.ldw, pl.t.splits, (float*)C, d->ldc, m,
                                      n, d->alpha, d->beta, d->epilogue, di->sms, st);
+      launches += 1;
+    }
+    if (e == cudaSuccess && pl.t.tail_splits > 1) {
+      const TailReduce t{p.tail_ws, static_cast<float*>(C), d->ldc, m, n, pl.t.tiles_m, pl.t.tiles_n, pl.t.band,
+                         pl.tile_m, pl.t.bn, pl.t.tail_tile0, tail_tiles, pl.t.tail_splits, (float)d->alpha,
+                         (float)d->beta, d->epilogue};
+      const int64_t vecs = (int64_t)tail_tiles * pl.tile_m * pl.t.bn / 4;
+      e = launch_after(true, tail_reduce_kernel, dim3((unsigned)std::min<int64_t>(ceil_div(vecs, 256), di->sms * 8)),
+                       256, 0, st, t);
       launches += 1;
     }
   } else {

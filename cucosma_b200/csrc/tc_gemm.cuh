@@ -69,6 +69,12 @@ struct TcParams {
   int64_t ws_split_stride;
   const int32_t* ea;  // Ozaki row exponents of A
   const int32_t* eb;  // Ozaki column exponents of B
+  // K-split last wave of an otherwise unsplit problem: the raster's tiles from
+  // tail_tile0 on run as tail_splits units each, of tail_kb k-blocks, whose raw
+  // partial tiles go to tail_ws as [split][tile][TILE_M][BN] for
+  // tail_reduce_kernel.  tail_splits 1: none (tail_tile0 is the tile count).
+  int tail_tile0, tail_splits, tail_kb;
+  float* tail_ws;
   WaitCtl ctl;
   int skip_stage;  // test hook: ring position whose loads the producer omits (-1: none)
   // Grouped launch: when ngroups > 0 the problems come from groups[] (all
@@ -102,11 +108,21 @@ struct OutCtx {
 };
 
 // A resolved work unit: operand descriptors, tile coordinates, K range.
+// Operands of tail_reduce_kernel: tiles tile0 .. tile0 + count - 1 of the raster.
+struct TailReduce {
+  const float* ws;
+  float* C;
+  int64_t ldc;
+  int m, n, tiles_m, tiles_n, band, tile_m, bn, tile0, count, splits;
+  float alpha, beta;
+  int epilogue;
+};
+
 struct Unit {
   const CUtensorMap* ta;
   const CUtensorMap* tb;
   int tm, tn, z, kb0, kb1;
-  int group;  // -1 when not grouped
+  int group;  // -1 when not grouped; -2 - i: the i-th K-split tile of the last wave (TcParams::tail_splits)
 };
 
 }  // namespace tc

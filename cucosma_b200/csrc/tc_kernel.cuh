@@ -71,15 +71,29 @@ __device__ __forceinline__ void unit_coords(int unit, int tiles, int tiles_m, in
 // problem and the tile (finding the problem here by binary search was nine
 // dependent loads for every role and unit); tiles are numbered down M first,
 // then across N.  Returns false at an empty position of the work list.
+// Units past tail_tile0 of a problem with a K-split last wave: split-major, so
+// that the tiles of one K range run together and share their operand panels
+// (TAIL: kernels that take such problems).
+template <bool TAIL>
 __device__ __forceinline__ bool resolve_unit(const TcParams& p, const CUtensorMap* tmA, const CUtensorMap* tmB,
                                              int unit, Unit& u) {
   if (p.ngroups == 0) {
-    unit_coords(unit, p.tiles_m * p.tiles_n, p.tiles_m, p.tiles_n, p.band, u.z, u.tm, u.tn);
-    u.kb0 = u.z * p.kb_per_split;
-    u.kb1 = min(p.kblocks, u.kb0 + p.kb_per_split);
+    const int tiles = p.tiles_m * p.tiles_n;
+    u.group = -1;
+    if (TAIL && p.tail_splits > 1 && unit >= p.tail_tile0) {
+      const int v = unit - p.tail_tile0, r = tiles - p.tail_tile0, split = v / r, i = v - split * r;
+      u.group = -2 - i;
+      unit_coords(p.tail_tile0 + i, tiles, p.tiles_m, p.tiles_n, p.band, u.z, u.tm, u.tn);
+      u.z = split;
+      u.kb0 = split * p.tail_kb;
+      u.kb1 = min(p.kblocks, u.kb0 + p.tail_kb);
+    } else {
+      unit_coords(unit, tiles, p.tiles_m, p.tiles_n, p.band, u.z, u.tm, u.tn);
+      u.kb0 = u.z * p.kb_per_split;
+      u.kb1 = min(p.kblocks, u.kb0 + p.kb_per_split);
+    }
     u.ta = tmA;
     u.tb = tmB;
-    u.group = -1;
   } else {
     const int2 item = p.unit_list[unit];
     if (item.x < 0) return false;
@@ -126,6 +140,7 @@ __device__ __forceinline__ void prefetch_c_block(const OutCtx& o, int row0, int 
   }
 }
 
+template <int TILE_M, int BN, bool TAIL>
 __device__ __forceinline__ OutCtx out_ctx(const TcParams& p, const Unit& u) {
   OutCtx o;
   o.epilogue = p.epilogue;
@@ -133,7 +148,7 @@ __device__ __forceinline__ OutCtx out_ctx(const TcParams& p, const Unit& u) {
   o.beta = p.beta;
   o.ctl = p.ctl;
   o.tbar = nullptr;
-  const bool whole = u.group < 0 && !p.partial;
+  const bool whole = (TAIL ? u.group == -1 : u.group < 0) && !p.partial;
   o.tmc = (whole && p.tma_out) ? &p.tmc : nullptr;
   o.tmc3 = (whole && p.tma_wide) ? &p.tmc3 : nullptr;
   o.tmc_pf = (o.tmc != nullptr || o.tmc3 != nullptr) ? &p.tmc_pf : nullptr;
@@ -146,6 +161,12 @@ __device__ __forceinline__ OutCtx out_ctx(const TcParams& p, const Unit& u) {
     o.ws_split_stride = p.ws_split_stride;
     o.ea = p.ea;
     o.eb = p.eb;
+    if (TAIL && u.group < -1) {  // element (row, col) of this tile at its place in the tile's own [TILE_M][BN] block
+      o.partial = 1;
+      o.out = p.tail_ws + (((int64_t)(-2 - u.group) - u.tm) * TILE_M * BN - (int64_t)u.tn * BN);
+      o.ldo = BN;
+      o.ws_split_stride = (int64_t)(p.tiles_m * p.tiles_n - p.tail_tile0) * TILE_M * BN;
+    }
   } else {
     const GroupEntry& e = p.groups[u.group];
     o.m = e.m;
@@ -268,7 +289,9 @@ __global__ void __maxnreg__(Tr::MAX_REGS)
   static_assert((2 * ST + 13 + 2 * Tr::EPI_WARPS) * 8 + 4 <= 512, "barrier area");
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int units = p.ngroups > 0 ? p.total_tiles : p.tiles_m * p.tiles_n * p.splits;
+  const int units = p.ngroups > 0                    ? p.total_tiles
+                    : Tr::kTail && p.tail_splits > 1 ? p.tail_tile0 + (p.tiles_m * p.tiles_n - p.tail_tile0) * p.tail_splits
+                                                     : p.tiles_m * p.tiles_n * p.splits;
   // CTA pair: rank 0 issues the MMAs of both CTAs; the pair (cluster) walks
   // the units together.  Single CTA: rank 0, one CTA per unit.
   const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
@@ -323,7 +346,7 @@ __global__ void __maxnreg__(Tr::MAX_REGS)
       bool ok = true;
       for (int unit = unit0; unit < units && ok; unit += unit_step) {
         Unit u;
-        if (!resolve_unit(p, &tmA, &tmB, unit, u)) continue;
+        if (!resolve_unit<Tr::kTail>(p, &tmA, &tmB, unit, u)) continue;
         const int tm = u.tm, tn = u.tn;
         for (int kb = u.kb0; kb < u.kb1; ++kb, ++it) {
           const int s = it % ST;
@@ -376,7 +399,7 @@ __global__ void __maxnreg__(Tr::MAX_REGS)
       bool ok = true;
       for (int unit = unit0; unit < units && ok; unit += unit_step) {
         Unit u;
-        if (!resolve_unit(p, &tmA, &tmB, unit, u)) continue;
+        if (!resolve_unit<Tr::kTail>(p, &tmA, &tmB, unit, u)) continue;
         const int kb1 = u.kb1;
         for (int cs = u.kb0; cs < kb1 && ok; cs += chunk, ++ci) {
           const int ce = min(kb1, cs + chunk);
@@ -444,7 +467,7 @@ __global__ void __maxnreg__(Tr::MAX_REGS)
       bool ok = true;
       for (int unit = unit0; unit < units && ok; unit += unit_step) {
         Unit u;
-        if (!resolve_unit(p, &tmA, &tmB, unit, u)) continue;
+        if (!resolve_unit<Tr::kTail>(p, &tmA, &tmB, unit, u)) continue;
         if constexpr (Tr::PROMOTE) {
           for (int cs = u.kb0; cs < u.kb1 && ok; cs += chunk, ++ci) {
             if constexpr (Tr::SPLIT)
@@ -480,7 +503,7 @@ __global__ void __maxnreg__(Tr::MAX_REGS)
     bool ok = true;
     for (int unit = unit0; unit < units && ok; unit += unit_step) {
       Unit u;
-      if (!resolve_unit(p, &tmA, &tmB, unit, u)) continue;
+      if (!resolve_unit<Tr::kTail>(p, &tmA, &tmB, unit, u)) continue;
       const int z = u.z;
       const int row0 = u.tm * TILE_M + (int)rank * 128 + 32 * q;
       const int col0 = u.tn * BN;
@@ -489,14 +512,14 @@ __global__ void __maxnreg__(Tr::MAX_REGS)
       auto prefetch_unit = [&](int un) {
         if (un >= units) return;
         Unit v;
-        if (!resolve_unit(p, &tmA, &tmB, un, v)) return;
-        prefetch_c_block(out_ctx(p, v), v.tm * TILE_M + (int)rank * 128 + 32 * q,
+        if (!resolve_unit<Tr::kTail>(p, &tmA, &tmB, un, v)) return;
+        prefetch_c_block(out_ctx<TILE_M, BN, Tr::kTail>(p, v), v.tm * TILE_M + (int)rank * 128 + 32 * q,
                          v.tn * BN + colsub, W, Tr::kInt8 ? 8 : 4, lane);
       };
       if (unit == unit0) prefetch_unit(unit);
       // the output context is built where it is used (fewer registers held across the chunk loop)
       auto octx = [&]() {
-        OutCtx o = out_ctx(p, u);
+        OutCtx o = out_ctx<TILE_M, BN, Tr::kTail>(p, u);
         o.tbar = &ebar[2 * (warp - 2)];
         return o;
       };
@@ -1109,6 +1132,8 @@ struct TraitsBase {
   // DIRECT: every unit's K fits one accumulator chunk (kPromoteChunk k-blocks),
   // so the epilogue reads TMEM straight into C blocks, 64 columns a warp.
   static constexpr bool DIRECT = DIRECT_;
+  // kTail: takes problems whose last wave is split along K (WithTail).
+  static constexpr bool kTail = false;
   // 4 epilogue warps (one per TMEM lane quadrant) or 8 (each quadrant
   // split into two column halves, so promoted register accumulators fit).
   static constexpr int EPI_WARPS = EPI_WARPS_;
@@ -1253,6 +1278,12 @@ struct Bf16x3Pair : TraitsBase<3, 256, 64, 2, 2, 1, false, EpiF32, true, kPromot
 // (0.47 ms against 0.43) than they gained on beta != 0 (0.54 against 0.52).
 struct Bf16x3PairDirect : TraitsBase<3, 256, 64, 2, 2, 1, false, EpiF32, false, 0, 8, 0, true, false, true> {
   static constexpr TermTable<3> kTerms{{1, 0, 0}, {0, 1, 0}, {0, 0, 0}, {true, false, false}};
+};
+// A kernel for problems whose last wave is split along K: its own instance,
+// since the extra state spills 24 bytes more a thread in either pair tile.
+template <class Tr>
+struct WithTail : Tr {
+  static constexpr bool kTail = true;
 };
 struct Bf16x3Pair128 : TraitsBase<3, 128, 64, 2, 2, 1, false, EpiF32, true, kPromoteChunk, 8, 0, true> {
   static constexpr TermTable<3> kTerms{{1, 0, 0}, {0, 1, 0}, {0, 0, 0}, {true, false, false}};
