@@ -210,6 +210,7 @@ size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 //           4 / 5 = 256 x 128 / 256 x 256 CTA pair, bit-identical to 1
 //   BF16X6  1 = 128 x 128, 2 = 256 x 256 CTA pair (split release)
 //   OZAKI   1 = 128 x ozaki_bn(slices)
+constexpr int kTileIds = 5;
 struct GTile {
   int id, tile_m, bn, pair;
 };
@@ -420,6 +421,17 @@ cucosma_status layout(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr
 
 }  // namespace
 }  // namespace tc
+
+size_t grouped_table_bytes(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr, int count,
+                           const DeviceInfo* di) {
+  size_t most = 0;
+  for (int id = 1; id <= tc::kTileIds; ++id) {
+    tc::Layout L;
+    if (tc::layout(d, pr, count, di->sms, L, id) == CUCOSMA_STATUS_SUCCESS) most = std::max(most, L.table_bytes);
+  }
+  return most;
+}
+
 }  // namespace cucosma
 
 using namespace cucosma;

@@ -18,6 +18,7 @@
 // a text file (cucosma_tune_cache_save / _load; loaded automatically from
 // $CUCOSMA_TUNE_CACHE on first use; CUCOSMA_TUNE=off disables lookups;
 // CUCOSMA_TUNE_COUNTERS=off skips the counter reading).
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -94,6 +95,24 @@ double elapsed_ms(cudaEvent_t a, cudaEvent_t b) {
   return ms;
 }
 
+
+// The tables of a plan that lives on the tuner's workspace: every candidate's
+// plan is made in the same place, with tiles and a work list of its own, and
+// the live plan's next launch would walk those (its list may even lie where a
+// candidate put operand planes).  Read before the first candidate, put back
+// when the tuner returns; the planes themselves are written by every launch.
+struct SavedTables {
+  void* workspace;
+  std::vector<uint8_t> bytes;
+  bool ok;
+  SavedTables(void* ws, size_t n, cudaStream_t st) : workspace(ws), bytes(n) {
+    ok = cudaStreamSynchronize(st) == cudaSuccess &&
+         (n == 0 || cudaMemcpy(bytes.data(), ws, n, cudaMemcpyDeviceToHost) == cudaSuccess);
+  }
+  ~SavedTables() {
+    if (ok && !bytes.empty()) cudaMemcpy(workspace, bytes.data(), bytes.size(), cudaMemcpyHostToDevice);
+  }
+};
 
 }  // namespace
 
@@ -286,6 +305,9 @@ extern "C" cucosma_status cucosma_tune_grouped(const cucosma_gemm_desc* d, const
   if (d->precision == CUCOSMA_PRECISION_BF16X3) tiles = {1, 2, 3};
   else if (d->precision == CUCOSMA_PRECISION_BF16X6) tiles = {1, 2};
   else tiles = {1};
+  if (!workspace) return CUCOSMA_STATUS_WORKSPACE_TOO_SMALL;
+  const SavedTables saved(workspace, std::min(workspace_bytes, grouped_table_bytes(d, problems, count, di)), st);
+  if (!saved.ok) return CUCOSMA_STATUS_LAUNCH_FAILED;
   cudaEvent_t e0, e1;
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) return CUCOSMA_STATUS_LAUNCH_FAILED;
   double best = 1e300;

@@ -277,7 +277,9 @@ CUCOSMA_API cucosma_status cucosma_grouped_plan_get_tile(cucosma_grouped_plan pl
  * one) are run on the problems (their C is overwritten) and the fastest is
  * cached for this batch's shape mix (SM count, dtype, precision, slices and
  * the problems' m, n, k in order).  cucosma_grouped_plan_create uses it when
- * the descriptor's tile is 0.  out->tile is the chosen grouped tile id. */
+ * the descriptor's tile is 0.  out->tile is the chosen grouped tile id.  The
+ * workspace may be that of a plan of these problems: the call waits for the
+ * stream first and leaves the plan's tables as they were. */
 CUCOSMA_API cucosma_status cucosma_tune_grouped(const cucosma_gemm_desc* d, const cucosma_gemm_problem* problems,
                                                 int count, void* workspace, size_t workspace_bytes,
                                                 cucosma_tune_result* out, void* stream);
