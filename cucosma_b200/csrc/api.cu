@@ -199,24 +199,42 @@ NativePlan plan_native(const cucosma_gemm_desc* d, int sms, size_t max_ws) {
   int64_t splits = d->split_k;
   int bm = heights[0];
   if (splits <= 0) {
-    // The (height, split) pair with the smallest modelled time wins; splits
-    // keep >= 4 k-blocks each (inside a cluster one is enough) and fit max_ws,
-    // and a candidate must beat the best so far by 2 % (ties keep the taller
-    // tile and the smaller split).
-    const int64_t smax = std::max<int64_t>(clusters ? std::min<int64_t>(kblocks, simt::kMaxCluster) : 1,
-                                           std::min<int64_t>(kblocks / 4, 512));
+    // The least splits: those of the fastest expected plan that adds its
+    // partial sums through the workspace, FP64 on 128 x 128 tiles.  Smaller
+    // tiles fill the SMs and clusters add cheaply with fewer, but each output
+    // would then be one longer chain of roundings (FP64 500^3 in 2 splits for
+    // 8, 1000 x 777 x 1531 in 2 for 5: twice and 1.6 times the rms error).
+    // Splits keep >= 4 k-blocks each and fit max_ws; a candidate must beat the
+    // best so far by 2 % (ties keep the taller tile and the smaller split).
+    const int64_t smax = std::max<int64_t>(1, std::min<int64_t>(kblocks / 4, 512));
     double best = 1e300;
     splits = 1;
-    for (int h = 0; h < nh; ++h) {
+    for (int h = 0; h < (fp32 ? nh : 1); ++h) {
       const int64_t tiles = tiles_of(heights[h]);
       for (int64_t s = 1; s <= smax; ++s) {
         if (s > 1 && (size_t)s * per_split > max_ws) break;
-        if (s > 1 && s > kblocks / 4 && !simt::cluster_splits(tiles, s)) break;
-        const double t = native_time_us(heights[h], fp32, tiles, s, kblocks, sms, per_split, clusters);
+        const double t = native_time_us(heights[h], fp32, tiles, s, kblocks, sms, per_split, false);
         if (t < best * 0.98) {
           best = t;
           splits = s;
           bm = heights[h];
+        }
+      }
+    }
+    // From there, the (height, split) pair with the smallest modelled time;
+    // inside a cluster a split may be as short as one k-block.
+    if (clusters) {
+      const int64_t least = splits, most = std::max(smax, std::min<int64_t>(kblocks, simt::kMaxCluster));
+      for (int h = 0; h < nh; ++h) {
+        const int64_t tiles = tiles_of(heights[h]);
+        for (int64_t s = least; s <= most; ++s) {
+          if (s > smax && !simt::cluster_splits(tiles, s)) break;
+          const double t = native_time_us(heights[h], fp32, tiles, s, kblocks, sms, per_split, true);
+          if (t < best * 0.98) {
+            best = t;
+            splits = s;
+            bm = heights[h];
+          }
         }
       }
     }
