@@ -145,7 +145,7 @@ static int simt_bk(int dtype) { return dtype == CUCOSMA_R_32F ? simt::Cfg<float>
 // planes of per_split bytes in and out at HBM speed, and a launch).  Fitted to B200 measurements of both FP32 tile
 // heights over square, flat, large-N and large-K shapes:
 //   * a 128 x 128 x 16 k-block step takes kUnitUs of an SM holding 16 warps
-//     (FP64: kUnitUsF64 a CTA, one CTA an SM);
+//     (FP64: kUnitUsF64 a CTA, one CTA an SM, or four 64 x 64 CTAs);
 //   * an SM holding fewer warps runs at occupancy_rate() of that (one 4-warp
 //     CTA alone: 0.71; 8 warps: 0.91);
 //   * the 64-row CTAs do a 64-row step in 0.95 of half a 128-row step (four
@@ -154,9 +154,16 @@ static int simt_bk(int dtype) { return dtype == CUCOSMA_R_32F ? simt::Cfg<float>
 //   * whole waves of resident CTAs run at full occupancy, and the last,
 //     partial wave at the occupancy it leaves.
 namespace {
-constexpr double kUnitUs = 1.45, kUnitUsF64 = 2.4, kTile64Factor = 0.95, kClusterUs = 1.75;
-constexpr double kTile64F64 = 1.0;  // the 64 x 64 FP64 CTA: a quarter of the 128 x 128 step (2000^3: 0.588 us of 0.6)
-constexpr int kWarpsF64 = 8;  // its occupancy counts as 8 warps: one DMMA warp a scheduler nearly fills the pipe
+constexpr double kUnitUs = 1.45, kUnitUsF64 = 2.4, kTile64Factor = 0.95;
+// A cluster's reduction.  A 128 x 128 FP64 tile is twice as many vectors a
+// thread as the others (2 to 8 splits on B200: 1 to 6 us; 100 x 1900 x 150
+// 13.0 us that way, 9.3 on 64 x 64 tiles through the workspace).
+constexpr double cluster_us(bool fp32, int bm) { return fp32 || bm == 64 ? 1.75 : 4.5; }
+// A lone 64 x 64 FP64 CTA on an SM (one DMMA warp a scheduler) runs at 0.61 of
+// the pipe's rate, two or more fill it (45 shapes on B200: 0.58 to 0.65, and
+// 0.98 to 1.09).  Counted as 0.91, 832 x 460 x 1218 took 7 splits of 64 x 64,
+// one whole wave and 136 lone CTAs, 47 us against 45 on 128 x 128 in 5.
+constexpr double kLoneF64 = 0.61;
 double occupancy_rate(int warps) {
   return warps >= 16 ? 1.0 : warps >= 14 ? 0.99 : warps >= 12 ? 0.97 : warps >= 10 ? 0.95 : warps >= 8 ? 0.91
                        : warps >= 6 ? 0.8 : 0.71;
@@ -165,18 +172,19 @@ double native_time_us(int bm, bool fp32, int64_t tiles, int64_t s, int64_t kbloc
                       bool clusters) {
   const int per_sm = fp32 ? (bm == 64 ? simt::SgemmShape<64>::kCtasPerSm : simt::SgemmShape<128>::kCtasPerSm)
                           : bm == 64 ? 4 : 1;
-  const int warps_per_cta = fp32 ? bm / 16 : bm == 64 ? kWarpsF64 : 16;  // FP64 128 x 128: one CTA fills its SM's rate
+  auto rate = [&](int r) { return fp32 ? occupancy_rate(r * bm / 16) : bm == 64 && r == 1 ? kLoneF64 : 1.0; };
   const double step = fp32 ? kUnitUs * (bm == 64 ? 0.5 * kTile64Factor : 1.0)
-                           : kUnitUsF64 * (bm == 64 ? 0.25 * kTile64F64 : 1.0);  // one CTA k-block, full SM
+                           : kUnitUsF64 * (bm == 64 ? 0.25 : 1.0);  // one CTA k-block, full SM
   const int64_t ctas = tiles * s, slots = (int64_t)sms * per_sm;
   const double kbs = (double)ceil_div(kblocks, s);
   const int64_t waves = ctas / slots, rest = ctas - waves * slots;
   double t = (double)waves * kbs * per_sm * step;
   if (rest > 0) {
     const int r = (int)ceil_div(rest, (int64_t)sms);  // CTAs on the busiest SM of the last wave
-    t += kbs * r * step / occupancy_rate(r * warps_per_cta);
+    t += kbs * r * step / rate(r);
   }
-  if (s > 1) t += clusters && simt::cluster_splits(tiles, s) ? kClusterUs : 2.0 + 2.0 * (double)s * (double)per_split / 6.0e6;
+  if (s > 1) t += clusters && simt::cluster_splits(tiles, s) ? cluster_us(fp32, bm)
+                                                             : 2.0 + 2.0 * (double)s * (double)per_split / 6.0e6;
   return t;
 }
 }  // namespace
@@ -225,6 +233,7 @@ NativePlan plan_native(const cucosma_gemm_desc* d, int sms, size_t max_ws) {
     // inside a cluster a split may be as short as one k-block.
     if (clusters) {
       const int64_t least = splits, most = std::max(smax, std::min<int64_t>(kblocks, simt::kMaxCluster));
+      best = 1e300;
       for (int h = 0; h < nh; ++h) {
         const int64_t tiles = tiles_of(heights[h]);
         for (int64_t s = least; s <= most; ++s) {
