@@ -201,7 +201,7 @@ NativePlan plan_native(const cucosma_gemm_desc* d, int sms, size_t max_ws) {
   int heights[2] = {simt::BM, 64};
   int nh = 1;
   if (fp32 && d->tile == 2) heights[0] = 64;
-  else if (d->tile == 0) nh = 2;
+  else if (d->tile == 0 && ceil_div(d->m, 64) <= 65535 * (int64_t)std::max(1, d->swizzle)) nh = 2;  // (tile rows are grid.y)
   auto tiles_of = [&](int bm) { return ceil_div(d->m, bm) * ceil_div(d->n, simt::tile_cols(fp32, bm)); };
   const bool clusters = max_ws == SIZE_MAX;
   int64_t splits = d->split_k;

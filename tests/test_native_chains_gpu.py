@@ -44,3 +44,21 @@ def test_rounding_error_of_the_chosen_plan(cuda, shape, splits):
     # shorter chains cannot err more; equal ones give the same bits.  The
     # sample of m * n errors says so to 4 / sqrt(2 m n).
     assert rms() <= rms(tile=1, split_k=splits) * (1 + 4 / np.sqrt(2 * m * n))
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("m", [65535 * 64, 65535 * 64 + 1])
+def test_most_tile_rows_of_a_grid(cuda, dtype, m):
+    """64-row tiles only while their count fits one grid dimension; sampled rows of a tall, narrow C."""
+    import torch
+
+    dt = getattr(torch, dtype)
+    n, k = 12, 20
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    A = torch.randint(-8, 9, (m, k), generator=g, device="cuda").to(dt)
+    B = torch.randint(-8, 9, (k, n), generator=g, device="cuda").to(dt)
+    C = torch.full((m, n), -1.0, dtype=dt, device="cuda")
+    assert -(-m // cc.get_plan(cc.make_desc(A, B, C))["tile_m"]) <= 65535
+    cc.gemm(A, B, C)
+    assert torch.equal(C, A @ B)  # small integers: exact in any order
