@@ -153,6 +153,27 @@ __global__ void __launch_bounds__(256, RPT <= 4 ? 4 : 2)
   }
 }
 
+// The last steps of thin_kernel's reduction, where the sums are largest, round
+// once: FP32 sums are added in 64 bits, FP64 ones with the rounding error of
+// each addition carried along (D. E. Knuth, TAOCP 2, 4.2.2, theorem B).
+struct SumF64 {
+  double hi, lo;
+};
+__device__ __forceinline__ double widen(float x) { return (double)x; }
+__device__ __forceinline__ SumF64 widen(double x) { return SumF64{x, 0.0}; }
+__device__ __forceinline__ double add(double a, double b) { return a + b; }
+__device__ __forceinline__ SumF64 add(SumF64 a, SumF64 b) {
+  const double s = a.hi + b.hi, t = s - a.hi;
+  return SumF64{s, a.lo + b.lo + ((a.hi - (s - t)) + (b.hi - t))};
+}
+__device__ __forceinline__ double shfl_xor(double x, int off) { return __shfl_xor_sync(0xffffffffu, x, off); }
+__device__ __forceinline__ SumF64 shfl_xor(SumF64 x, int off) {
+  return SumF64{__shfl_xor_sync(0xffffffffu, x.hi, off), __shfl_xor_sync(0xffffffffu, x.lo, off)};
+}
+__device__ __forceinline__ float narrow(double x) { return (float)x; }
+// (an infinite or NaN sum has no error term)
+__device__ __forceinline__ double narrow(SumF64 x) { return isfinite(x.hi) ? x.hi + x.lo : x.hi; }
+
 // Thin kernel: lanes take consecutive k, so a warp's load of a row of the A
 // block is one contiguous line, and its loads of 32 rows of the B block
 // (32-byte FP32 rows) contiguous too when B is as narrow as the block; KU
@@ -217,34 +238,49 @@ __global__ void __launch_bounds__(256, skinny::thin_ctas<T>(RS, CS))
   // lane keeps (ending with one or two consecutive ones, or, for fewer outputs
   // than lanes, one that several lanes hold), then warps 0..7 in order.
   constexpr int OUT = RS * CS;
-  __shared__ T red[8][OUT];
+  using Wide = decltype(widen(T(0)));
+  __shared__ Wide red[8][OUT];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   T v[OUT];
 #pragma unroll
   for (int i = 0; i < OUT; ++i) v[i] = acc[i / CS][i % CS];
-  int first = 0;  // the output v[0] is the sum of
+  int first = 0;  // the output v[0] (w[0]) is the sum of
 #pragma unroll
-  for (int off = 16, half = OUT / 2; off > 0; off >>= 1, half >>= 1) {
+  for (int off = 16, half = OUT / 2; off > 2; off >>= 1, half >>= 1) {
+    const bool up = (lane & off) != 0;
+    if (up) first += half;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const T keep = up ? v[i + half] : v[i], send = up ? v[i] : v[i + half];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+  }
+  Wide w[OUT / 8];
+#pragma unroll
+  for (int i = 0; i < OUT / 8; ++i) w[i] = widen(v[i]);
+#pragma unroll
+  for (int off = 2, half = OUT / 16; off > 0; off >>= 1, half >>= 1) {
     if (half > 0) {
       const bool up = (lane & off) != 0;
       if (up) first += half;
 #pragma unroll
       for (int i = 0; i < half; ++i) {
-        const T keep = up ? v[i + half] : v[i], send = up ? v[i] : v[i + half];
-        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+        const Wide keep = up ? w[i + half] : w[i], send = up ? w[i] : w[i + half];
+        w[i] = add(keep, shfl_xor(send, off));
       }
     } else {
-      v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+      w[0] = add(w[0], shfl_xor(w[0], off));
     }
   }
-  if constexpr (OUT == 64) red[warp][first + 1] = v[1];
-  red[warp][first] = v[0];
+  if constexpr (OUT == 64) red[warp][first + 1] = w[1];
+  red[warp][first] = w[0];
   __syncthreads();
   if (threadIdx.x < OUT) {
     const int i = threadIdx.x / CS, j = threadIdx.x % CS;
-    T s = red[0][threadIdx.x];
+    Wide sum = red[0][threadIdx.x];
 #pragma unroll
-    for (int w = 1; w < 8; ++w) s += red[w][threadIdx.x];
+    for (int q = 1; q < 8; ++q) sum = add(sum, red[q][threadIdx.x]);
+    const T s = narrow(sum);
     if (i < rows && j < cols) {
       const int64_t r = m0 + i, c = n0 + j;
       if (partial) {
@@ -304,10 +340,14 @@ SkinnyPlan plan_skinny(int64_t m, int64_t n, int64_t k, int dtype_bytes, int spl
   p.kind = 2;
   p.tile_m = p.tile_n = skinny::kThin;
   const int64_t groups = ceil_div(m, skinny::kThin) * ceil_div(n, skinny::kThin);
-  // one wave of resident CTAs
+  // One wave of resident CTAs; whole waves more, up to four CTAs an SM, while a
+  // thread would add up more than 40 (FP64: 32) products in a row (12 x 7 x
+  // 1,435,677 FP64 in one wave, 76: rms error 1.3 times that of four CTAs an SM).
   const int ctas = dtype_bytes == 4 ? skinny::thin_ctas<float>(skinny::thin_side(m), skinny::thin_side(n))
                                     : skinny::thin_ctas<double>(skinny::thin_side(m), skinny::thin_side(n));
   int64_t splits = split_k > 0 ? split_k : ceil_div(ctas * (int64_t)sms, groups);
+  for (int waves = 2; split_k <= 0 && waves * ctas <= 4 && ceil_div(k, splits) > (dtype_bytes == 4 ? 40 : 32) * 256; waves *= 2)
+    splits = ceil_div(waves * ctas * (int64_t)sms, groups);
   splits = std::max<int64_t>(1, std::min<int64_t>({splits, ceil_div(k, 256), 65535}));
   p.kchunk = round_up(ceil_div(k, splits), 32);  // whole 128-byte (FP64: 256) lines per split
   p.splits = (int)ceil_div(k, p.kchunk);
