@@ -336,7 +336,7 @@ cucosma_status native_gemm_gated(const cucosma_gemm_desc* d, const NativePlan& p
 
 // Skinny-shape kernels (skinny.cu) for native precision: tiny K, or tiny M or N.
 static SkinnyPlan plan_skinny_for(const cucosma_gemm_desc* d, int sms) {
-  return plan_skinny(d->m, d->n, d->k, d->dtype == CUCOSMA_R_32F ? 4 : 8, d->split_k, d->tile, sms);
+  return plan_skinny(d->m, d->n, d->k, d->dtype == CUCOSMA_R_32F ? 4 : 8, d->split_k, d->tile, d->beta, sms);
 }
 
 template <typename T>

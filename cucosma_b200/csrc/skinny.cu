@@ -2,12 +2,13 @@
 //
 // Kind 1, small K (K <= 16): the whole K fits one shared-memory tile; a CTA
 // produces a 64-row x (64 * VEC)-column block of C (M <= 4: 4 x (256 * VEC),
-// M <= 8: 8 x (128 * VEC)), each thread 16 (4) rows x VEC columns with one
-// vector store per row.  The kernel is bound by writing C
+// M <= 8: 8 x (128 * VEC) or 8 x (256 * VEC)), each thread 16 (4, 8) rows x VEC
+// columns with one vector store per row.  The kernel is bound by writing C
 // (and reading it when beta != 0), the form of 38416 x 38416 x 4 and
 // 4 x 3,000,000 x 4 (B200: 21.7 -> 14.9 us, 6.4 TB/s, with 4 rows a thread,
 // four B rows in flight and C's loads ahead; 4 x 2,000,000 x 6 FP64, beta 0.5,
-// 62 -> 39 us; 8 x 1,000,000 x 16, beta 0.5, 27 -> 23 us against 8 rows a thread).
+// 62 -> 39 us; 8 x 1,000,000 x 16, beta 0.5, 27 -> 24 us; plan_skinny says when
+// M of 5 to 8 takes which form).
 //
 // Kind 2, thin M or N (<= 8) with K > 16: a CTA owns an 8 x 8 output block and
 // one K split; its 256 threads stride over K, each keeping the 64 partial
@@ -26,8 +27,16 @@
 
 namespace cucosma {
 
+// Of a form with RPT rows a thread: resident CTAs an SM, and rows of B whose
+// loads are in flight when it comes straight from global memory.
+template <typename T, int RPT>
+struct SmallK {
+  static constexpr bool kF32 = sizeof(T) == 4;
+  static constexpr int kCtas = RPT <= 4 ? 4 : RPT > 8 ? 2 : kF32 ? 4 : 3;
+  static constexpr int kRowsB = RPT <= 4 ? 4 : kF32 ? 2 : 3;
+};
 template <typename T, int RG, int RPT>
-__global__ void __launch_bounds__(256, RPT <= 4 ? 4 : 2)
+__global__ void __launch_bounds__(256, SmallK<T, RPT>::kCtas)
     smallk_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ B, int64_t ldb, T* C, int64_t ldc,
                   int m, int n, int k, T alpha, T beta, int epi, int tiles_n, int64_t tiles) {
   // RG row groups of RPT rows x (256 / RG) column groups of VEC columns.  With
@@ -74,8 +83,8 @@ __global__ void __launch_bounds__(256, RPT <= 4 ? 4 : 2)
     for (int r = 0; r < RPT; ++r)
 #pragma unroll
       for (int e = 0; e < VEC; ++e) acc[r][e] = T(0);
-    // M <= 8: the tile's C loads go out first, beside those of B
-    constexpr bool EARLY_C = !SHARE_B;
+    // four rows a thread: the tile's C loads go out first, beside those of B
+    constexpr bool EARLY_C = !SHARE_B && RPT <= 4;
     V cold[EARLY_C ? RPT : 1];
     if (EARLY_C && beta != T(0) && col + VEC <= n) {
 #pragma unroll
@@ -84,7 +93,7 @@ __global__ void __launch_bounds__(256, RPT <= 4 ? 4 : 2)
           cold[r] = *reinterpret_cast<const V*>(C + (int64_t)(m0 + rg * RPT + r) * ldc + col);
     }
     // B straight from global memory: KU rows' loads in flight at a time
-    constexpr int KU = SHARE_B ? 1 : 4;
+    constexpr int KU = SHARE_B ? 1 : SmallK<T, RPT>::kRowsB;
     for (int k0 = 0; k0 < k; k0 += KU) {
       V bv[KU];
 #pragma unroll
@@ -123,7 +132,7 @@ __global__ void __launch_bounds__(256, RPT <= 4 ? 4 : 2)
       V cv[4];
       if constexpr (EARLY_C) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) cv[q] = cold[q];
+        for (int q = 0; q < 4; ++q) cv[q] = cold[r0 + q];
       } else if (beta != T(0) && col + VEC <= n) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -324,16 +333,24 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-SkinnyPlan plan_skinny(int64_t m, int64_t n, int64_t k, int dtype_bytes, int split_k, int tile, int sms) {
+SkinnyPlan plan_skinny(int64_t m, int64_t n, int64_t k, int dtype_bytes, int split_k, int tile, double beta, int sms) {
   SkinnyPlan p{};
   if (tile == 1 || tile == 2 || m <= 0 || n <= 0 || k <= 0) return p;  // tile ids 1, 2: always the tile kernel
   const int vec = 16 / dtype_bytes;
   if (k <= skinny::kMaxSmallK) {
     p.kind = 1;
     p.splits = 1;
-    // 4 x (256 vec) blocks when M <= 4, 8 x (128 vec) when M <= 8, else 64 x (64 vec)
+    // 4 x (256 vec) blocks when M <= 4, 8 x (128 vec) when M <= 8, else 64 x
+    // (64 vec).  The second in two groups of four rows, which both read B: that
+    // shows once C fills more than one wave of them and (FP32, whose wide form
+    // has no registers left for C ahead of its use) C is only written; then 8
+    // rows a thread (B200, beta 0: 5 x 361,026 x 2 FP32 5.7 us in groups, 4.9
+    // so; 5 x 361,026 x 13 FP64 12.8 and 10.2; 8 x 2,500,000 x 13 FP32 51.6 and
+    // 48.7.  FP32, beta 0.5, 8 x 1,000,000 x 16: 23.7 in groups).
     p.tile_m = m <= skinny::kThin ? skinny::kThin : 64;
-    p.tile_n = m <= 4 ? 256 * vec : m <= skinny::kThin ? 128 * vec : 64 * vec;
+    const bool whole = m > 4 && m <= skinny::kThin && ceil_div(n, 128 * vec) > 4 * (int64_t)sms &&
+                       (dtype_bytes == 8 || beta == 0.0);
+    p.tile_n = m <= 4 || whole ? 256 * vec : m <= skinny::kThin ? 128 * vec : 64 * vec;
     return p;
   }
   if (m > skinny::kThin && n > skinny::kThin) return p;
@@ -366,6 +383,9 @@ cudaError_t launch_skinny(const SkinnyPlan& pl, const T* A, int64_t lda, const T
     const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)sms * 8));
     if (pl.tile_m == skinny::kThin && m <= 4)  // M <= 8: one row group, B straight from global memory
       smallk_kernel<T, 1, 4><<<(unsigned)grid, 256, 0, st>>>(A, lda, B, ldb, C, ldc, m, n, k, (T)alpha, (T)beta, epi,
+                                                             tiles_n, tiles);
+    else if (pl.tile_m == skinny::kThin && pl.tile_n == 256 * Vec<T>::n)
+      smallk_kernel<T, 1, 8><<<(unsigned)grid, 256, 0, st>>>(A, lda, B, ldb, C, ldc, m, n, k, (T)alpha, (T)beta, epi,
                                                              tiles_n, tiles);
     else if (pl.tile_m == skinny::kThin)
       smallk_kernel<T, 2, 4><<<(unsigned)grid, 256, 0, st>>>(A, lda, B, ldb, C, ldc, m, n, k, (T)alpha, (T)beta, epi,

@@ -34,7 +34,7 @@ constexpr int thin_ctas(int rs, int cs) {
 }  // namespace skinny
 
 // desc must describe a native-precision GEMM with m, n, k > 0.
-SkinnyPlan plan_skinny(int64_t m, int64_t n, int64_t k, int dtype_bytes, int split_k, int tile, int sms);
+SkinnyPlan plan_skinny(int64_t m, int64_t n, int64_t k, int dtype_bytes, int split_k, int tile, double beta, int sms);
 
 template <typename T>
 cudaError_t launch_skinny(const SkinnyPlan& pl, const T* A, int64_t lda, const T* B, int64_t ldb, T* C, int64_t ldc,

@@ -187,7 +187,7 @@ extern "C" cucosma_status cucosma_tune(const cucosma_gemm_desc* d, const void* A
     // FP32 tile kernel: 128-row (tile 1) and 64-row (tile 2) CTA tiles
     if (d->dtype == CUCOSMA_R_32F) tiles = {1, 2};
     // a skinny shape: its kernel (tile 0, no block remap) against the tile kernel (tile 1)
-    if (plan_skinny(d->m, d->n, d->k, d->dtype == CUCOSMA_R_32F ? 4 : 8, 0, 0, di->sms).kind) {
+    if (plan_skinny(d->m, d->n, d->k, d->dtype == CUCOSMA_R_32F ? 4 : 8, 0, 0, d->beta, di->sms).kind) {
       bands = {1};
       tiles = {0, 1};
     }
