@@ -34,16 +34,21 @@ struct cucosma_grouped_plan_st {
 namespace cucosma {
 namespace tc {
 
-// Problem owning pre-pass block b: the number of starts <= b, less one.  The
-// block counts the (ascending) starts together -- one load latency, where a
-// binary search by every thread was nine in a row.
+// Problem owning pre-pass block b: the last one whose (ascending) start is <=
+// b.  The block's 256 threads probe as many starts at a time -- one load
+// latency for batches of up to 256 problems, two up to 65536; a binary search
+// by every thread was nine in a row for 512, and counting all starts 256 at a
+// time grew with the batch (20,000 problems of 8 to 32 a side, BF16x3: 1009 us,
+// 877 by binary search).
 __device__ __forceinline__ int find_entry(const int* __restrict__ starts, int count, int b) {
-  int n = 0;
-  for (int i = 0; i < count; i += 256) {
-    const int j = i + (int)threadIdx.x;
-    n += __syncthreads_count(j < count && starts[j] <= b);
+  int lo = 0, n = count;  // the owner is one of problems lo .. lo + n - 1
+  while (n > 1) {
+    const int step = (n + 255) / 256, at = (int)threadIdx.x * step;
+    const int below = __syncthreads_count(at < n && starts[lo + at] <= b) - 1;
+    lo += below * step;
+    n = min(step, n - below * step);
   }
-  return n - 1;
+  return lo;
 }
 
 // BF16 split of every problem (NT terms).  Blocks [0, a_blocks): kRowsPerBlock
