@@ -23,7 +23,7 @@ struct cucosma_grouped_plan_st {
   cucosma_gemm_desc desc;
   int count = 0, kind = 0, slices = 0, total_tiles = 0, grid = 0;
   int tile = 1, tile_m = 128, tile_n = 128, pair = 0, from_cache = 0;
-  int pre_a_blocks = 0, pre_b_blocks = 0, exp_a_blocks = 0, exp_b_blocks = 0;
+  int pre_depth = 1, pre_a_blocks = 0, pre_b_blocks = 0, exp_a_blocks = 0, exp_b_blocks = 0;
   int device = 0;
   void* workspace = nullptr;
   cucosma::tc::GroupEntry* table = nullptr;  // device copy inside the workspace
@@ -51,15 +51,16 @@ __device__ __forceinline__ int find_entry(const int* __restrict__ starts, int co
   return lo;
 }
 
-// BF16 split of every problem (NT terms).  Blocks [0, a_blocks): kRowsPerBlock
-// row units of some A; blocks after that: up to kStripTiles 64 x 64 tiles of
-// one column strip of some B, transposed.  Several units a block, because each
-// block first waits for its problem's table entry.
-constexpr int kRowsPerBlock = 32, kStripTiles = 4;
+// BF16 split of every problem (NT terms).  Blocks [0, a_blocks): 8 * depth row
+// units of some A; blocks after that: up to depth 64 x 64 tiles of one column
+// strip of some B, transposed.  Large batches take kPreDepth of them a block,
+// because each block first waits for its problem's table entry; batches whose
+// blocks would not fill the SMs then (four a block's loads in series) one.
+constexpr int kPreDepth = 4;
 template <int NT>
 __global__ void __launch_bounds__(256, 4)
     grouped_split_bf16_kernel(const GroupEntry* __restrict__ g, const int* __restrict__ starts, int count,
-                              int a_blocks) {
+                              int a_blocks, int depth) {
   __shared__ __align__(16) float tile[64 * 64];
   int b = blockIdx.x;
   SplitJob j{};
@@ -71,9 +72,9 @@ __global__ void __launch_bounds__(256, 4)
     j.cols = e.k;
     j.out_r = static_cast<__nv_bfloat16*>(e.planes_a);
     j.kpad_r = e.kpad;
-    const int64_t u0 = (int64_t)(b - e.pre_a_start) * kRowsPerBlock + (threadIdx.x >> 5);
+    const int64_t u0 = (int64_t)(b - e.pre_a_start) * (8 * depth) + (threadIdx.x >> 5);
 #pragma unroll 1
-    for (int i = 0; i < kRowsPerBlock; i += 8) split_rows_unit<NT>(j, u0 + i);
+    for (int i = 0; i < 8 * depth; i += 8) split_rows_unit<NT>(j, u0 + i);
   } else {
     b -= a_blocks;
     const GroupEntry& e = g[find_entry(starts + count, count, b)];
@@ -84,7 +85,7 @@ __global__ void __launch_bounds__(256, 4)
     j.cols = e.n;
     j.out_c = static_cast<__nv_bfloat16*>(e.planes_b);
     j.kpad_c = e.kpad;
-    const int tk0 = t / tiles_n * kStripTiles, tk1 = min(tk0 + kStripTiles, (int)((e.kpad + 63) / 64));
+    const int tk0 = t / tiles_n * depth, tk1 = min(tk0 + depth, (int)((e.kpad + 63) / 64));
     split_cols_strip<NT>(j, tk0, tk1, t % tiles_n, tile);
   }
 }
@@ -246,8 +247,16 @@ struct Layout {
   std::vector<size_t> off_a, off_b, off_ea, off_eb;
   std::vector<int2> units;  // work list
   int slots;                // CTAs (pairs) that walk it
-  int pre_a, pre_b, exp_a, exp_b;
+  int pre_depth, pre_a, pre_b, exp_a, exp_b;
 };
+
+// Blocks of the BF16 split of one problem's A and B, depth units a block.
+int64_t split_a_blocks(const cucosma_gemm_problem& q, int64_t kpad, int depth) {
+  return ceil_div(q.m * ceil_div(kpad / 8, kRowUnit), 8 * depth);
+}
+int64_t split_b_blocks(const cucosma_gemm_problem& q, int64_t kpad, int depth) {
+  return ceil_div(kpad, 64 * depth) * ceil_div(q.n, 64);
+}
 
 // Work list of a tile: the units (tiles of the problems, longest K first) in
 // rounds of one per slot, each round's longest to the slot with the least work
@@ -375,6 +384,10 @@ cucosma_status layout(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr
   L.off_b.resize(count);
   L.off_ea.resize(count);
   L.off_eb.resize(count);
+  int64_t deep_blocks = 0;
+  for (int i = 0; i < count; ++i)
+    deep_blocks += split_a_blocks(pr[i], round_up(pr[i].k, 8), kPreDepth) + split_b_blocks(pr[i], round_up(pr[i].k, 8), kPreDepth);
+  L.pre_depth = deep_blocks < 4 * (int64_t)sms ? 1 : kPreDepth;  // (four resident blocks an SM)
   int pa = 0, pb = 0, xa = 0, xb = 0;
   for (int i = 0; i < count; ++i) {
     const cucosma_gemm_problem& q = pr[order[i]];
@@ -398,9 +411,9 @@ cucosma_status layout(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr
     e.lda = q.lda;
     e.ldb = q.ldb;
     e.pre_a_start = pa;
-    pa += (int)(L.kind == 2 ? ceil_div(q.m, 8) : ceil_div(q.m * ceil_div(e.kpad / 8, kRowUnit), kRowsPerBlock));
+    pa += (int)(L.kind == 2 ? ceil_div(q.m, 8) : split_a_blocks(q, e.kpad, L.pre_depth));
     e.pre_b_start = pb;
-    pb += L.kind == 2 ? (int)(ceil_div(e.kpad, 32) * ceil_div(q.n, 64)) : (int)(ceil_div(e.kpad, 64 * kStripTiles) * ceil_div(q.n, 64));
+    pb += L.kind == 2 ? (int)(ceil_div(e.kpad, 32) * ceil_div(q.n, 64)) : (int)split_b_blocks(q, e.kpad, L.pre_depth);
     e.exp_a_start = xa;
     xa += (int)ceil_div(q.m, 8);
     e.exp_b_start = xb;
@@ -527,6 +540,7 @@ extern "C" cucosma_status cucosma_grouped_plan_create(const cucosma_gemm_desc* d
   p->tile_n = L.bn;
   p->pair = L.pair;
   p->from_cache = from_cache;
+  p->pre_depth = L.pre_depth;
   p->pre_a_blocks = L.pre_a;
   p->pre_b_blocks = L.pre_b;
   p->exp_a_blocks = L.exp_a;
@@ -591,9 +605,11 @@ extern "C" cucosma_status cucosma_gemm_grouped(cucosma_grouped_plan plan, void* 
   if (plan->kind != 2) {
     const unsigned blocks = (unsigned)(plan->pre_a_blocks + plan->pre_b_blocks);
     if (plan->slices == 3)
-      grouped_split_bf16_kernel<3><<<blocks, 256, 0, st>>>(plan->table, plan->starts, plan->count, plan->pre_a_blocks);
+      grouped_split_bf16_kernel<3><<<blocks, 256, 0, st>>>(plan->table, plan->starts, plan->count, plan->pre_a_blocks,
+                                                           plan->pre_depth);
     else
-      grouped_split_bf16_kernel<2><<<blocks, 256, 0, st>>>(plan->table, plan->starts, plan->count, plan->pre_a_blocks);
+      grouped_split_bf16_kernel<2><<<blocks, 256, 0, st>>>(plan->table, plan->starts, plan->count, plan->pre_a_blocks,
+                                                           plan->pre_depth);
     e = cudaGetLastError();
     if (e != cudaSuccess) return CUCOSMA_STATUS_LAUNCH_FAILED;
     prof_begin(st);

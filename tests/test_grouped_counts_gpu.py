@@ -38,3 +38,27 @@ def test_counts(cuda, count, precision):
     cc.grouped(probs, precision=precision)()
     assert torch.equal(Cs, As @ Bs) and torch.equal(Cb, Ab @ Bb)
     assert cc.device_status() == (cc.SUCCESS, 0)
+
+
+@pytest.mark.parametrize("precision", ["bf16x3", "bf16x6"])
+@pytest.mark.parametrize("copies", [1, 8, 60])
+def test_prepass_depth(cuda, copies, precision):
+    """Batches on both sides of the pre-pass's choice of row units and tiles a
+    block (one copy takes some 65 blocks at the greater depth, 60 take 3900),
+    with rows of more than one unit and column strips of one to many tiles."""
+    import torch
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(6)
+
+    def ints(r, c):
+        t = torch.zeros((r, -(-c // 4) * 4), device="cuda")
+        t[:, :c] = torch.randint(-8, 9, (r, c), generator=g, device="cuda").float()
+        return t[:, :c]
+
+    shapes = [(300, 200, 701), (33, 70, 2113), (31, 65, 64), (100, 1, 257), (1, 129, 4099)]
+    probs = [(ints(m, k), ints(k, n), ints(m, n)) for _ in range(copies) for m, n, k in shapes]
+    cc.grouped(probs, precision=precision)()
+    for A, B, C in probs:
+        assert torch.equal(C, A @ B)  # integers: below 2^24, exact in any order
+    assert cc.device_status() == (cc.SUCCESS, 0)
