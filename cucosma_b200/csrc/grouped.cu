@@ -13,6 +13,7 @@
 // no longer leave most of the GPU idle the way one launch per problem does.
 #include <algorithm>
 #include <cstring>
+#include <new>
 #include <vector>
 
 #include "split_device.cuh"
@@ -245,7 +246,8 @@ struct Layout {
   size_t table_bytes, total_bytes, off_starts, off_units;
   std::vector<GroupEntry> entries;  // pointers relative to the workspace base (offsets)
   std::vector<size_t> off_a, off_b, off_ea, off_eb;
-  std::vector<int2> units;  // work list
+  std::vector<int> order;   // table order of the problems
+  int64_t positions;        // of the work list: whole rounds of one unit a slot
   int slots;                // CTAs (pairs) that walk it
   int pre_depth, pre_a, pre_b, exp_a, exp_b;
 };
@@ -275,9 +277,9 @@ int64_t work_list(const cucosma_gemm_problem* pr, const std::vector<int>& order,
   int next = slots;                                   // slots of this round served so far
   for (int e = 0; e < (int)order.size(); ++e) {
     const cucosma_gemm_problem& p = pr[order[e]];
-    const int tiles = (int)(ceil_div(p.m, tile_m) * ceil_div(p.n, bn));
+    const int64_t tiles = ceil_div(p.m, tile_m) * ceil_div(p.n, bn);
     const int64_t work = ceil_div(p.k, 32) + kUnitOverhead;
-    for (int t = 0; t < tiles; ++t) {
+    for (int64_t t = 0; t < tiles; ++t) {
       if (next == slots) {
         const int64_t least = *std::min_element(load.begin(), load.end());
         for (int s = 0; s < slots; ++s) round[s] = {(load[s] - least) / work, s};
@@ -287,7 +289,7 @@ int64_t work_list(const cucosma_gemm_problem* pr, const std::vector<int>& order,
       }
       const int s = round[next++].second;
       load[s] += work;
-      if (list) (*list)[list->size() - slots + s] = int2{e, t};
+      if (list) (*list)[list->size() - slots + s] = int2{e, (int)t};
     }
   }
   return *std::max_element(load.begin(), load.end());
@@ -298,10 +300,29 @@ int launch_slots(int64_t units, int pair, int sms) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(units, pair ? max_pair_clusters<Bf16x3PairSmall>(sms) : sms));
 }
 
+// Tiles of all problems; their numbers and the work list's positions are ints,
+// so batches of more are refused.
+constexpr int64_t kMaxUnits = INT32_MAX - 4096;
 int64_t unit_count(const cucosma_gemm_problem* pr, int count, int tile_m, int bn) {
   int64_t n = 0;
-  for (int i = 0; i < count; ++i) n += ceil_div(pr[i].m, tile_m) * ceil_div(pr[i].n, bn);
+  for (int i = 0; i < count && n <= kMaxUnits; ++i) n += ceil_div(pr[i].m, tile_m) * ceil_div(pr[i].n, bn);
   return n;
+}
+
+// Work of the busiest slot.  Past kWalkUnits units a slot has thousands, whose
+// spread no longer matters, and dealing them out would take the host longer
+// than it saves: the mean and one unit more stand for it.
+constexpr int64_t kWalkUnits = 1 << 20;
+double busiest_slot(const cucosma_gemm_problem* pr, const std::vector<int>& order, int tile_m, int bn, int64_t units,
+                    int slots) {
+  if (units <= kWalkUnits) return (double)work_list(pr, order, tile_m, bn, slots, nullptr);
+  double total = 0.0, most = 0.0;
+  for (int e : order) {
+    const double work = (double)(ceil_div(pr[e].k, 32) + kUnitOverhead);
+    total += work * (double)(ceil_div(pr[e].m, tile_m) * ceil_div(pr[e].n, bn));
+    most = std::max(most, work);
+  }
+  return total / slots + most;
 }
 
 // Automatic tile: of the tiles that give bit-identical results, the one whose
@@ -323,8 +344,9 @@ int automatic_tile(int kind, const cucosma_gemm_problem* pr, const std::vector<i
   int best = 1;
   double t_best = 1e300;
   for (const Option* o = kind == 0 ? kV3 : kV6, *end = o + (kind == 0 ? 3 : 2); o != end; ++o) {
-    const int slots = launch_slots(unit_count(pr, count, o->tile_m, o->bn), o->pair, sms);
-    const double t = o->us * (double)work_list(pr, order, o->tile_m, o->bn, slots, nullptr);
+    const int64_t units = unit_count(pr, count, o->tile_m, o->bn);
+    const int slots = launch_slots(units, o->pair, sms);
+    const double t = o->us * busiest_slot(pr, order, o->tile_m, o->bn, units, slots);
     if (t < t_best) {
       t_best = t;
       best = o->id;
@@ -356,13 +378,15 @@ cucosma_status layout(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr
   }
   // Table order: K descending (stable): the long-K tiles are dealt out first
   // and the short ones even out the end.
-  std::vector<int> order(count);
+  std::vector<int>& order = L.order;
+  order.resize(count);
   for (int i = 0; i < count; ++i) order[i] = i;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return pr[a].k > pr[b].k; });
   if (tile < 0) tile = d->tile;
   GTile g{};
-  if (!grouped_tile(L.kind, L.slices, tile > 0 ? tile : automatic_tile(L.kind, pr, order, sms), g))
-    return CUCOSMA_STATUS_NOT_SUPPORTED;
+  if (!grouped_tile(L.kind, L.slices, tile != 0 ? tile : 1, g)) return CUCOSMA_STATUS_NOT_SUPPORTED;
+  if (unit_count(pr, count, g.tile_m, g.bn) > kMaxUnits) return CUCOSMA_STATUS_NOT_SUPPORTED;
+  if (tile == 0) grouped_tile(L.kind, L.slices, automatic_tile(L.kind, pr, order, sms), g);
   L.bn = g.bn;
   L.tile_m = g.tile_m;
   L.pair = g.pair;
@@ -371,13 +395,11 @@ cucosma_status layout(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr
   const int es_pl = L.kind == 2 ? 1 : 2;
   const int64_t kmax_exact = ((int64_t)2147483647 / ((int64_t)L.slices * 127 * 127)) / 32 * 32;
   const int64_t units = unit_count(pr, count, L.tile_m, L.bn);
-  if (units > (1 << 26)) return CUCOSMA_STATUS_NOT_SUPPORTED;  // (the work list: 2^26 tiles are 8 bytes each)
   L.slots = launch_slots(units, L.pair, sms);
-  L.units.clear();
-  work_list(pr, order, L.tile_m, L.bn, L.slots, &L.units);
+  L.positions = ceil_div(units, L.slots) * L.slots;
   L.off_starts = al256(sizeof(GroupEntry) * (size_t)count);
   L.off_units = L.off_starts + al256(sizeof(int) * 4 * (size_t)count);
-  L.table_bytes = L.off_units + al256(sizeof(int2) * L.units.size());
+  L.table_bytes = L.off_units + al256(sizeof(int2) * (size_t)L.positions);
   size_t off = L.table_bytes;
   L.entries.assign(count, GroupEntry{});
   L.off_a.resize(count);
@@ -455,10 +477,8 @@ size_t grouped_table_bytes(const cucosma_gemm_desc* d, const cucosma_gemm_proble
 using namespace cucosma;
 using namespace cucosma::tc;
 
-extern "C" cucosma_status cucosma_grouped_workspace_size(const cucosma_gemm_desc* d,
-                                                         const cucosma_gemm_problem* problems, int count,
-                                                         size_t* bytes) {
-  if (!bytes) return CUCOSMA_STATUS_INVALID_VALUE;
+static cucosma_status grouped_workspace_size(const cucosma_gemm_desc* d, const cucosma_gemm_problem* problems,
+                                             int count, size_t* bytes) {
   const DeviceInfo* di = device_info();
   const int sms = di ? di->sms : 148;  // (sizes can be asked for without a device)
   Layout L;
@@ -472,12 +492,8 @@ extern "C" cucosma_status cucosma_grouped_workspace_size(const cucosma_gemm_desc
   return CUCOSMA_STATUS_SUCCESS;
 }
 
-extern "C" cucosma_status cucosma_grouped_plan_create(const cucosma_gemm_desc* d,
-                                                      const cucosma_gemm_problem* problems, int count,
-                                                      void* workspace, size_t workspace_bytes,
-                                                      cucosma_grouped_plan* plan) {
-  if (!plan) return CUCOSMA_STATUS_INVALID_VALUE;
-  *plan = nullptr;
+static cucosma_status grouped_plan_create(const cucosma_gemm_desc* d, const cucosma_gemm_problem* problems, int count,
+                                          void* workspace, size_t workspace_bytes, cucosma_grouped_plan* plan) {
   const DeviceInfo* di = device_info();
   if (!di) return CUCOSMA_STATUS_LAUNCH_FAILED;
   if (di->cc_major != 10 || di->cc_minor != 0) return CUCOSMA_STATUS_ARCH_MISMATCH;
@@ -525,7 +541,10 @@ extern "C" cucosma_status cucosma_grouped_plan_create(const cucosma_gemm_desc* d
     starts[2 * count + i] = e.exp_a_start;
     starts[3 * count + i] = e.exp_b_start;
   }
-  std::memcpy(image.data() + L.off_units, L.units.data(), sizeof(int2) * L.units.size());
+  std::vector<int2> units;
+  units.reserve((size_t)L.positions);
+  work_list(problems, L.order, L.tile_m, L.bn, L.slots, &units);
+  std::memcpy(image.data() + L.off_units, units.data(), sizeof(int2) * units.size());
   if (cudaMemcpy(workspace, image.data(), L.table_bytes, cudaMemcpyHostToDevice) != cudaSuccess)
     return CUCOSMA_STATUS_LAUNCH_FAILED;
   auto* p = new cucosma_grouped_plan_st;
@@ -533,7 +552,7 @@ extern "C" cucosma_status cucosma_grouped_plan_create(const cucosma_gemm_desc* d
   p->count = count;
   p->kind = L.kind;
   p->slices = L.slices;
-  p->total_tiles = (int)L.units.size();
+  p->total_tiles = (int)L.positions;
   p->grid = L.slots * (L.pair ? 2 : 1);
   p->tile = L.tile;
   p->tile_m = L.tile_m;
@@ -557,6 +576,31 @@ extern "C" cucosma_status cucosma_grouped_plan_create(const cucosma_gemm_desc* d
 extern "C" cucosma_status cucosma_grouped_plan_destroy(cucosma_grouped_plan plan) {
   delete plan;
   return CUCOSMA_STATUS_SUCCESS;
+}
+
+// The tables are built in host memory first; a batch too large for that is an error, not an exception.
+extern "C" cucosma_status cucosma_grouped_workspace_size(const cucosma_gemm_desc* d,
+                                                         const cucosma_gemm_problem* problems, int count,
+                                                         size_t* bytes) {
+  if (!bytes) return CUCOSMA_STATUS_INVALID_VALUE;
+  try {
+    return grouped_workspace_size(d, problems, count, bytes);
+  } catch (const std::bad_alloc&) {
+    return CUCOSMA_STATUS_ALLOC_FAILED;
+  }
+}
+
+extern "C" cucosma_status cucosma_grouped_plan_create(const cucosma_gemm_desc* d,
+                                                      const cucosma_gemm_problem* problems, int count,
+                                                      void* workspace, size_t workspace_bytes,
+                                                      cucosma_grouped_plan* plan) {
+  if (!plan) return CUCOSMA_STATUS_INVALID_VALUE;
+  *plan = nullptr;
+  try {
+    return grouped_plan_create(d, problems, count, workspace, workspace_bytes, plan);
+  } catch (const std::bad_alloc&) {
+    return CUCOSMA_STATUS_ALLOC_FAILED;
+  }
 }
 
 extern "C" cucosma_status cucosma_grouped_plan_get_tile(cucosma_grouped_plan plan, int32_t* tile, int32_t* tile_m,
