@@ -86,6 +86,9 @@ int grouped_tuned_tile(const cucosma_gemm_desc* d, const cucosma_gemm_problem* p
 // (problem table, block starts, work list): the most any tile takes.
 size_t grouped_table_bytes(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr, int count,
                            const DeviceInfo* di);
+// The tile a plan of this batch takes by itself (tile 0, nothing tuned), 0 for a batch that is refused.
+int grouped_automatic_tile(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr, int count,
+                           const DeviceInfo* di);
 
 // Launch accounting and optional timing of the main GEMM kernel of each call:
 // note_launches() counts every kernel the library enqueues; prof_begin /

@@ -217,7 +217,6 @@ size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 //           4 / 5 = 256 x 128 / 256 x 256 CTA pair, bit-identical to 1
 //   BF16X6  1 = 128 x 128, 2 = 256 x 256 CTA pair (split release)
 //   OZAKI   1 = 128 x ozaki_bn(slices)
-constexpr int kTileIds = 5;
 struct GTile {
   int id, tile_m, bn, pair;
 };
@@ -244,6 +243,7 @@ bool grouped_tile(int kind, int slices, int id, GTile& g) {
 struct Layout {
   int kind, slices, bn, tile_m, pair, tile;
   size_t table_bytes, total_bytes, off_starts, off_units;
+  size_t most_table_bytes;  // table_bytes of the tile with the longest work list
   std::vector<GroupEntry> entries;  // pointers relative to the workspace base (offsets)
   std::vector<size_t> off_a, off_b, off_ea, off_eb;
   std::vector<int> order;   // table order of the problems
@@ -395,11 +395,18 @@ cucosma_status layout(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr
   const int es_pl = L.kind == 2 ? 1 : 2;
   const int64_t kmax_exact = ((int64_t)2147483647 / ((int64_t)L.slices * 127 * 127)) / 32 * 32;
   const int64_t units = unit_count(pr, count, L.tile_m, L.bn);
+  auto list_length = [&](int64_t n, int slots) { return ceil_div(n, slots) * slots; };
   L.slots = launch_slots(units, L.pair, sms);
-  L.positions = ceil_div(units, L.slots) * L.slots;
+  L.positions = list_length(units, L.slots);
   L.off_starts = al256(sizeof(GroupEntry) * (size_t)count);
   L.off_units = L.off_starts + al256(sizeof(int) * 4 * (size_t)count);
   L.table_bytes = L.off_units + al256(sizeof(int2) * (size_t)L.positions);
+  L.most_table_bytes = L.table_bytes;
+  for (int id = 1; grouped_tile(L.kind, L.slices, id, g); ++id) {
+    const int64_t n = unit_count(pr, count, g.tile_m, g.bn);
+    if (n <= kMaxUnits)
+      L.most_table_bytes = std::max(L.most_table_bytes, L.off_units + al256(sizeof(int2) * (size_t)list_length(n, launch_slots(n, g.pair, sms))));
+  }
   size_t off = L.table_bytes;
   L.entries.assign(count, GroupEntry{});
   L.off_a.resize(count);
@@ -464,12 +471,14 @@ cucosma_status layout(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr
 
 size_t grouped_table_bytes(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr, int count,
                            const DeviceInfo* di) {
-  size_t most = 0;
-  for (int id = 1; id <= tc::kTileIds; ++id) {
-    tc::Layout L;
-    if (tc::layout(d, pr, count, di->sms, L, id) == CUCOSMA_STATUS_SUCCESS) most = std::max(most, L.table_bytes);
-  }
-  return most;
+  tc::Layout L;
+  return tc::layout(d, pr, count, di->sms, L, 1) == CUCOSMA_STATUS_SUCCESS ? L.most_table_bytes : 0;
+}
+
+int grouped_automatic_tile(const cucosma_gemm_desc* d, const cucosma_gemm_problem* pr, int count,
+                           const DeviceInfo* di) {
+  tc::Layout L;
+  return tc::layout(d, pr, count, di->sms, L, 0) == CUCOSMA_STATUS_SUCCESS ? L.tile : 0;
 }
 
 }  // namespace cucosma
@@ -484,11 +493,9 @@ static cucosma_status grouped_workspace_size(const cucosma_gemm_desc* d, const c
   Layout L;
   cucosma_status s = layout(d, problems, count, sms, L);
   if (s != CUCOSMA_STATUS_SUCCESS) return s;
-  *bytes = L.total_bytes;
-  // a plan with tile 0 may take the tuner's tile, whose work list can be longer
-  const int tuned = d->tile == 0 && di ? grouped_tuned_tile(d, problems, count, di) : 0;
-  if (tuned > 0 && layout(d, problems, count, sms, L, tuned) == CUCOSMA_STATUS_SUCCESS)
-    *bytes = std::max(*bytes, L.total_bytes);
+  // tile 0: room for the list of any tile, so that the tuner can try them all
+  // here and a plan made after it can take its choice
+  *bytes = L.total_bytes + (d->tile == 0 ? L.most_table_bytes - L.table_bytes : 0);
   return CUCOSMA_STATUS_SUCCESS;
 }
 

@@ -300,11 +300,14 @@ extern "C" cucosma_status cucosma_tune_grouped(const cucosma_gemm_desc* d, const
   const DeviceInfo* di = device_info();
   if (!di) return CUCOSMA_STATUS_LAUNCH_FAILED;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // Candidate tiles of the grouped launch (see cucosma_grouped_plan_create).
+  // Candidate tiles of the grouped launch (see cucosma_grouped_plan_create),
+  // the batch's automatic one among them: tuning never loses to it.
   std::vector<int> tiles;
   if (d->precision == CUCOSMA_PRECISION_BF16X3) tiles = {1, 2, 3};
   else if (d->precision == CUCOSMA_PRECISION_BF16X6) tiles = {1, 2};
   else tiles = {1};
+  const int automatic = grouped_automatic_tile(d, problems, count, di);
+  if (automatic > 0 && std::find(tiles.begin(), tiles.end(), automatic) == tiles.end()) tiles.push_back(automatic);
   if (!workspace) return CUCOSMA_STATUS_WORKSPACE_TOO_SMALL;
   const SavedTables saved(workspace, std::min(workspace_bytes, grouped_table_bytes(d, problems, count, di)), st);
   if (!saved.ok) return CUCOSMA_STATUS_LAUNCH_FAILED;

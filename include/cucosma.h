@@ -273,12 +273,13 @@ CUCOSMA_API cucosma_status cucosma_grouped_plan_get_tile(cucosma_grouped_plan pl
                                                          int32_t* tile_n, int32_t* from_cache);
 
 /* The grouped launch's counterpart: its candidate tiles (BF16X3: 128 x 128,
- * 128 x 256, 256 x 256 CTA pair; BF16X6: 128 x 128, 256 x 256 pair; Ozaki:
- * one) are run on the problems (their C is overwritten) and the fastest is
+ * 128 x 256, 256 x 256 CTA pair, and 4 or 5 where a plan with tile 0 takes
+ * it; BF16X6: 128 x 128, 256 x 256 pair; Ozaki: one) are run on the problems (their C is overwritten) and the fastest is
  * cached for this batch's shape mix (SM count, dtype, precision, slices and
  * the problems' m, n, k in order).  cucosma_grouped_plan_create uses it when
- * the descriptor's tile is 0.  out->tile is the chosen grouped tile id.  The
- * workspace may be that of a plan of these problems: the call waits for the
+ * the descriptor's tile is 0.  out->tile is the chosen grouped tile id.  A
+ * workspace of the size asked for with tile 0 holds any of them; candidates
+ * that do not fit a smaller one are skipped.  The workspace may be that of a plan of these problems: the call waits for the
  * stream first and leaves the plan's tables as they were. */
 CUCOSMA_API cucosma_status cucosma_tune_grouped(const cucosma_gemm_desc* d, const cucosma_gemm_problem* problems,
                                                 int count, void* workspace, size_t workspace_bytes,

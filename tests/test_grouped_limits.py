@@ -46,3 +46,11 @@ def test_tile_ids(precision, ids):
     for tile in range(-2, 8):
         ok = 0 <= tile <= ids
         assert query([(300, 200, 100)], precision, tile)[0] == (cc.SUCCESS if ok else cc.NOT_SUPPORTED), tile
+
+
+@pytest.mark.parametrize("precision,ids", [("bf16x3", 5), ("bf16x6", 2), ("ozaki", 1)])
+def test_size_asked_for_with_tile_0_holds_every_tile(precision, ids):
+    waves = [(2048, 1500, 200), (1000, 2048, 777), (700, 1100, 1300), (2040, 260, 64), (130, 1999, 2300)]
+    for probs in (waves, waves * 20, [(10, 10, 10)], [(900, 1, 30)] * 700):
+        any_tile = query(probs, precision)[1]
+        assert any_tile == max(query(probs, precision, tile)[1] for tile in range(1, ids + 1))

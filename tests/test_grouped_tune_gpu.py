@@ -53,3 +53,24 @@ def test_plan_outlives_a_tune_on_its_workspace(cuda, precision, tile):
         assert cc.device_status() == (cc.SUCCESS, 0)
     finally:
         cc.tune_cache_clear()
+
+
+@pytest.mark.parametrize("precision,candidates", [("bf16x3", 4), ("bf16x6", 2)])
+def test_tune_measures_the_automatic_tile(cuda, precision, candidates):
+    """A batch whose automatic tile (BF16x3) is not 128 x 128: every tile fits the
+    plan's workspace, and the automatic one is measured with the others."""
+    import torch
+
+    cc.tune_cache_clear()
+    try:
+        probs = problems(torch, WAVES)
+        plan = cc.grouped(probs, precision=precision)
+        automatic = plan.tile()[0]
+        assert automatic != 1 or precision == "bf16x6"
+        r = plan.tune()
+        assert r["candidates"] == candidates and r["tile"] in {1, 2, 3, automatic}
+        tuned = cc.grouped(probs, precision=precision)
+        assert tuned.tile()[0] == r["tile"] and tuned.tile()[3]
+        assert tuned.workspace.numel() == plan.workspace.numel()
+    finally:
+        cc.tune_cache_clear()
