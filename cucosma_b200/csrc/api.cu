@@ -381,7 +381,7 @@ static cucosma_status run_gemm(const cucosma_gemm_desc* d, const void* A, const 
   if (!di) return CUCOSMA_STATUS_LAUNCH_FAILED;
   if (di->cc_major != 10 || di->cc_minor != 0) return CUCOSMA_STATUS_ARCH_MISMATCH;
   cucosma_gemm_desc tuned;
-  d = apply_tuning(d, &tuned, di);
+  if (!(prep & kAsGiven)) d = apply_tuning(d, &tuned, di);
   const bool fp32 = d->dtype == CUCOSMA_R_32F;
   if (d->k == 0 || d->alpha == 0.0) {
     cudaError_t e = fp32 ? simt::launch_scale<float>((float*)C, d->ldc, (int)d->m, (int)d->n, d->beta, d->epilogue,
@@ -514,7 +514,10 @@ extern "C" cucosma_status cucosma_gemm_get_plan(const cucosma_gemm_desc* d, cuco
   const DeviceInfo* di = device_info();
   if (!di) return CUCOSMA_STATUS_LAUNCH_FAILED;
   cucosma_gemm_desc tuned;
-  d = apply_tuning(d, &tuned, di);
+  return plan_as_given(apply_tuning(d, &tuned, di), info, di);
+}
+
+cucosma_status cucosma::plan_as_given(const cucosma_gemm_desc* d, cucosma_plan_info* info, const DeviceInfo* di) {
   if (d->precision == CUCOSMA_PRECISION_NATIVE && plan_skinny_for(d, di->sms).kind) {
     const SkinnyPlan sp = plan_skinny_for(d, di->sms);
     info->path = 0;

@@ -22,7 +22,8 @@ void wait_ctl(const DeviceInfo* di, int** status, unsigned long long* timeout_ns
 // Operand pre-passes of the tensor-core paths (see tc_gemm_ex).
 // kNoFused: never the fused-split kernel, even with both pre-passes (the
 // host-buffer call's row blocks share B's planes, which it does not write).
-enum : int { kPrepA = 1, kPrepB = 2, kNoFused = 4 };
+// kAsGiven: the descriptor as it is, whatever the tuning cache holds for it (the tuner's own runs).
+enum : int { kPrepA = 1, kPrepB = 2, kNoFused = 4, kAsGiven = 8 };
 
 struct NativePlan {
   int bm;  // CTA tile rows: 128, or 64 (FP32 only); 128 columns either way
@@ -43,6 +44,10 @@ cucosma_status gemm(const cucosma_gemm_desc* d, const void* A, const void* B, vo
 // (kPrepA / kPrepB; the native paths have none).
 cucosma_status gemm_ex(const cucosma_gemm_desc* d, const void* A, const void* B, void* C, void* ws, size_t ws_bytes,
                        cudaStream_t st, int prep);
+
+// Workspace and plan of the descriptor as it is, whatever the tuning cache holds.
+cucosma_status workspace_size(const cucosma_gemm_desc* d, size_t* bytes, const DeviceInfo* di);
+cucosma_status plan_as_given(const cucosma_gemm_desc* d, cucosma_plan_info* info, const DeviceInfo* di);
 
 bool encode_2d(CUtensorMap* map, CUtensorMapDataType dt, int elem_bytes, const void* base, uint64_t inner,
                uint64_t outer, uint64_t row_stride_elems, uint32_t box_inner, uint32_t box_outer,

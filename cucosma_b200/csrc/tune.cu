@@ -173,9 +173,9 @@ extern "C" cucosma_status cucosma_tune(const cucosma_gemm_desc* d, const void* A
   cucosma_gemm_desc base = *d;
   base.split_k = base.swizzle = base.tile = 0;
 
-  // Candidate set.
-  cucosma_plan_info pi;
-  if ((s = cucosma_gemm_get_plan(&base, &pi)) != CUCOSMA_STATUS_SUCCESS) return s;
+  // Candidate set: around the automatic plan, which is in it.
+  cucosma_plan_info pi{};
+  if ((s = plan_as_given(&base, &pi, di)) != CUCOSMA_STATUS_SUCCESS) return s;
   const int64_t kblocks = (d->k + pi.tile_k - 1) / pi.tile_k;
   std::vector<int> splits = {pi.splits};
   for (int sk : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64})
@@ -195,9 +195,10 @@ extern "C" cucosma_status cucosma_tune(const cucosma_gemm_desc* d, const void* A
     bands = {8, 4, 16};
     // tensor-core tiles: BF16x3 128x128, 128x256, 256x256 (CTA pair);
     // BF16x6 128x128, 256x128 (pair), 256x256 (pair); with operands of 32 MB
-    // or more also the fused-split pair (BF16x3 tile 5, BF16x6 tile 4); Ozaki
-    // one tile per slice count
-    const bool big = ((double)d->m * d->k + (double)d->k * d->n) * 4.0 >= 32.0 * (1 << 20) && d->flags == 0;
+    // or more, or where the automatic plan takes it, also the fused-split pair
+    // (BF16x3 tile 5, BF16x6 tile 4); Ozaki one tile per slice count
+    const bool big = pi.fused ||
+                     (((double)d->m * d->k + (double)d->k * d->n) * 4.0 >= 32.0 * (1 << 20) && d->flags == 0);
     if (d->precision == CUCOSMA_PRECISION_BF16X3) tiles = big ? std::vector<int>{2, 3, 4, 5} : std::vector<int>{2, 3, 4};
     if (d->precision == CUCOSMA_PRECISION_BF16X6) tiles = big ? std::vector<int>{1, 2, 3, 4} : std::vector<int>{1, 2, 3};
   }
@@ -205,11 +206,18 @@ extern "C" cucosma_status cucosma_tune(const cucosma_gemm_desc* d, const void* A
     int sk, sw, ti;
   };
   std::vector<Cand> cands;
+  // A K-split last wave has no tile id and split count of its own: the
+  // descriptor that leaves all to the library stands for it (and is then what
+  // the cache holds).
+  if (pi.path != 0 && pi.path != 3 && !pi.fused && pi.splits == 1 && pi.launches == 3) cands.push_back({0, 0, 0});
   for (int ti : tiles)
     for (int sw : bands)
       for (int sk : splits) cands.push_back({sk, sw, ti});
   if (max_candidates > 0 && (int)cands.size() > max_candidates) cands.resize(max_candidates);
 
+  auto run = [&](const cucosma_gemm_desc& t) {
+    return gemm_ex(&t, A, B, C, workspace, workspace_bytes, st, kPrepA | kPrepB | kAsGiven);
+  };
   cudaEvent_t e0, e1;
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) return CUCOSMA_STATUS_LAUNCH_FAILED;
   double best = 1e300;
@@ -221,12 +229,12 @@ extern "C" cucosma_status cucosma_tune(const cucosma_gemm_desc* d, const void* A
     t.swizzle = c.sw;
     t.tile = c.ti;
     size_t need = 0;
-    if (cucosma_gemm_workspace_size(&t, &need) != CUCOSMA_STATUS_SUCCESS || need > workspace_bytes) continue;
-    if (gemm(&t, A, B, C, workspace, workspace_bytes, st) != CUCOSMA_STATUS_SUCCESS) continue;  // warm-up
+    if (workspace_size(&t, &need, di) != CUCOSMA_STATUS_SUCCESS || need > workspace_bytes) continue;
+    if (run(t) != CUCOSMA_STATUS_SUCCESS) continue;  // warm-up
     double tmin = 1e300;
     for (int r = 0; r < 3; ++r) {
       cudaEventRecord(e0, st);
-      gemm(&t, A, B, C, workspace, workspace_bytes, st);
+      run(t);
       cudaEventRecord(e1, st);
       if (cudaEventSynchronize(e1) != cudaSuccess) {
         cudaEventDestroy(e0);
@@ -255,8 +263,7 @@ extern "C" cucosma_status cucosma_tune(const cucosma_gemm_desc* d, const void* A
       t.split_k = pick.sk;
       t.swizzle = pick.sw;
       t.tile = pick.ti;
-      measure_counters([&] { return gemm(&t, A, B, C, workspace, workspace_bytes, st) == CUCOSMA_STATUS_SUCCESS; }, st,
-                       &cr);
+      measure_counters([&] { return run(t) == CUCOSMA_STATUS_SUCCESS; }, st, &cr);
     } else {
       cr.why = "disabled by CUCOSMA_TUNE_COUNTERS=off";
     }
@@ -279,8 +286,8 @@ extern "C" cucosma_status cucosma_tune(const cucosma_gemm_desc* d, const void* A
     t.split_k = pick.sk;
     t.swizzle = pick.sw;
     t.tile = pick.ti;
-    cucosma_plan_info pk;
-    cucosma_gemm_get_plan(&t, &pk);
+    cucosma_plan_info pk{};
+    plan_as_given(&t, &pk, di);
     if (d->precision == CUCOSMA_PRECISION_NATIVE)
       out->occupancy = d->dtype == CUCOSMA_R_32F ? simt::occupancy<float>(pk.tile_m == 64 ? 64 : simt::BM)
                                                  : simt::occupancy<double>();

@@ -178,7 +178,7 @@ CUCOSMA_API cucosma_status cucosma_dgemm(int m, int n, int k, double alpha, cons
  * all 0.  The cache is saved / loaded as a text file; $CUCOSMA_TUNE_CACHE is
  * loaded on first use, CUCOSMA_TUNE=off disables lookups. */
 typedef struct cucosma_tune_result {
-  int32_t split_k, swizzle, tile; /* the chosen configuration */
+  int32_t split_k, swizzle, tile; /* the chosen configuration (all 0: the library's own choice was fastest) */
   int32_t candidates;             /* configurations measured */
   int32_t occupancy;              /* resident CTAs per SM of the chosen kernel */
   int32_t reserved;
