@@ -290,7 +290,7 @@ extern "C" cucosma_status cucosma_tune(const cucosma_gemm_desc* d, const void* A
     plan_as_given(&t, &pk, di);
     if (d->precision == CUCOSMA_PRECISION_NATIVE)
       out->occupancy = d->dtype == CUCOSMA_R_32F ? simt::occupancy<float>(pk.tile_m == 64 ? 64 : simt::BM)
-                                                 : simt::occupancy<double>();
+                                                 : simt::occupancy<double>(pk.tile_m == 64 ? 64 : simt::BM);
     else
       out->occupancy = 1;  // persistent kernel, one CTA per SM by construction
     out->l2_hit_rate = cr.l2_hit_pct;

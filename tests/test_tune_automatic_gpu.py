@@ -65,3 +65,20 @@ def test_fused_tile_is_a_candidate_where_the_plan_takes_it(cuda, precision, tile
         assert per_tile == 1 and few["candidates"] % 4 == 0  # four tiles of as many bands and splits each
     finally:
         cc.tune_cache_clear()
+
+
+@pytest.mark.parametrize("m,n,k", [(200, 300, 500), (3000, 2900, 200)])
+def test_occupancy_of_the_fp64_tile(cuda, m, n, k):
+    """Four 64 x 64 CTAs an SM, one of 128 x 128."""
+    import torch
+
+    cc.tune_cache_clear()
+    try:
+        A, B, C = (t.double() for t in operands(torch, m, n, k))
+        A, B, C = (torch.zeros((t.shape[0], t.shape[1] + t.shape[1] % 2), dtype=t.dtype, device="cuda")[:, :t.shape[1]]
+                   .copy_(t) for t in (A, B, C))
+        r = cc.tune(A, B, C)
+        tile_m = cc.get_plan(cc.make_desc(A, B, C))["tile_m"]
+        assert r["occupancy"] == (4 if tile_m == 64 else 1)
+    finally:
+        cc.tune_cache_clear()
