@@ -46,6 +46,7 @@ const DeviceInfo* device_info() {
     d.cc_major = prop.major;
     d.cc_minor = prop.minor;
     d.l2_bytes = prop.l2CacheSize;
+    d.mem_bytes = prop.totalGlobalMem;
     d.smem_optin = (int)prop.sharedMemPerBlockOptin;
     void* st = nullptr;
     if (cudaGetSymbolAddress(&st, g_device_status) != cudaSuccess) return nullptr;

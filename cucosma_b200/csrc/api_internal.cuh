@@ -12,6 +12,7 @@ namespace cucosma {
 struct DeviceInfo {
   bool valid = false;
   int sms = 0, cc_major = 0, cc_minor = 0, l2_bytes = 0, smem_optin = 0;
+  size_t mem_bytes = 0;
   int* status = nullptr;  // device address of the status word on this device
 };
 const DeviceInfo* device_info();

@@ -75,7 +75,10 @@ extern "C" cucosma_status cucosma_gemm_backward_workspace_size(const cucosma_gem
   if (!di) return CUCOSMA_STATUS_LAUNCH_FAILED;
   // Each product's plan as the backward call builds it: tuned, and with its
   // planes prepared here (never the fused-split kernel, which keeps none).
-  // The planes of both exist at once, one part after the other.
+  // The planes of both exist at once, one part after the other, unless they
+  // would take more than an eighth of the GPU's memory: gradients that size fit
+  // with the larger product's planes alone, and forming G twice is then less
+  // than a hundredth of the products' time.
   auto need = [&](int64_t m, int64_t n, int64_t k, int64_t ldc) {
     cucosma_gemm_desc d0, tuned;
     cucosma_plan_info pi;
@@ -83,7 +86,8 @@ extern "C" cucosma_status cucosma_gemm_backward_workspace_size(const cucosma_gem
     tc_plan_info(apply_tuning(&d0, &tuned, di), di, &pi, false);
     return part_bytes(pi.workspace_bytes);
   };
-  *bytes = need(f->m, f->k, f->n, f->k) + need(f->k, f->n, f->m, f->n);
+  const size_t da = need(f->m, f->k, f->n, f->k), db = need(f->k, f->n, f->m, f->n);
+  *bytes = da + db <= di->mem_bytes / 8 ? da + db : std::max(da, db);
   return CUCOSMA_STATUS_SUCCESS;
 }
 

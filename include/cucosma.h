@@ -208,8 +208,9 @@ CUCOSMA_API int cucosma_tune_cache_size(void);
  *     dA = G * B^T   (m x k, row stride ldda)      dB = A^T * G   (k x n, lddb)
  * on the tensor cores, with epi' fused into the operand pre-pass; either of
  * dA / dB may be NULL to skip it.  Overwrites dA and dB.  The queried
- * workspace holds the operand planes of both products; with one that holds
- * only the larger product the call runs them one after the other (slower). */
+ * workspace holds the operand planes of both products, or, where those are
+ * more than an eighth of the GPU's memory, of the larger one; with room for
+ * one only the call runs the products one after the other. */
 CUCOSMA_API cucosma_status cucosma_gemm_backward_workspace_size(const cucosma_gemm_desc* fwd, size_t* bytes);
 CUCOSMA_API cucosma_status cucosma_gemm_backward(const cucosma_gemm_desc* fwd, const void* A, const void* B,
                                                  const void* Y, int64_t ldy, const void* dY, int64_t lddy, void* dA,
