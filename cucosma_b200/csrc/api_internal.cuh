@@ -27,7 +27,7 @@ void wait_ctl(const DeviceInfo* di, int** status, unsigned long long* timeout_ns
 enum : int { kPrepA = 1, kPrepB = 2, kNoFused = 4, kAsGiven = 8 };
 
 struct NativePlan {
-  int bm;  // CTA tile rows: 128, or 64 (FP32 only); 128 columns either way
+  int bm;  // CTA tile rows: 128 or 64 (columns: simt::tile_cols())
   int tiles_m, tiles_n, splits, swizzle;
   int cluster;  // 1: the splits are a cluster that reduces through shared memory (no workspace, no second kernel)
   int64_t kchunk, ldw;

@@ -10,7 +10,7 @@
 //   dA: A-planes = rows of G (computed from dY and Y inside the split),
 //       B-planes = rows of B itself (B^T's K-major layout is B);
 //   dB: A-planes = columns of A (A^T, transposing split),
-//       B-planes = columns of G (G^T, transposing split, G computed again).
+//       B-planes = columns of G (G^T, transposing split).
 // Three launches: every plane in one split kernel (G is formed once and
 // written in both layouts), then the two GEMMs, each product with its own
 // part of the caller's workspace.  A workspace that holds only the larger

@@ -8,9 +8,10 @@
 //   BF16x3 / BF16x6: one table-driven split kernel for the A rows and the B
 //                    tiles of every problem + the persistent GEMM kernel;
 //   Ozaki:           exponents, slices (both table-driven) + the GEMM kernel.
-// The GEMM kernel numbers the tiles of all problems consecutively and each
-// CTA walks them round-robin (tc_kernel.cuh, resolve_unit), so small problems
-// no longer leave most of the GPU idle the way one launch per problem does.
+// The tiles of all problems are dealt out to the GEMM's CTAs (or pairs) by the
+// plan's work list (work_list below; tc_kernel.cuh, resolve_unit), so small
+// problems no longer leave most of the GPU idle the way one launch per problem
+// does.
 #include <algorithm>
 #include <cstring>
 #include <new>

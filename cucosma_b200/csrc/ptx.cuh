@@ -189,10 +189,6 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* m, const void* s
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// All but the most recent group have read their shared memory.
-__device__ __forceinline__ void bulk_wait_read_but_last() {
-  asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-}
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // Arrive-with-transaction returning the phase token, and the bounded wait
 // for that phase (no parity bookkeeping for a barrier one thread reuses).

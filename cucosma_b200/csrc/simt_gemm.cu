@@ -9,9 +9,9 @@
 //   * FP32 (simt_sgemm_kernel) transposes each A stage into a k-major buffer,
 //     so a k-step is 4 LDS.128 feeding 32 two-lane FFMA2 (sm_100's packed
 //     FP32 FMA, each lane an fmaf), 8x8 outputs a thread, two CTAs per SM;
-//   * FP64 (simt_dgemm_kernel) runs on FP64 tensor-core MMAs with a 64x32
-//     warp tile;
-//   * 8 warps hold a 128x128 CTA tile;
+//   * FP64 (simt_dgemm_kernel) runs on FP64 tensor-core MMAs, a 64x32 warp
+//     tile in 128x128 CTAs and 32x32 in 64x64 ones;
+//   * a CTA is 8 warps on 128 rows, 4 on 64;
 //   * the K splits of a small launch are a cluster that adds its partial tiles
 //     through distributed shared memory; others write raw partial tiles to a
 //     caller-provided workspace and a separate kernel reduces them.  Both add
@@ -316,8 +316,8 @@ __global__ void __launch_bounds__(simt::SgemmShape<BM_>::kThreads, simt::SgemmSh
 // tile reads half as much a product and lost 0.6 % to the eight boxes).
 // Thread 0 refills a stage two stages after it was consumed, so its wait on
 // the stage's empty barrier rarely blocks.  Bound by the FP64 pipe (37.2
-// TFLOP/s): 35.4 at 4096^3 on 128 x 128; on 64 x 64 31.4 at 2000^3 (30.1 on 128
-// x 128), 1000 x 777 x 1531 101 -> 92 us, 256^3 16.2 -> 8.6.
+// TFLOP/s): 35.4 at 4096^3 on 128 x 128; on 64 x 64 33.6 at 3000^3 (33.0 on 128
+// x 128), 1000 x 777 x 1531 101 -> 90 us, 256^3 16.2 -> 8.6.
 namespace simt {
 template <int EDGE>
 struct DgemmShape {

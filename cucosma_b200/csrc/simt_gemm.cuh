@@ -31,24 +31,21 @@ struct SimtParams {
 };
 
 namespace simt {
-constexpr int BM = 128, BN = 128, STAGES = 4;
-// Eight warps, all computing; thread 0 also issues the TMA loads.  (A ninth,
-// producer-only warp would put three warps in one register-file quadrant
-// and cap every thread at 168 registers, which the FP64 8x8 tile exceeds.)
+constexpr int BM = 128, BN = 128;
+// All warps compute; thread 0 also issues the TMA loads.  (A producer-only warp
+// beside eight would put three warps in one register-file quadrant and cap
+// every thread at 168 registers, which the FP64 128 x 128 tile exceeds.)
 // The splits of a small launch form a cluster that reduces through shared
 // memory: at most kMaxCluster splits (the portable cluster size) and
 // kMaxClusterCtas CTAs in all.  More CTAs than that and the scheduler doubles
 // clusters up on some SMs while others idle (B200: 400^3 FP32, 28 tiles x 5:
 // 12.0 us against 10.6 through the workspace; 1000 x 777 x 1531 FP64, 56 x 5:
-// 154 against 101), while 200 x 136 x 96 FP32 (8 x 6) takes 5.4 us against 9.8
-// unsplit and 100 x 1900 x 150 FP64 (15 x 5) 13.0 against 18.4.
+// 154 against 101), while 200 x 136 x 96 FP32 (8 x 6) takes 4.9 us against 9.3
+// unsplit and 256^3 FP64 on 64 x 64 tiles (16 x 4) 8.6 against 16.2 before them.
 constexpr int kMaxCluster = 8, kMaxClusterCtas = 80;
 constexpr bool cluster_splits(int64_t tiles, int64_t splits) {
   return splits > 1 && splits <= kMaxCluster && tiles * splits <= kMaxClusterCtas;
 }
-constexpr int kComputeWarps = 8;
-constexpr int kThreads = kComputeWarps * 32;
-
 template <typename T>
 struct Cfg;
 template <>

@@ -7,33 +7,8 @@
 namespace cucosma {
 
 // x = t0 + t1 (+ t2) + residual: each term the round-to-nearest-even BF16 of
-// what is left; every subtraction is exact in FP32 (Sterbenz).
-__device__ __forceinline__ void split_bf16_value(float x, int nterms, __nv_bfloat16 (&t)[3]) {
-  float r = x;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    if (i < nterms) {
-      t[i] = __float2bfloat16_rn(r);
-      r = r - __bfloat162float(t[i]);
-    }
-  }
-}
-
-// The same with the term count known at compile time (no local memory).
-template <int NT>
-__device__ __forceinline__ void split_bf16_n(float x, __nv_bfloat16 (&t)[NT]) {
-  float r = x;
-#pragma unroll
-  for (int i = 0; i < NT; ++i) {
-    t[i] = __float2bfloat16_rn(r);
-    r = r - __bfloat162float(t[i]);
-  }
-}
-
-// Two values at once: w[i] holds term i of x0 in its low half and of x1 in
-// its high half (cvt.rn.bf16x2.f32 rounds each to nearest even, as
-// __float2bfloat16_rn does), so the words equal pack_bf16x2 of
-// split_bf16_n's terms bit for bit.
+// what is left; every subtraction is exact in FP32 (Sterbenz).  Two values at
+// once: w[i] holds term i of x0 in its low half and of x1 in its high half.
 template <int NT>
 __device__ __forceinline__ void split_bf16x2_n(float x0, float x1, uint32_t (&w)[NT]) {
   float r0 = x0, r1 = x1;
@@ -45,11 +20,6 @@ __device__ __forceinline__ void split_bf16x2_n(float x0, float x1, uint32_t (&w)
       r1 = r1 - __uint_as_float(w[i] & 0xffff0000u);
     }
   }
-}
-
-__device__ __forceinline__ uint32_t pack_bf16x2(__nv_bfloat16 lo, __nv_bfloat16 hi) {
-  __nv_bfloat162 v = __halves2bfloat162(lo, hi);
-  return *reinterpret_cast<uint32_t*>(&v);
 }
 
 // frexp-style exponent of the largest magnitude: |x| < 2^e for all x.

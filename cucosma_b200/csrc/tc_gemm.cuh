@@ -107,7 +107,6 @@ struct OutCtx {
   WaitCtl ctl;
 };
 
-// A resolved work unit: operand descriptors, tile coordinates, K range.
 // Operands of tail_reduce_kernel: tiles tile0 .. tile0 + count - 1 of the raster.
 struct TailReduce {
   const float* ws;
@@ -118,6 +117,7 @@ struct TailReduce {
   int epilogue;
 };
 
+// A resolved work unit: operand descriptors, tile coordinates, K range.
 struct Unit {
   const CUtensorMap* ta;
   const CUtensorMap* tb;

@@ -82,13 +82,16 @@ typedef struct cucosma_gemm_desc {
                            * NATIVE 1 = always the 128 x 128 tile kernel (no skinny-shape kernels),
                            *        2 = the 64 x 128 tile kernel (FP32; FP64 runs 128 x 128);
                            * BF16X3 1 = 128 x 256 without promotion, 2 = 128 x 128 promoted,
-                           *        3 = 128 x 256 promoted, 4 = 256 x 256 CTA pair (default when m > 128),
+                           *        3 = 128 x 256 promoted, 4 = 256 x 256 CTA pair,
                            *        5 = 256 x 128 pair with the split fused in;
                            * BF16X6 1 = 128 x 128, 2 = 256 x 128 CTA pair,
-                           *        3 = 256 x 256 CTA pair (default when m > 128),
+                           *        3 = 256 x 256 CTA pair,
                            *        4 = 256 x 128 pair with the split fused in.
-                           * Auto (0) picks the fused kernels where the separate split pass
-                           * would cost more than a quarter of the GEMM (large K, large N) */
+                           * 0: BF16 operands that fit L2 take the tile and K split of the
+                           * smallest modelled time; larger ones the 256 x 256 pair (m > 128), or
+                           * the fused one where the separate split pass would cost more than a
+                           * quarter of the GEMM (large K, large N).  NATIVE takes skinny-shape
+                           * kernels, else 128- or 64-row tiles (FP64: 128 x 128 or 64 x 64) */
   int32_t flags;          /* 0, or CUCOSMA_FLAG_TEST_SKIP_STAGE */
 } cucosma_gemm_desc;
 
