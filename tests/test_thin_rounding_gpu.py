@@ -1,7 +1,7 @@
 """The thin kernel's rounding errors: no larger than those of the form with
 four CTAs an SM and four (FP64: two) consecutive k a lane, whose rms errors on
 the same kind of operands, relative to the rms of the result, are given here
-(errors pooled over seeds, 10^4 or more, so that they are known to 1 %)."""
+(errors pooled over seeds, a thousand or more, known to 3 %)."""
 import pytest
 
 import cucosma_b200 as cc
@@ -14,7 +14,8 @@ CASES = [((5, 30000, 100), "float32", 7.17e-8, 1), ((5, 30000, 100), "float64", 
          ((4, 8, 3000), "float32", 1.05e-7, 200), ((4, 8, 3000), "float64", 1.70e-16, 200),
          ((1, 4096, 4096), "float32", 1.03e-7, 3), ((1, 4096, 4096), "float64", 1.65e-16, 3),
          ((64, 5, 5000), "float32", 1.16e-7, 40), ((8, 8, 40000), "float32", 1.10e-7, 150),
-         ((12, 7, 1435677), "float64", 2.47e-16, 20)]
+         ((12, 7, 1435677), "float64", 2.47e-16, 20), ((8, 16, 3000000), "float32", 1.67e-7, 20),
+         ((8, 16, 3000000), "float64", 2.79e-16, 20), ((1, 16, 1570806), "float32", 1.39e-7, 40)]
 
 
 @pytest.mark.parametrize("shape,dtype,limit,seeds", CASES, ids=["%dx%dx%d-%s" % (c[0] + (c[1],)) for c in CASES])
@@ -51,4 +52,4 @@ def test_thin_rounding(cuda, shape, dtype, limit, seeds):
         ref2 += float(ref.pow(2).sum())
     samples = seeds * m * n
     # the limit's own sampling error and this sample's, three deviations of each
-    assert (err2 / ref2) ** 0.5 <= limit * (1 + 0.01 + 3 / (2 * samples) ** 0.5)
+    assert (err2 / ref2) ** 0.5 <= limit * (1 + 0.03 + 3 / (2 * samples) ** 0.5)
