@@ -163,11 +163,11 @@ __global__ void __launch_bounds__(256, SmallK<T, RPT>::kCtas)
 }
 
 // The last steps of thin_kernel's reduction and the sum over its splits, where
-// the sums are largest, round once: FP32 sums are added in 64 bits, FP64 ones with the rounding error of
-// each addition carried along (D. E. Knuth, TAOCP 2, 4.2.2, theorem B).  The rms
-// error is 0.5 to 0.9 of that of four CTAs an SM with four (FP64: two)
-// consecutive k a lane, which this kernel replaced; 0.9 to 1.6 without.  2 % of
-// the time over 110 shapes on B200.
+// the sums are largest, round once: FP32 sums are added in 64 bits, FP64 ones
+// with the rounding error of each addition carried along (D. E. Knuth, TAOCP 2,
+// 4.2.2, theorem B).  The rms error is 0.5 to 0.9 of that of four CTAs an SM
+// with four (FP64: two) consecutive k a lane, which this kernel replaced; 0.9
+// to 1.6 without.  2 % of the time over 110 shapes on B200.
 struct SumF64 {
   double hi, lo;
 };

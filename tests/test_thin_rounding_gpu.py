@@ -53,3 +53,25 @@ def test_thin_rounding(cuda, shape, dtype, limit, seeds):
     samples = seeds * m * n
     # the limit's own sampling error and this sample's, three deviations of each
     assert (err2 / ref2) ** 0.5 <= limit * (1 + 0.03 + 3 / (2 * samples) ** 0.5)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("k", [100, 70001])
+def test_infinities_and_nan(cuda, dtype, k):
+    """Infinite and NaN products reach their outputs, and no others, through every step of the reduction."""
+    import torch
+
+    dt = getattr(torch, dtype)
+    m, n = 6, 8
+    A = torch.zeros((m, -(-k // 4) * 4), dtype=dt, device="cuda")[:, :k]
+    B = torch.ones((k, n), dtype=dt, device="cuda")
+    A.fill_(0.5)
+    inf = float("inf")
+    A[1, 0], A[2, k - 1], A[3, 17], A[4, 33], A[4, k - 2] = inf, -inf, float("nan"), inf, -inf
+    A[5, 64] = torch.finfo(dt).max
+    C = torch.zeros((m, n), dtype=dt, device="cuda")
+    cc.cosma_sgemm(A, B, C, 1.0, 0.0)
+    want = torch.tensor([0.5 * k, inf, -inf, float("nan"), float("nan"), torch.finfo(dt).max], dtype=dt, device="cuda")
+    assert torch.equal(C.isnan(), want.isnan()[:, None].expand(m, n))
+    ok = [0, 1, 2, 5]
+    assert torch.equal(C[ok], want[ok, None].expand(len(ok), n))
