@@ -199,7 +199,8 @@ __device__ __forceinline__ bool inplace_convert_b1(uint8_t* stage, int c, Sync&&
 // of promoting it into registers: one rolled copy of the epilogue's code (the
 // unrolled one missed in the instruction cache, the roles of this kernel
 // evicting one another: 3.2 stalled warps an issue on the sigmoid form).
-template <class Tr, int STG, bool DIRECT>
+// ROWS_C (with STG = 1): unsplit, C read and N no multiple of 4 (EpiF32::update_block).
+template <class Tr, int STG, bool DIRECT, bool ROWS_C>
 __global__ void __maxnreg__((FusedInplaceCfg<Tr, STG>::MAX_REGS))
     tc_fused_inplace_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                             const __grid_constant__ TcParams p) {
@@ -400,7 +401,7 @@ __global__ void __maxnreg__((FusedInplaceCfg<Tr, STG>::MAX_REGS))
         if (ok) {
           prefetch_unit(unit + unit_step);
           const OutCtx o = octx();
-          Tr::template finish<STG>(o, master, stg, lane, row0, col0 + colsub, u.z, loaded, cph);
+          Tr::template finish<STG, ROWS_C>(o, master, stg, lane, row0, col0 + colsub, u.z, loaded, cph);
         }
       }
       if (!ok) {
@@ -495,13 +496,13 @@ static cudaError_t launch_fused_kernel(K kernel, int threads, int smem, std::ato
 
 // BF16x3: a = A [128 rows][64 K] boxes, b = B [64 K][64 columns] boxes (no swizzle);
 // BF16x6: a = A [128 rows][32 K] boxes (128-byte swizzle), b = B [32 K][64 columns].
-template <class Tr, int STG, bool DIRECT = false>
+template <class Tr, int STG, bool DIRECT = false, bool ROWS_C = false>
 static cudaError_t launch_fused_inplace(const CUtensorMap& a, const CUtensorMap& b, const TcParams& p, int sms,
                                         cudaStream_t st) {
   using F = FusedInplaceCfg<Tr, STG>;
   static std::atomic<uint64_t> attr_set{0};
   static std::atomic<int> clusters_cached[64];
-  return launch_fused_kernel(tc_fused_inplace_kernel<Tr, STG, DIRECT>, F::THREADS, F::SMEM, attr_set, clusters_cached, a, b, p,
+  return launch_fused_kernel(tc_fused_inplace_kernel<Tr, STG, DIRECT, ROWS_C>, F::THREADS, F::SMEM, attr_set, clusters_cached, a, b, p,
                              sms, st);
 }
 

@@ -749,6 +749,28 @@ struct EpiF32 {
     __syncwarp();
   }
 
+  // One block whose C comes and goes by rows, with one staging block: C first,
+  // all rows in flight, the accumulators combined with it in place.  (A kernel
+  // instance of its own: beside the box path in one instance it took registers
+  // from both, 512 x 8192 x 4096 BF16x3 161 -> 167 us.)
+  static __device__ __noinline__ void rows_in(const float* w, int64_t ldo, float* stg, int lane, int rows) {
+#pragma unroll 4
+    for (int r = 0; r < rows; ++r) cp_async4(&stg[sw(r, lane)], w + (int64_t)r * ldo);
+    cp_async_wait_all();
+  }
+  static __device__ __forceinline__ void update_block(const OutCtx& p, float* o, const float (&acc)[32], float* stg,
+                                                      int lane, int row0, int col) {
+    if (col >= p.n) return;  // the whole block lies right of C (col is the block's first column)
+    float* w = o + (int64_t)row0 * p.ldo + col + lane;  // this lane's column
+    const int rows = col + lane < p.n ? min(32, p.m - row0) : 0;
+    rows_in(w, p.ldo, stg, lane, rows);
+    __syncwarp();
+    combine_row(p.epilogue, reinterpret_cast<float4*>(stg) + lane * 8, acc, (float)p.alpha, (float)p.beta, lane);
+    __syncwarp();
+    rows_out<1>(w, p.ldo, stg, lane, rows, -1, 0.f, 0.f);
+    __syncwarp();
+  }
+
   // 64-column blocks through the 3-D map: one 8 KB staging block [32 rows]
   // [2 chunks][32] (line 2r + h of row r, chunk h, 128-byte swizzle per line),
   // one box load of C (beta != 0) and one box store, 256-byte row requests
@@ -913,8 +935,9 @@ struct EpiF32 {
   // the matching paths exist.  With two, 64-column blocks go through the 3-D
   // map; the first block's C load was started by load_c64 before the last
   // accumulator chunk was waited for (loaded; parity: its barrier phase, left
-  // at the phase the next load will complete).
-  template <int BN, int STG>
+  // at the phase the next load will complete).  ROWS_C (with one block): C is
+  // read (beta != 0) and moves by rows.
+  template <int BN, int STG, bool ROWS_C>
   static __device__ __forceinline__ void finish(const OutCtx& p, const float (&master)[BN], uint8_t* stg_raw,
                                                 int lane, int row0, int col0, int z, bool loaded, uint32_t& parity) {
     float* stg = reinterpret_cast<float*>(stg_raw);
@@ -967,7 +990,9 @@ struct EpiF32 {
     }
 #pragma unroll
     for (int c0 = 0; c0 < BN; c0 += 32) {
-      if (p.tmc != nullptr)
+      if constexpr (ROWS_C)
+        update_block(p, o, cols32(master, c0), stg, lane, row0, col0 + c0);
+      else if (p.tmc != nullptr)
         store_block_tma(p, cols32(master, c0), stg, lane, row0, col0 + c0);
       else
         store_block<1>(p, o, cols32(master, c0), stg, lane, row0, col0 + c0);
@@ -1200,10 +1225,10 @@ struct TraitsBase {
   static __device__ __forceinline__ void accumulate_one(uint32_t tacc, int d, float (&master)[COLS_PER_EW]) {
     if constexpr (PROMOTE) Epi::template accumulate<COLS_PER_EW, BN, 1>(tacc + (uint32_t)(d * BN), master);
   }
-  template <int STG = STAGING_PER_WARP / 4096>
+  template <int STG = STAGING_PER_WARP / 4096, bool ROWS_C = false>
   static __device__ __forceinline__ void finish(const OutCtx& p, const float (&master)[COLS_PER_EW], uint8_t* stg,
                                                 int lane, int row0, int col0, int z, bool loaded, uint32_t& parity) {
-    if constexpr (PROMOTE) Epi::template finish<COLS_PER_EW, STG>(p, master, stg, lane, row0, col0, z, loaded, parity);
+    if constexpr (PROMOTE) Epi::template finish<COLS_PER_EW, STG, ROWS_C>(p, master, stg, lane, row0, col0, z, loaded, parity);
   }
   template <class Release>
   static __device__ __forceinline__ void direct(const OutCtx& p, uint32_t tacc, uint8_t* stg, int lane, int row0,
