@@ -542,30 +542,31 @@ __global__ void splitk_reduce_kernel(const T* __restrict__ ws, int64_t split_str
     const int c = (int)(idx - r * nv) * VEC;
     const T* w = ws + r * ldw + c;
     T* o = C + r * ldc + c;
-    if (c + VEC <= n) {
-      V s = *reinterpret_cast<const V*>(w);
-      T* ps = reinterpret_cast<T*>(&s);
-      // Splits are added in ascending order; the loads of a batch of 8 are
-      // issued before its adds so that many splits do not serialise on load
-      // latency.
-      int z = 1;
-      for (; z + 8 <= splits; z += 8) {
-        V t[8];
+    // (planes are padded to whole vectors: elements past n are read, never used)
+    V s = *reinterpret_cast<const V*>(w);
+    T* ps = reinterpret_cast<T*>(&s);
+    // Splits are added in ascending order; the loads of a batch of 8 are
+    // issued before its adds so that many splits do not serialise on load
+    // latency.
+    int z = 1;
+    for (; z + 8 <= splits; z += 8) {
+      V t[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) t[j] = *reinterpret_cast<const V*>(w + (int64_t)(z + j) * split_stride);
+      for (int j = 0; j < 8; ++j) t[j] = *reinterpret_cast<const V*>(w + (int64_t)(z + j) * split_stride);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const T* pt = reinterpret_cast<const T*>(&t[j]);
-#pragma unroll
-          for (int e = 0; e < VEC; ++e) ps[e] += pt[e];
-        }
-      }
-      for (; z < splits; ++z) {
-        const V t = *reinterpret_cast<const V*>(w + (int64_t)z * split_stride);
-        const T* pt = reinterpret_cast<const T*>(&t);
+      for (int j = 0; j < 8; ++j) {
+        const T* pt = reinterpret_cast<const T*>(&t[j]);
 #pragma unroll
         for (int e = 0; e < VEC; ++e) ps[e] += pt[e];
       }
+    }
+    for (; z < splits; ++z) {
+      const V t = *reinterpret_cast<const V*>(w + (int64_t)z * split_stride);
+      const T* pt = reinterpret_cast<const T*>(&t);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) ps[e] += pt[e];
+    }
+    if (c + VEC <= n) {
       V cv;
       if (beta != T(0)) cv = *reinterpret_cast<const V*>(o);
       const T* pc = reinterpret_cast<const T*>(&cv);
@@ -573,11 +574,9 @@ __global__ void splitk_reduce_kernel(const T* __restrict__ ws, int64_t split_str
       for (int e = 0; e < VEC; ++e) ps[e] = apply_epi(combine(ps[e], alpha, beta, pc + e), epi);
       *reinterpret_cast<V*>(o) = s;
     } else {
-      for (int e = 0; c + e < n; ++e) {
-        T s = w[e];
-        for (int z = 1; z < splits; ++z) s += w[z * split_stride + e];
-        o[e] = apply_epi(combine(s, alpha, beta, o + e), epi);
-      }
+#pragma unroll
+      for (int e = 0; e < VEC; ++e)
+        if (c + e < n) o[e] = apply_epi(combine(ps[e], alpha, beta, o + e), epi);
     }
   }
 }
