@@ -27,16 +27,10 @@
 
 namespace cucosma {
 
-// Of a form with RPT rows a thread: resident CTAs an SM, and rows of B whose
-// loads are in flight when it comes straight from global memory.
-template <typename T, int RPT>
-struct SmallK {
-  static constexpr bool kF32 = sizeof(T) == 4;
-  static constexpr int kCtas = RPT <= 4 ? 4 : RPT > 8 ? 2 : kF32 ? 4 : 3;
-  static constexpr int kRowsB = RPT <= 4 ? 4 : kF32 ? 2 : 3;
-};
-template <typename T, int RG, int RPT>
-__global__ void __launch_bounds__(256, SmallK<T, RPT>::kCtas)
+// CTAS: resident CTAs an SM.  ROWS_B: rows of B whose loads are in flight when it
+// comes straight from global memory.
+template <typename T, int RG, int RPT, int CTAS, int ROWS_B>
+__global__ void __launch_bounds__(256, CTAS)
     smallk_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ B, int64_t ldb, T* C, int64_t ldc,
                   int m, int n, int k, T alpha, T beta, int epi, int tiles_n, int64_t tiles) {
   // RG row groups of RPT rows x (256 / RG) column groups of VEC columns.  With
@@ -93,7 +87,7 @@ __global__ void __launch_bounds__(256, SmallK<T, RPT>::kCtas)
           cold[r] = *reinterpret_cast<const V*>(C + (int64_t)(m0 + rg * RPT + r) * ldc + col);
     }
     // B straight from global memory: KU rows' loads in flight at a time
-    constexpr int KU = SHARE_B ? 1 : SmallK<T, RPT>::kRowsB;
+    constexpr int KU = SHARE_B ? 1 : ROWS_B;
     for (int k0 = 0; k0 < k; k0 += KU) {
       V bv[KU];
 #pragma unroll
@@ -345,15 +339,16 @@ SkinnyPlan plan_skinny(int64_t m, int64_t n, int64_t k, int dtype_bytes, int spl
     p.kind = 1;
     p.splits = 1;
     // 4 x (256 vec) blocks when M <= 4, 8 x (128 vec) when M <= 8, else 64 x
-    // (64 vec).  The second in two groups of four rows, which both read B: that
-    // shows once C fills more than one wave of them and (FP32, whose wide form
-    // has no registers left for C ahead of its use) C is only written; then 8
-    // rows a thread (B200, beta 0: 5 x 361,026 x 2 FP32 5.7 us in groups, 4.9
-    // so; 5 x 361,026 x 13 FP64 12.8 and 10.2; 8 x 2,500,000 x 13 FP32 51.6 and
-    // 48.7.  FP32, beta 0.5, 8 x 1,000,000 x 16: 23.7 in groups).
+    // (64 vec).  The second in two groups of four rows, which both read B and
+    // are twice as many: once they exceed a wave, 8 rows a thread in blocks of
+    // twice the columns (B200, beta 0: 5 x 361,026 x 2 FP32 5.7 us in groups,
+    // 4.9 so; 5 x 361,026 x 13 FP64 12.8 and 10.2; 8 x 2,500,000 x 13 FP32 51.6
+    // and 48.7).  FP32 that reads C has no registers left to load it ahead in
+    // that form, so it takes it only while it saves a wave (5 x 600,000 x 13,
+    // beta 0.5, 11.5 us in groups, 8 x 1,000,000 x 16 23.7 in groups and 27).
     p.tile_m = m <= skinny::kThin ? skinny::kThin : 64;
     const bool whole = m > 4 && m <= skinny::kThin && ceil_div(n, 128 * vec) > 4 * (int64_t)sms &&
-                       (dtype_bytes == 8 || beta == 0.0);
+                       (dtype_bytes == 8 || beta == 0.0 || ceil_div(n, 256 * vec) <= 4 * (int64_t)sms);
     p.tile_n = m <= 4 || whole ? 256 * vec : m <= skinny::kThin ? 128 * vec : 64 * vec;
     return p;
   }
@@ -386,18 +381,19 @@ cudaError_t launch_skinny(const SkinnyPlan& pl, const T* A, int64_t lda, const T
     const int tiles_n = (int)ceil_div(n, pl.tile_n);
     const int64_t tiles = ceil_div(m, pl.tile_m) * (int64_t)tiles_n;
     const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)sms * 8));
-    if (pl.tile_m == skinny::kThin && m <= 4)  // M <= 8: one row group, B straight from global memory
-      smallk_kernel<T, 1, 4><<<(unsigned)grid, 256, 0, st>>>(A, lda, B, ldb, C, ldc, m, n, k, (T)alpha, (T)beta, epi,
-                                                             tiles_n, tiles);
-    else if (pl.tile_m == skinny::kThin && pl.tile_n == 256 * Vec<T>::n)
-      smallk_kernel<T, 1, 8><<<(unsigned)grid, 256, 0, st>>>(A, lda, B, ldb, C, ldc, m, n, k, (T)alpha, (T)beta, epi,
-                                                             tiles_n, tiles);
-    else if (pl.tile_m == skinny::kThin)
-      smallk_kernel<T, 2, 4><<<(unsigned)grid, 256, 0, st>>>(A, lda, B, ldb, C, ldc, m, n, k, (T)alpha, (T)beta, epi,
-                                                             tiles_n, tiles);
-    else
-      smallk_kernel<T, 4, 16><<<(unsigned)grid, 256, 0, st>>>(A, lda, B, ldb, C, ldc, m, n, k, (T)alpha, (T)beta, epi,
-                                                              tiles_n, tiles);
+    // 8 rows a thread: three rows of B in flight leave registers for three CTAs
+    // an SM.  FP32 blocks that fit at once only as four, and those of several
+    // waves, take four CTAs and one or two rows (5 x 600,000 x 13, beta 0.5, 9.7
+    // us with one, 11.0 with two, 12.1 as three CTAs).
+    constexpr bool kF32 = sizeof(T) == 4;
+    const int64_t per_sm = ceil_div(tiles, (int64_t)sms);
+    auto* kernel = pl.tile_m != skinny::kThin     ? smallk_kernel<T, 4, 16, 2, 1>
+                   : m <= 4                       ? smallk_kernel<T, 1, 4, 4, 4>
+                   : pl.tile_n == 128 * Vec<T>::n ? smallk_kernel<T, 2, 4, 4, 4>
+                   : !kF32 || per_sm <= 3         ? smallk_kernel<T, 1, 8, 3, 3>
+                   : per_sm <= 4                  ? smallk_kernel<T, 1, 8, kF32 ? 4 : 3, kF32 ? 1 : 3>
+                                                  : smallk_kernel<T, 1, 8, kF32 ? 4 : 3, kF32 ? 2 : 3>;
+    kernel<<<(unsigned)grid, 256, 0, st>>>(A, lda, B, ldb, C, ldc, m, n, k, (T)alpha, (T)beta, epi, tiles_n, tiles);
     return cudaGetLastError();
   }
   const int groups_n = (int)ceil_div(n, skinny::kThin);
