@@ -24,6 +24,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <new>
 #include <tuple>
 #include <vector>
 
@@ -300,9 +301,8 @@ extern "C" cucosma_status cucosma_tune(const cucosma_gemm_desc* d, const void* A
   return CUCOSMA_STATUS_SUCCESS;
 }
 
-extern "C" cucosma_status cucosma_tune_grouped(const cucosma_gemm_desc* d, const cucosma_gemm_problem* problems,
-                                               int count, void* workspace, size_t workspace_bytes,
-                                               cucosma_tune_result* out, void* stream) {
+static cucosma_status tune_grouped(const cucosma_gemm_desc* d, const cucosma_gemm_problem* problems, int count,
+                                   void* workspace, size_t workspace_bytes, cucosma_tune_result* out, void* stream) {
   if (!d || !problems || count <= 0) return CUCOSMA_STATUS_INVALID_VALUE;
   const DeviceInfo* di = device_info();
   if (!di) return CUCOSMA_STATUS_LAUNCH_FAILED;
@@ -385,6 +385,17 @@ extern "C" cucosma_status cucosma_tune_grouped(const cucosma_gemm_desc* d, const
     out->counter_passes = cr.passes;
   }
   return CUCOSMA_STATUS_SUCCESS;
+}
+
+// (as the planner: a batch whose tables host memory does not hold is an error, not an exception)
+extern "C" cucosma_status cucosma_tune_grouped(const cucosma_gemm_desc* d, const cucosma_gemm_problem* problems,
+                                               int count, void* workspace, size_t workspace_bytes,
+                                               cucosma_tune_result* out, void* stream) {
+  try {
+    return tune_grouped(d, problems, count, workspace, workspace_bytes, out, stream);
+  } catch (const std::bad_alloc&) {
+    return CUCOSMA_STATUS_ALLOC_FAILED;
+  }
 }
 
 extern "C" cucosma_status cucosma_tune_cache_save(const char* path) {
