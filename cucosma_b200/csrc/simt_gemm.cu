@@ -524,9 +524,66 @@ __global__ void __launch_bounds__(simt::DgemmShape<EDGE>::kThreads, simt::DgemmS
                    acc[mt][nt][2 * h + 1]);
 }
 
+// Sum of the planes' vectors at w.  Splits are added in ascending order; the
+// loads of a batch of 8 are issued before its adds so that many splits do not
+// serialise on load latency.  With more splits than kShortSum the next batch's
+// loads are in flight while one is added (LONG): a small C in hundreds of
+// splits is bound by that latency alone (10 x 96 x 194295 FP32, 288 splits,
+// 100 -> 89 us; 64 x 50 x 22358 FP64, 280 splits, 46 -> 28).  It doubles the
+// registers.  Up to kShortSum splits there is no second batch to load, and the
+// reductions that start beside their GEMM (8 splits and fewer) would only take
+// its room: 512^3 FP64 18.7 -> 21.5.
+constexpr int kShortSum = 16;
+template <typename T, bool LONG>
+__device__ __forceinline__ typename Vec<T>::type sum_planes(const T* __restrict__ w, int64_t split_stride, int splits) {
+  constexpr int VEC = Vec<T>::n;
+  using V = typename Vec<T>::type;
+  V s = *reinterpret_cast<const V*>(w);
+  T* ps = reinterpret_cast<T*>(&s);
+  auto load = [&](V (&t)[8], int z) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) t[j] = *reinterpret_cast<const V*>(w + (int64_t)(z + j) * split_stride);
+  };
+  auto add = [&](const V (&t)[8]) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const T* pt = reinterpret_cast<const T*>(&t[j]);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) ps[e] += pt[e];
+    }
+  };
+  int z = 1;
+  if constexpr (LONG) {  // splits > kShortSum
+    V t[8];
+    load(t, z);
+    for (; z + 16 <= splits; z += 8) {
+      V next[8];
+      load(next, z + 8);
+      add(t);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) t[j] = next[j];
+    }
+    add(t);
+    z += 8;
+  } else {
+    for (; z + 8 <= splits; z += 8) {
+      V t[8];
+      load(t, z);
+      add(t);
+    }
+  }
+  for (; z < splits; ++z) {
+    const V u = *reinterpret_cast<const V*>(w + (int64_t)z * split_stride);
+    const T* pu = reinterpret_cast<const T*>(&u);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) ps[e] += pu[e];
+  }
+  return s;
+}
+
 // Deterministic split-K reduction: C = epi(alpha * sum_z ws[z] + beta*C),
 // z ascending, the sum accumulated in T (cosmaSplitKReduce.cuh:31-40).
-template <typename T>
+template <typename T, bool LONG>
 __global__ void splitk_reduce_kernel(const T* __restrict__ ws, int64_t split_stride, int64_t ldw, int splits, T* C,
                                      int64_t ldc, int m, int n, double alpha_d, double beta_d, int epi,
                                      const int* gate, int gate_value) {
@@ -542,31 +599,9 @@ __global__ void splitk_reduce_kernel(const T* __restrict__ ws, int64_t split_str
     const int c = (int)(idx - r * nv) * VEC;
     const T* w = ws + r * ldw + c;
     T* o = C + r * ldc + c;
-    // (planes are padded to whole vectors: elements past n are read, never used)
-    V s = *reinterpret_cast<const V*>(w);
-    T* ps = reinterpret_cast<T*>(&s);
-    // Splits are added in ascending order; the loads of a batch of 8 are
-    // issued before its adds so that many splits do not serialise on load
-    // latency.
-    int z = 1;
-    for (; z + 8 <= splits; z += 8) {
-      V t[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) t[j] = *reinterpret_cast<const V*>(w + (int64_t)(z + j) * split_stride);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const T* pt = reinterpret_cast<const T*>(&t[j]);
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) ps[e] += pt[e];
-      }
-    }
-    for (; z < splits; ++z) {
-      const V t = *reinterpret_cast<const V*>(w + (int64_t)z * split_stride);
-      const T* pt = reinterpret_cast<const T*>(&t);
-#pragma unroll
-      for (int e = 0; e < VEC; ++e) ps[e] += pt[e];
-    }
     if (c + VEC <= n) {
+      V s = sum_planes<T, LONG>(w, split_stride, splits);
+      T* ps = reinterpret_cast<T*>(&s);
       V cv;
       if (beta != T(0)) cv = *reinterpret_cast<const V*>(o);
       const T* pc = reinterpret_cast<const T*>(&cv);
@@ -574,6 +609,9 @@ __global__ void splitk_reduce_kernel(const T* __restrict__ ws, int64_t split_str
       for (int e = 0; e < VEC; ++e) ps[e] = apply_epi(combine(ps[e], alpha, beta, pc + e), epi);
       *reinterpret_cast<V*>(o) = s;
     } else {
+      // (planes are padded to whole vectors: elements past n are read, never used)
+      V s = sum_planes<T, LONG>(w, split_stride, splits);
+      const T* ps = reinterpret_cast<const T*>(&s);
 #pragma unroll
       for (int e = 0; e < VEC; ++e)
         if (c + e < n) o[e] = apply_epi(combine(ps[e], alpha, beta, o + e), epi);
@@ -672,8 +710,9 @@ cudaError_t launch_reduce(const T* ws, int64_t split_stride, int64_t ldw, int sp
   int64_t blocks = ceil_div(work, threads);
   blocks = std::min<int64_t>(blocks, (int64_t)num_sms * 8);
   if (blocks < 1) blocks = 1;
-  return launch_after(splits <= 8, splitk_reduce_kernel<T>, dim3((unsigned)blocks), threads, 0, stream, ws, split_stride, ldw,
-                      splits, C, ldc, m, n, alpha, beta, epi, gate, gate_value);
+  return launch_after(splits <= 8, splits > kShortSum ? splitk_reduce_kernel<T, true> : splitk_reduce_kernel<T, false>,
+                      dim3((unsigned)blocks), threads, 0, stream, ws, split_stride, ldw, splits, C, ldc, m, n, alpha, beta,
+                      epi, gate, gate_value);
 }
 
 template <typename T>
