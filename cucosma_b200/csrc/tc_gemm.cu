@@ -397,6 +397,18 @@ static Plan make_plan(const cucosma_gemm_desc* d, const DeviceInfo* di, bool all
 // TMEM directly.
 static bool one_chunk(const Tiling& t) { return t.splits == 1 && t.kblocks <= kPromoteChunk; }
 
+// BF16x6 128 x 128 tiles: eight epilogue warps, or four and a deeper ring with
+// the same sums.  Four where the MMAs wait for operands that come from HBM, as
+// they and their planes (10 bytes an element) exceed L2, and units are long
+// enough for that to outweigh their epilogue.  B200, eight / four: 26 x 6656 x
+// 23052 510 / 492 us, 128 x 18944 x 1024 70.8 / 68.4, 128 x 60000 x 256 64.7 /
+// 61.3; but from L2 512 x 512 x 4096 29.2 / 31.2, 128 x 6656 x 1024 30.0 / 31.9,
+// and 4 k-blocks a unit, beta 0.5, 128 x 100000 x 128 60.0 / 68.0.
+static bool deep_ring(const cucosma_gemm_desc* d, const Tiling& t, const DeviceInfo* di) {
+  const double elems = (double)d->m * (double)d->k + (double)d->k * (double)d->n;
+  return elems * 10.0 > (double)di->l2_bytes && t.kb_per_split >= 8;
+}
+
 static int plan_launches(const Plan& pl) {
   if (pl.fused) return 1 + (pl.t.splits > 1 ? 1 : 0);
   if (pl.kind != 2) return 2 + (pl.t.splits > 1 || pl.t.tail_splits > 1 ? 1 : 0);  // the split of A and B, the GEMM
@@ -626,7 +638,9 @@ cucosma_status tc_gemm_ex(const cucosma_gemm_desc* d, const void* A, const void*
     auto pair_grid = [&](int clusters) { return 2 * std::max(1, std::min(units, clusters)); };
     prof_begin(st);
     switch (pl.variant) {
-      case kV6Single: e = launch<Bf16x6>(ta, tb, p, grid, st); break;
+      case kV6Single:
+        e = deep_ring(d, pl.t, di) ? launch<Bf16x6Deep>(ta, tb, p, grid, st) : launch<Bf16x6>(ta, tb, p, grid, st);
+        break;
       case kV6Pair: e = launch<Bf16x6Pair>(ta, tb, p, pair_grid(max_pair_clusters<Bf16x6Pair>(di->sms)), st); break;
       case kV6PairWide:
         if (pl.t.tail_splits > 1)

@@ -1279,6 +1279,11 @@ struct Bf16x6 : TraitsBase<6, 128, 64, 3, 3, 2, false, EpiF32, true, kPromoteChu
   static constexpr TermTable<6> kTerms{
       {2, 1, 1, 0, 0, 0}, {0, 1, 0, 2, 1, 0}, {1, 1, 1, 1, 1, 0}, {true, false, false, false, false, true}};
 };
+// Bf16x6 with four epilogue warps: half the staging, so four 48 KB ring stages
+// instead of three, which hide more of the operands' latency.
+struct Bf16x6Deep : TraitsBase<6, 128, 64, 3, 3, 2, false, EpiF32, true, kPromoteChunk, 4> {
+  static constexpr TermTable<6> kTerms = Bf16x6::kTerms;
+};
 
 // CTA-pair tiles (256 rows): half the shared-memory operand reads and L2
 // traffic per output of the 128-row tiles at the same MMA N.
