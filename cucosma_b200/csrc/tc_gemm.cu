@@ -122,7 +122,7 @@ static Tiling make_tiling(const Plan& pl, int slices, int bn, const cucosma_gemm
   t.tiles_m = (int)ceil_div(M, pl.tile_m);
   t.tiles_n = (int)ceil_div(N, bn);
   t.kblocks = (int)ceil_div(K, pl.bk);
-  const int64_t tiles = (int64_t)t.tiles_m * t.tiles_n;
+  const int64_t tiles = std::max<int64_t>(1, (int64_t)t.tiles_m * t.tiles_n);  // (plans of empty problems are queried)
   // Work slots: one per SM, or one per SM pair for pair tiles.
   const int slots = pl.pair ? di->sms / 2 : di->sms;
   int64_t min_splits = 1, kbmax = INT32_MAX;
@@ -142,9 +142,10 @@ static Tiling make_tiling(const Plan& pl, int slices, int bn, const cucosma_gemm
     const int64_t waves = ceil_div(tiles * splits, (int64_t)slots);
     splits = std::max(splits, waves * slots / tiles);
   }
-  splits = std::min<int64_t>(splits, t.kblocks);
-  t.kb_per_split = (int)std::min<int64_t>(ceil_div(t.kblocks, splits), kbmax);
-  t.splits = (int)ceil_div(t.kblocks, t.kb_per_split);
+  const int64_t kblocks = std::max(1, t.kblocks);
+  splits = std::min(splits, kblocks);
+  t.kb_per_split = (int)std::min<int64_t>(ceil_div(kblocks, splits), kbmax);
+  t.splits = (int)ceil_div(kblocks, t.kb_per_split);
   // Raster band (tiles of M visited together): measured best at 8192^3 and
   // 16384^3 -- 16 for the BF16 paths (128 x 256 tiles), 4 for Ozaki; pair
   // tiles keep the same band height in rows (8 tiles of 256).
