@@ -599,22 +599,28 @@ __global__ void splitk_reduce_kernel(const T* __restrict__ ws, int64_t split_str
     const int c = (int)(idx - r * nv) * VEC;
     const T* w = ws + r * ldw + c;
     T* o = C + r * ldc + c;
-    if (c + VEC <= n) {
-      V s = sum_planes<T, LONG>(w, split_stride, splits);
-      T* ps = reinterpret_cast<T*>(&s);
-      V cv;
-      if (beta != T(0)) cv = *reinterpret_cast<const V*>(o);
-      const T* pc = reinterpret_cast<const T*>(&cv);
+    const bool whole = c + VEC <= n;
+    V cv;  // (C's loads go out beside those of the planes)
+    T* pc = reinterpret_cast<T*>(&cv);
+    if (beta != T(0)) {
+      if (whole) {
+        cv = *reinterpret_cast<const V*>(o);
+      } else {
 #pragma unroll
-      for (int e = 0; e < VEC; ++e) ps[e] = apply_epi(combine(ps[e], alpha, beta, pc + e), epi);
+        for (int e = 0; e < VEC; ++e)
+          if (c + e < n) pc[e] = o[e];
+      }
+    }
+    V s = sum_planes<T, LONG>(w, split_stride, splits);  // (planes are padded to whole vectors)
+    T* ps = reinterpret_cast<T*>(&s);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) ps[e] = apply_epi(combine(ps[e], alpha, beta, pc + e), epi);
+    if (whole) {
       *reinterpret_cast<V*>(o) = s;
     } else {
-      // (planes are padded to whole vectors: elements past n are read, never used)
-      V s = sum_planes<T, LONG>(w, split_stride, splits);
-      const T* ps = reinterpret_cast<const T*>(&s);
 #pragma unroll
       for (int e = 0; e < VEC; ++e)
-        if (c + e < n) o[e] = apply_epi(combine(ps[e], alpha, beta, o + e), epi);
+        if (c + e < n) o[e] = ps[e];
     }
   }
 }
