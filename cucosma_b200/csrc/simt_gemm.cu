@@ -98,8 +98,15 @@ __device__ __forceinline__ void cluster_reduce(const SimtParams& p, const T* til
   V cnext;
   auto load_c = [&](int v) {
     const int r = m0 + v / VPR, c = n0 + (v % VPR) * VEC;
-    if (beta != T(0) && v < ROWS * VPR && r < p.m && c + VEC <= p.n)
-      cnext = *reinterpret_cast<const V*>(reinterpret_cast<const T*>(p.out) + (int64_t)r * p.ldo + c);
+    if (beta == T(0) || v >= ROWS * VPR || r >= p.m) return;
+    const T* o = reinterpret_cast<const T*>(p.out) + (int64_t)r * p.ldo + c;
+    if (c + VEC <= p.n) {
+      cnext = *reinterpret_cast<const V*>(o);
+    } else {
+#pragma unroll
+      for (int e = 0; e < VEC; ++e)
+        if (c + e < p.n) reinterpret_cast<T*>(&cnext)[e] = o[e];
+    }
   };
   int v = (int)cluster_ctarank() * THREADS + (int)threadIdx.x;
   load_c(v);
@@ -124,15 +131,15 @@ __device__ __forceinline__ void cluster_reduce(const SimtParams& p, const T* til
         for (int e = 0; e < VEC; ++e) sum[e] += t[e];
       }
     T* o = reinterpret_cast<T*>(p.out) + (int64_t)r * p.ldo + c;
-    if (c + VEC <= p.n) {
-      const T* pc = reinterpret_cast<const T*>(&cv);
+    const T* pc = reinterpret_cast<const T*>(&cv);
 #pragma unroll
-      for (int e = 0; e < VEC; ++e) sum[e] = apply_epi(combine(sum[e], alpha, beta, pc + e), p.epilogue);
+    for (int e = 0; e < VEC; ++e) sum[e] = apply_epi(combine(sum[e], alpha, beta, pc + e), p.epilogue);
+    if (c + VEC <= p.n) {
       *reinterpret_cast<V*>(o) = part[0];
     } else {
 #pragma unroll
       for (int e = 0; e < VEC; ++e)
-        if (c + e < p.n) o[e] = apply_epi(combine(sum[e], alpha, beta, o + e), p.epilogue);
+        if (c + e < p.n) o[e] = sum[e];
     }
   }
   __syncwarp();
