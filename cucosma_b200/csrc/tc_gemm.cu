@@ -410,6 +410,25 @@ static bool deep_ring(const cucosma_gemm_desc* d, const Tiling& t, const DeviceI
   return elems * 10.0 > (double)di->l2_bytes && t.kb_per_split >= 8;
 }
 
+// Fused tiles, C-heavy: whether the epilogue outlasts a unit's conversions and
+// MMAs, so that its two staging blocks are worth a pipeline stage.  Lines
+// between K of 48 and 800, 128 to 1500 rows or columns by 20,000 to 150,000, on
+// B200; us with two blocks / one at 150,000 x 200 x K: BF16x3, beta 0.5, K = 256
+// 126 / 135, 400 205 / 171; BF16x6, beta 0.5, 160 129 / 135, 256 168 / 150; beta
+// 0 BF16x6 64 72 / 70, 256 142 / 132; sigmoid at beta 0.5 BF16x3 640 254 / 260,
+// 800 317 / 309.  With two blocks the last N % 32 columns leave by rows, which
+// beside a whole chunk in the same 64 columns is slower than one block's boxes
+// where C is not read (60,000 x 500 x 128 BF16x3 sigmoid 100 / 80, 30,000 x 1000
+// x 250 121 / 94; few such tiles in a wide C).  With one block rows that do not
+// end on 16 bytes leave one by one: two blocks there.
+static bool epilogue_bound(const cucosma_gemm_desc* d, const Plan& pl) {
+  // most k-blocks of a unit: [precision][C read][sigmoid]
+  constexpr int kMost[2][2][2] = {{{4, 8}, {8, 20}}, {{3, 5}, {5, 14}}};
+  if (d->n % 4 != 0 || pl.t.splits > 1) return true;
+  if (d->beta == 0.0 && d->n % 64 > 32 && d->n < 4096) return false;
+  return pl.t.kblocks <= kMost[pl.kind][d->beta != 0.0][d->epilogue == CUCOSMA_EPILOGUE_SIGMOID];
+}
+
 static int plan_launches(const Plan& pl) {
   if (pl.fused) return 1 + (pl.t.splits > 1 ? 1 : 0);
   if (pl.kind != 2) return 2 + (pl.t.splits > 1 || pl.t.tail_splits > 1 ? 1 : 0);  // the split of A and B, the GEMM
@@ -591,10 +610,13 @@ cucosma_status tc_gemm_ex(const cucosma_gemm_desc* d, const void* A, const void*
     // (256 x 1,048,576 x 256, beta 0.5: 0.85 against 0.94 ms on B200)
     const double c_bytes = (double)d->m * d->n * 4.0 * (d->beta != 0.0 ? 2.0 : 1.0);
     const double ab_bytes = ((double)d->m * d->k + (double)d->k * d->n) * 4.0;
-    const bool c_heavy = c_bytes > 0.25 * ab_bytes;
+    const bool c_heavy = c_bytes > 0.25 * ab_bytes && epilogue_bound(d, pl);
     const TcParams p = tc_params(d, pl.t, pl, C, w, di, !c_heavy);
     prof_begin(st);
-    const bool direct = c_heavy && one_chunk(pl.t);
+    // (BF16x3 that neither reads C nor takes the sigmoid has nothing to gain
+    // from it: 256 x 200,001 x 64 84.4 us promoted, 88.3 direct)
+    const bool direct = c_heavy && one_chunk(pl.t) &&
+                        (pl.kind == 1 || d->beta != 0.0 || d->epilogue == CUCOSMA_EPILOGUE_SIGMOID);
     // C read by rows, not boxes: 512 x 8191 x 4096 BF16x3, beta 0.5, 168 us,
     // 199 with C read beside its stores, 182 on the two-block variant
     const bool rows_c = !c_heavy && !p.tma_out && !p.partial && d->beta != 0.0;
