@@ -235,6 +235,19 @@ static Tail plan_tail(int64_t tiles, int64_t slots, int64_t kblocks, double unit
   return best;
 }
 
+// C's taller than the time model's calls with K of at most 12 k-blocks, whose
+// operands, planes and C pass L2: the model counts the pre-pass and C at the
+// rates of data in L2.  Fused where fused_pays says so: 72,739 x 200 x 161 BF16x3
+// 67.6 us by the model, 49.1 fused, 28,640 x 892 x 371, beta 0.5, 140 / 109,
+// 107,248 x 252 x 56 75.8 / 51.8; but within L2 33,722 x 452 x 207 45.8 / 53.3,
+// wide 352 x 105,992 x 91 75.9 / 100.6, and rows not ending on 16 bytes 81,451 x
+// 530 x 201 131 / 158.  68 tall calls: 0.95 of the time of the model alone.
+static bool tall_short_k(const cucosma_gemm_desc* d, int slices, const DeviceInfo* di) {
+  const double M = (double)d->m, N = (double)d->n, K = (double)d->k;
+  return d->split_k <= 0 && d->m > 8192 && d->k <= 12 * 32 && d->n % 4 == 0 &&
+         (M * K + K * N) * (4.0 + 2.0 * slices) + M * N * 4.0 > 0.95 * (double)di->l2_bytes && fused_pays(d, slices);
+}
+
 // The (tile, splits) with the smallest modelled time; forced > 0 fixes the splits.
 static void choose_bf16(const cucosma_gemm_desc* d, int kind, const DeviceInfo* di, bool allow_fused, int& variant,
                         int64_t& splits) {
@@ -309,10 +322,13 @@ static Plan make_plan(const cucosma_gemm_desc* d, const DeviceInfo* di, bool all
         }
         [[fallthrough]];
       default:
-        // Auto.  Operands that fit L2: the time model.  Larger ones: pair
+        // Auto.  Operands that fit L2: the time model, but for C's longer than
+        // its calls had (8192) with K short enough that moving C decides
+        // (long_short_k).  Larger ones: pair
         // tiles (unless there is a single 128-row block), fused where the
         // pre-pass's HBM traffic would show, splits by make_tiling.
-        if (((double)M * K + (double)K * N) * 4.0 <= (double)di->l2_bytes)
+        if (((double)M * K + (double)K * N) * 4.0 <= (double)di->l2_bytes &&
+            !(allow_fused && tall_short_k(d, slices, di)))
           choose_bf16(d, pl.kind, di, allow_fused, pl.variant, splits);
         else if (M <= 128)
           pl.variant = pl.kind == 0 ? kV3Promoted : kV6Single;

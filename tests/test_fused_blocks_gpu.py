@@ -33,3 +33,29 @@ def test_equals_the_prepass_path(cuda, precision, ftile, utile, epilogue, beta, 
     cc.gemm(A, B, C, 1.0, beta, tile=ftile, **kw)
     cc.gemm(A, B, D, 1.0, beta, tile=utile, **kw)
     assert torch.equal(C, D)
+
+
+@pytest.mark.parametrize("precision,utile", [("bf16x3", 4), ("bf16x6", 2)])
+@pytest.mark.parametrize("m,n,k,fused", [(72739, 200, 161, 1), (30011, 1000, 384, None), (8193, 2052, 96, None),
+                                         (8200, 132, 384, None), (60001, 331, 100, None)])
+def test_tall_calls_of_short_k(cuda, precision, utile, m, n, k, fused):
+    """Automatic calls with a tall C beyond L2 are fused; any plan's result
+    equals the pre-pass path's, bit for bit."""
+    import torch
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m)
+    A = torch.zeros((m, -(-k // 4) * 4), device="cuda")[:, :k]
+    A.copy_(torch.rand((m, k), generator=g, device="cuda") * 2 - 1)
+    B, C, D = (torch.zeros((r, -(-n // 4) * 4), device="cuda")[:, :n] for r in (k, m, m))
+    B.copy_(torch.rand((k, n), generator=g, device="cuda") * 2 - 1)
+    plan = cc.get_plan(cc.make_desc(A, B, C, precision=precision))
+    assert fused is None or plan["fused"] == fused
+    cc.gemm(A, B, C, precision=precision)
+    if plan["fused"]:
+        cc.gemm(A, B, D, precision=precision, tile=utile, split_k=plan["splits"])
+        assert torch.equal(C, D)
+    else:
+        ref = A.double() @ B.double()
+        err = (C - ref).abs().amax() / (A.abs().double() @ B.abs().double()).amax()
+        assert float(err) <= 2.0 ** (-15 if precision == "bf16x3" else -21)
